@@ -24,18 +24,42 @@ __device__ __forceinline__ void st9(float* p, size_t i, const float* v) {
 struct BeePtrs { float* y[13]; };
 struct BeeGrads { const float* g[13]; };
 
-__global__ void bee_fwd_kernel(const float* __restrict__ l0, const float* __restrict__ l1, const float* __restrict__ l2,
-                               const float* __restrict__ r0, const float* __restrict__ r1, const float* __restrict__ r2,
-                               BeePtrs out, size_t n) {
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+// A warp's 32 consecutive results of S components each, as contiguous 128-byte stores: stored lane by lane they would be
+// S stores at a stride of S floats, each touching every sector of the run (36 k edges x 128 channels: 0.72 ms for the
+// thirteen outputs, 1.2 GB, against 0.22 ms staged). wbuf: 32 * S floats of this warp (S odd: no bank conflicts);
+// live: how many of the 32 exist.
+template <int S>
+__device__ __forceinline__ void warp_store(float* __restrict__ g, float* wbuf, int lane, int live, const float* v) {
+#pragma unroll
+  for (int s = 0; s < S; s++) wbuf[lane * S + s] = v[s];
+  __syncwarp();
+#pragma unroll
+  for (int j = 0; j < S; j++)
+    if (lane + 32 * j < live * S) g[lane + 32 * j] = wbuf[lane + 32 * j];
+  __syncwarp();
+}
+
+constexpr int BEE_WARPS = 8;
+
+__global__ void __launch_bounds__(BEE_WARPS * 32)
+bee_fwd_kernel(const float* __restrict__ l0, const float* __restrict__ l1, const float* __restrict__ l2,
+               const float* __restrict__ r0, const float* __restrict__ r1, const float* __restrict__ r2, BeePtrs out, size_t n) {
+  __shared__ float s_buf[BEE_WARPS][288];
+  const int lane = threadIdx.x & 31;
+  float* wb = s_buf[threadIdx.x >> 5];
+  for (size_t i0 = (size_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31); i0 < n; i0 += (size_t)gridDim.x * blockDim.x) {
+    const int live = n - i0 < 32 ? (int)(n - i0) : 32;
+    const size_t i = i0 + (lane < live ? lane : 0);   // lanes past the end repeat the first element and store nothing
     float a1[3], a2[9], b1[3], b2[9];
     ld3(l1, i, a1); ld9(l2, i, a2); ld3(r1, i, b1); ld9(r2, i, b2);
     BeeOut o;
     bee_fwd_point(l0[i], a1, a2, r0[i], b1, b2, &o);
-    out.y[0][i] = o.y000; out.y[1][i] = o.y110; out.y[2][i] = o.y220;
-    st3(out.y[3], i, o.y011); st3(out.y[4], i, o.y101); st3(out.y[5], i, o.y121); st3(out.y[6], i, o.y211);
-    st9(out.y[7], i, o.y022); st9(out.y[8], i, o.y202); st9(out.y[9], i, o.y112); st9(out.y[10], i, o.y222);
-    st3(out.y[11], i, o.y111); st9(out.y[12], i, o.y212);
+    if (lane < live) { out.y[0][i] = o.y000; out.y[1][i] = o.y110; out.y[2][i] = o.y220; }
+    warp_store<3>(out.y[3] + i0 * 3, wb, lane, live, o.y011); warp_store<3>(out.y[4] + i0 * 3, wb, lane, live, o.y101);
+    warp_store<3>(out.y[5] + i0 * 3, wb, lane, live, o.y121); warp_store<3>(out.y[6] + i0 * 3, wb, lane, live, o.y211);
+    warp_store<9>(out.y[7] + i0 * 9, wb, lane, live, o.y022); warp_store<9>(out.y[8] + i0 * 9, wb, lane, live, o.y202);
+    warp_store<9>(out.y[9] + i0 * 9, wb, lane, live, o.y112); warp_store<9>(out.y[10] + i0 * 9, wb, lane, live, o.y222);
+    warp_store<3>(out.y[11] + i0 * 3, wb, lane, live, o.y111); warp_store<9>(out.y[12] + i0 * 9, wb, lane, live, o.y212);
   }
 }
 
@@ -271,7 +295,7 @@ extern "C" int ld_bee_fwd(const float* l0, const float* l1, const float* l2, con
   if (n == 0) return LD_OK;
   BeePtrs P;
   for (int k = 0; k < 13; k++) P.y[k] = out13[k];
-  bee_fwd_kernel<<<grid_for(n), 256, 0, (cudaStream_t)stream>>>(l0, l1, l2, r0, r1, r2, P, n);
+  bee_fwd_kernel<<<grid_for(n), BEE_WARPS * 32, 0, (cudaStream_t)stream>>>(l0, l1, l2, r0, r1, r2, P, n);
   LD_LAUNCH_CHECK();
   return LD_OK;
 }
