@@ -1,0 +1,551 @@
+// PaiNN message step at FP32 accuracy with the distance MLP on the tensor cores: the computation of painn_message.cu
+// (Message.forward, archs/meanflow_painn8.py:77-100) with operands split into two FP16 values (split_f16.cuh).
+//
+// What bounds it: the shared-memory port. The two 4n x 4n layers are 3 x 2 x (4n)^2 flops an edge on the tensor cores; an MMA
+// of 128 x 64 x 16 (n = 128) takes 48 cycles, the time to read its 6 KB of operands, not the 32 of the tensor pipe, and the
+// weight slabs (2 MB per tile) come in through the same port: 433 cycles a slab of six MMAs measured, 416 by that count.
+// n = 128, 8 radial functions, 562 k edges: 3.04 ms, against 22.8 ms on the FMA pipe (painn_message.cu); n = 64, 11 k edges:
+// 61 us against 195. Error against 64 bits: 6.1e-7, against 7.5e-7.
+//
+// A block owns a node-aligned, contiguous slice of the CSR and walks it 256 / (n / 32) edges at a time. Roles:
+//   * 16 working warps: geometry, radial features -> activation planes in shared memory; per layer each thread adds the
+//     partial sums of its channel (64 edges) from tensor memory into registers, then writes bias + SiLU back as the next
+//     layer's planes; after the last layer the product with the neighbour's activation goes to shared memory in FP32 and
+//     is turned into messages and per-node sums, 16 edges per thread, joined in edge order (no atomics, fixed order, every
+//     node written once).
+//   * 2 MMA warps and 1 producer warp (lane 0 of each): six MMAs per 16 KB weight slab; slabs stream through a ring.
+// Every wait is bounded (LD_FLAG_TIMEOUT): a failed wait is OR-ed into the next block barrier so that all threads leave
+// together.
+#include "common.cuh"
+#include "split_f16.cuh"
+#include "tp_math.h"
+
+namespace {
+
+constexpr int WORK_WARPS = 16, WORK_THREADS = WORK_WARPS * 32;
+// Two issuing warps take the slabs in turn: a poll of a barrier costs about 220 cycles in the issuing thread even when the
+// barrier is ready, and no MMA of that thread is queued meanwhile (one 288-cycle slab per poll: 532 cycles a slab measured);
+// with two threads one polls while the other's MMAs run. A slab's accumulator belongs to one thread, so its order is fixed.
+constexpr int MMA_WARPS = 2, MMA_WARP = WORK_WARPS, PROD_WARP = WORK_WARPS + MMA_WARPS;
+constexpr int THREADS = (WORK_WARPS + MMA_WARPS + 1) * 32;
+constexpr int SYNC_THREADS = (WORK_WARPS + MMA_WARPS) * 32;   // working and MMA warps meet at barrier 1
+constexpr int STAGES = 5;                             // weight slabs in the ring
+constexpr int EPT = 16;                               // edges per thread in the message phase
+
+// MB: blocks of 128 channels; n = 32 MB
+template <int MB>
+struct Shape {
+  static constexpr int N = 128 * MB, n = 32 * MB;
+  static constexpr int NE = 256 / MB;                 // edges per tile = N of an MMA
+  static constexpr int PANEL = NE * 16 + 16;          // bytes between panels of 8 channels (the 16 spread a warp's stores over the banks)
+  static constexpr int PLANE = (N / 8) * PANEL;
+  static constexpr int ACT = 2 * PLANE;               // also the FP32 products [N][NE + 1]
+  static constexpr int SLOTS = 2 * MB;                // accumulators of NE columns in tensor memory
+  static constexpr int G = WORK_THREADS / n;          // threads per channel in the message phase
+  static_assert(N * (NE + 1) * 4 <= ACT, "the products reuse the activation planes");
+  static_assert(G * EPT == NE, "the message phase covers the tile");
+  static constexpr size_t SMEM = (size_t)ACT + STAGES * sf::SLAB_BYTES + 3 * N * 4;
+};
+
+struct SplitParams {
+  const int* row_ptr; const int* dst; const float* rij;
+  int Nt, n_rbf, k0p, radial_kind, seg_nodes;
+  float rmax, pi_over_rmax, eps;
+  const __half* w[3];      // packed slabs per layer
+  const float* b[3];
+  const float* scales;     // [3] input scales, [3] weight scales, [3] their inverse products
+  const float* actv; const float* x_v; const float* res_a; const float* res_v;
+  float* out_a; float* out_v;
+  long long* edge_counter;
+  int* status;
+};
+
+__device__ __forceinline__ int work_lower_bound(const int* __restrict__ row_ptr, int lo, int hi, long long target) {
+  const long long base = (long long)row_ptr[lo] + lo;
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if ((long long)row_ptr[mid] + mid - base < target) lo = mid + 1; else hi = mid;
+  }
+  return lo;
+}
+
+struct BlockRange { int n_begin, n_end; long long e_begin, e_end, ntiles; };
+
+// node-aligned share of segment [lo, hi) for this block, balanced over edges + nodes
+__device__ __forceinline__ BlockRange block_range(const int* __restrict__ row_ptr, int lo, int hi, int tile) {
+  BlockRange r;
+  const long long work = ((long long)row_ptr[hi] - row_ptr[lo]) + (hi - lo);
+  long long per = (work + gridDim.x - 1) / gridDim.x;
+  if (per < tile) per = tile;
+  r.n_begin = blockIdx.x == 0 ? lo : work_lower_bound(row_ptr, lo, hi, per * blockIdx.x);
+  r.n_end = blockIdx.x == gridDim.x - 1 ? hi : work_lower_bound(row_ptr, lo, hi, per * (blockIdx.x + 1));
+  r.e_begin = r.n_begin < r.n_end ? row_ptr[r.n_begin] : 0;
+  r.e_end = r.n_begin < r.n_end ? row_ptr[r.n_end] : 0;
+  r.ntiles = (r.e_end - r.e_begin + tile - 1) / tile;
+  return r;
+}
+
+// barrier 1: working warps + MMA warps; returns the OR of `flag` over its participants
+__device__ __forceinline__ int sync_or(int flag) {
+  int out;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.u32 q, %1, 0;\n\t"
+      "barrier.cta.red.or.pred p, 1, %2, q;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(out) : "r"(flag), "n"(SYNC_THREADS) : "memory");
+  return out;
+}
+// barrier 2: working warps only
+__device__ __forceinline__ void sync_workers() { asm volatile("barrier.cta.sync 2, %0;" ::"n"(WORK_THREADS) : "memory"); }
+
+// the two factors of a Gaussian radial feature (radial_feature, kind 1), the envelope once per edge
+__device__ __forceinline__ float radial_envelope(float d, float rmax) {
+  return 0.5f * (cosf(3.14159265358979323846f * d / rmax) + 1.0f);
+}
+__device__ __forceinline__ float radial_gaussian(int m, int n, float d, float rmax) {
+  const float width = n > 1 ? rmax / (float)(n - 1) : rmax;
+  const float u = (d - (float)m * width) / width;
+  return expf(-0.5f * u * u);
+}
+// SiLU with the quotient from the reciprocal instruction (2 ulp)
+__device__ __forceinline__ float silu_fdiv(float x) { return __fdividef(x, 1.0f + expf(-x)); }
+
+template <int MB>
+__global__ void __launch_bounds__(THREADS, 1)
+painn_message_split_kernel(const __grid_constant__ SplitParams P) {
+  using S = Shape<MB>;
+  constexpr int N = S::N, n = S::n, NE = S::NE, SLOTS = S::SLOTS;
+  extern __shared__ __align__(1024) unsigned char smem[];
+  __shared__ __align__(8) uint64_t bar_full[STAGES], bar_done[SLOTS], bar_taken[2];
+  __shared__ uint32_t tmem_slot;
+  __shared__ float s_dir[NE][3];
+  __shared__ float s_dist[NE], s_env[NE];
+  __shared__ int s_dst[NE], s_src[NE];
+  __shared__ int s_rowwin[NE + 1];   // row_ptr[node_lo .. node_lo + NE] of the coming tile
+
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  unsigned char* act = smem;                                              // two activation planes
+  float* prod = reinterpret_cast<float*>(smem);                           // [N][NE + 1], after the last layer
+  unsigned char* ring = smem + S::ACT;
+  float* s_bias = reinterpret_cast<float*>(ring + STAGES * sf::SLAB_BYTES);   // [3][N]
+
+  for (int i = tid; i < 3 * N; i += THREADS) s_bias[i] = P.b[i / N][i % N];
+  if (tid == 0) {
+    for (int s = 0; s < STAGES; s++) tc::mbar_init(&bar_full[s], 1);
+    for (int s = 0; s < SLOTS; s++) tc::mbar_init(&bar_done[s], 1);      // MMAs of slab q: slot q % SLOTS
+    for (int s = 0; s < 2; s++) tc::mbar_init(&bar_taken[s], WORK_WARPS);   // partial sums of a chunk are in registers
+    tc::mbar_init_fence();
+  }
+  if (warp == 0) { tc::tmem_alloc(&tmem_slot, 512); tc::tmem_relinquish(); }
+  tc::fence_before_sync();
+  __syncthreads();
+  tc::fence_after_sync();
+  const uint32_t tmem_base = tmem_slot;
+  const int seg_nodes = P.seg_nodes > 0 ? P.seg_nodes : P.Nt;
+  int fail = 0;
+
+  if (warp == PROD_WARP) {
+    // ===== producer: weight slabs through the ring, independent of the data ====================================
+    if (lane == 0) {
+      uint32_t loads = 0;
+      for (int seg_lo = 0; seg_lo < P.Nt && !fail; seg_lo += seg_nodes) {
+        const long long ntiles = block_range(P.row_ptr, seg_lo, min(seg_lo + seg_nodes, P.Nt), NE).ntiles;
+        for (long long t = 0; t < ntiles && !fail; t++)
+          for (int layer = 0; layer < 3 && !fail; layer++) {
+            const int K = layer == 0 ? P.k0p : N;
+            const unsigned char* src = reinterpret_cast<const unsigned char*>(P.w[layer]);
+            for (int k0 = 0; k0 < K && !fail; k0 += sf::SLAB_K) {
+              const uint32_t bytes = 2u * 128u * 2u * (uint32_t)min(sf::SLAB_K, K - k0);
+              for (int m = 0; m < MB; m++, loads++, src += bytes) {
+                const uint32_t st = loads % STAGES, old = loads - STAGES;   // the slab that held this stage
+                if (loads >= STAGES && !tc::mbar_wait(&bar_done[old % SLOTS], (old / SLOTS) & 1)) { fail = 1; break; }
+                tc::mbar_expect_tx(&bar_full[st], bytes);
+                tc::bulk_g2s(ring + (size_t)st * sf::SLAB_BYTES, src, bytes, &bar_full[st]);
+              }
+            }
+          }
+      }
+      if (fail) {
+        // copies already requested still land in this block's shared memory: give them a bounded chance
+        for (uint32_t i = loads > STAGES ? loads - STAGES : 0; i < loads; i++) tc::mbar_wait(&bar_full[i % STAGES], (i / STAGES) & 1);
+      }
+    }
+  } else if (warp >= MMA_WARP) {
+    // ===== MMA issue ==============================================================================================
+    // the issuing thread runs alone in its warp, so every instruction between two MMAs is exposed: descriptors and ring
+    // positions advance by additions, accumulators are waited for once per chunk of MB slabs, and one commit per slab
+    // reports both that the partial sum is complete and that the ring stage is free
+    const uint32_t me = warp - MMA_WARP;
+    uint32_t chunks = 0, st = me, full_phase = 0;
+    const uint64_t b1 = tc::smem_desc(tc::smem_u32(act), S::PANEL, 128), b2 = tc::smem_desc(tc::smem_u32(act + S::PLANE), S::PANEL, 128);
+    const uint64_t a0 = tc::smem_desc(tc::smem_u32(ring), 128 * 16, 128);
+    constexpr uint64_t b_step = (2 * S::PANEL) >> 4, st_step = sf::SLAB_BYTES >> 4;
+    constexpr uint32_t idesc = sf::idesc_f16(128, NE);
+    for (int seg_lo = 0; seg_lo < P.Nt && !fail; seg_lo += seg_nodes) {
+      const long long ntiles = block_range(P.row_ptr, seg_lo, min(seg_lo + seg_nodes, P.Nt), NE).ntiles;
+      for (long long t = 0; t < ntiles; t++) {
+        if (sync_or(fail)) { fail = 1; break; }      // [G] geometry staged
+        for (int layer = 0; layer < 3; layer++) {
+          if (sync_or(fail)) { fail = 1; break; }    // [X] this layer's activations are written
+          if (lane == 0) {
+            const int K = layer == 0 ? P.k0p : N;
+            uint64_t x1 = b1, x2 = b2;
+            for (int k0 = 0; k0 < K && !fail; k0 += sf::SLAB_K, chunks++, x1 += 2 * b_step, x2 += 2 * b_step) {
+              const uint32_t ks = K - k0 > 16 ? 2 : 1;
+              if (MB == 1 && (chunks & 1) != me) continue;
+              // the partial sums that lie in this half of tensor memory have been taken
+              if (chunks >= 2 && !tc::mbar_wait(&bar_taken[chunks & 1], ((chunks >> 1) - 1) & 1)) { fail = 1; break; }
+              tc::fence_after_sync();
+#pragma unroll
+              for (int h = 0; h < (MB + 1) / 2; h++) {
+                const uint32_t slot = (chunks & 1) * MB + (MB == 1 ? 0 : 2 * h + me);   // slabs are numbered chunk * MB + block
+                if (!tc::mbar_wait(&bar_full[st], full_phase)) { fail = 1; break; }
+                sf::slab_mmas(tmem_base + slot * NE, a0 + st * st_step, ks, x1, x2, b_step, idesc);
+                tc::mma_commit(&bar_done[slot]);
+                st += MMA_WARPS;
+                if (st >= STAGES) { st -= STAGES; full_phase ^= 1; }
+              }
+            }
+          }
+          fail = __shfl_sync(0xffffffffu, fail, 0);
+          if (sync_or(fail)) { fail = 1; break; }    // [A] every partial sum of the layer has been taken
+        }
+        if (fail) break;
+      }
+    }
+  } else {
+    // ===== working warps ============================================================================================
+    const int mblk = (warp >> 2) % MB, half = (warp >> 2) / MB, quarter = warp & 3;
+    const int o = mblk * 128 + quarter * 32 + lane;   // this thread's channel, and edges [64 half, 64 half + 64)
+    const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + half * 64;
+    const float sx1 = P.scales[1], sx2 = P.scales[2];
+    const float inv0 = P.scales[6], inv1 = P.scales[7], inv2 = P.scales[8];
+    uint32_t chunks = 0;                              // partial sums taken so far by this thread's channel block
+    const int mc = tid % n, mg = tid / n;             // message phase: channel, group of EPT edges
+    long long edges_done = 0;
+
+    for (int seg_lo = 0; seg_lo < P.Nt && !fail; seg_lo += seg_nodes) {
+      const BlockRange br = block_range(P.row_ptr, seg_lo, min(seg_lo + seg_nodes, P.Nt), NE);
+      const int n_begin = br.n_begin, n_end = br.n_end;
+      float carry = 0.f;          // thread tid < 4n: sum of output (component tid / n, channel tid % n) of node `cur`
+      int cur = n_begin;
+      int node_lo = n_begin;      // source node of the next tile's first edge (or an earlier one)
+      sync_workers();             // the previous segment's last readers of s_rowwin are done
+      for (int i = tid; i <= NE; i += WORK_THREADS) s_rowwin[i] = P.row_ptr[min(node_lo + i, n_end > n_begin ? n_end : n_begin)];
+      sync_workers();
+
+      auto write_out = [&](int v, int c, int k, float val) {
+        if (k < 3) {
+          const size_t off = ((size_t)v * n + c) * 3 + k;
+          P.out_v[off] = P.res_v != nullptr ? val + P.res_v[off] : val;
+        } else {
+          const size_t off = (size_t)v * n + c;
+          P.out_a[off] = P.res_a != nullptr ? val + P.res_a[off] : val;
+        }
+      };
+      // output of node `from`, zeros for the nodes (from, next)
+      auto flush_until = [&](int from, int next, float val) {
+        if (tid < 4 * n)
+          for (int v = from; v < next; v++) write_out(v, mc, mg, v == from ? val : 0.f);
+      };
+
+      for (long long e0 = br.e_begin; e0 < br.e_end; e0 += NE) {
+        const int cnt = (int)(br.e_end - e0 < NE ? br.e_end - e0 : NE);
+        // ---- geometry --------------------------------------------------------------------------------------------
+        if (tid < NE) {
+          float dx = 0.f, dy = 0.f, dz = 0.f;
+          int j = 0, s = -1;
+          if (tid < cnt) {
+            const long long e = e0 + tid;
+            dx = P.rij[e * 3]; dy = P.rij[e * 3 + 1]; dz = P.rij[e * 3 + 2];
+            j = P.dst[e];
+            // source node: largest v with row_ptr[v] <= e, in the staged window first
+            int lo, hi;
+            if ((long long)s_rowwin[NE] > e) {
+              lo = 0; hi = NE;
+              while (hi - lo > 1) { const int mid = (lo + hi) >> 1; if ((long long)s_rowwin[mid] > e) hi = mid; else lo = mid; }
+              s = node_lo + lo;
+            } else {
+              lo = node_lo + NE; hi = n_end;   // row_ptr[lo] <= e < row_ptr[hi]
+              while (hi - lo > 1) { const int mid = (lo + hi) >> 1; if ((long long)P.row_ptr[mid] > e) hi = mid; else lo = mid; }
+              s = lo;
+            }
+          }
+          const float r2 = dx * dx + dy * dy + dz * dz;
+          const float inv = 1.0f / sqrtf(P.eps + r2);
+          s_dir[tid][0] = dx * inv; s_dir[tid][1] = dy * inv; s_dir[tid][2] = dz * inv;
+          const float d = sqrtf(r2);
+          s_dist[tid] = d;
+          s_env[tid] = P.radial_kind == 1 && d < P.rmax ? radial_envelope(d, P.rmax) : 0.f;
+          s_dst[tid] = j;
+          s_src[tid] = s;
+        }
+        if (sync_or(fail)) { fail = 1; break; }                                              // [G]
+        // ---- radial features -> planes of the first layer (|feature| <= 1) ----------------------------------------
+        for (int i = tid; i < NE * P.k0p; i += WORK_THREADS) {
+          const int e = i % NE, k = i / NE;
+          float f = 0.f;
+          if (e < cnt && k < P.n_rbf)
+            f = P.radial_kind == 1 ? radial_gaussian(k, P.n_rbf, s_dist[e], P.rmax) * s_env[e]
+                                   : radial_feature(0, k, P.n_rbf, s_dist[e], P.rmax, P.pi_over_rmax);
+          __half h1, h2;
+          sf::split(f * 16384.f, &h1, &h2);
+          unsigned char* at = act + (k >> 3) * S::PANEL + e * 16 + (k & 7) * 2;
+          *reinterpret_cast<__half*>(at) = h1;
+          *reinterpret_cast<__half*>(at + S::PLANE) = h2;
+        }
+        tc::fence_async_smem();
+        // ---- three layers ------------------------------------------------------------------------------------------
+        float acc[64];
+        for (int layer = 0; layer < 3; layer++) {
+          if (sync_or(fail)) { fail = 1; break; }                                            // [X]
+          const int nch = ((layer == 0 ? P.k0p : N) + sf::SLAB_K - 1) / sf::SLAB_K;
+#pragma unroll
+          for (int i = 0; i < 64; i++) acc[i] = 0.f;
+          for (int ch = 0; ch < nch && !fail; ch++, chunks++) {
+            const uint32_t slot = (chunks & 1) * MB + mblk;
+            if (!tc::mbar_wait(&bar_done[slot], (chunks >> 1) & 1)) { fail = 1; break; }
+            tc::fence_after_sync();
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+              float v[16];
+              tc::tmem_ld16(taddr + slot * NE + 16 * q, v);
+#pragma unroll
+              for (int i = 0; i < 16; i++) acc[16 * q + i] += v[i];
+            }
+            tc::fence_before_sync();
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(&bar_taken[chunks & 1]);
+          }
+          fail = __any_sync(0xffffffffu, fail);
+          if (sync_or(fail)) { fail = 1; break; }                                            // [A] the planes may be overwritten
+          const float bias = s_bias[layer * N + o], inv = layer == 0 ? inv0 : (layer == 1 ? inv1 : inv2);
+          if (layer < 2) {
+            const float sx = layer == 0 ? sx1 : sx2;
+            unsigned char* a1 = act + (o >> 3) * S::PANEL + (half * 64) * 16 + (o & 7) * 2;
+#pragma unroll
+            for (int i = 0; i < 64; i++) {
+              __half h1, h2;
+              sf::split(silu_fdiv(fmaf(acc[i], inv, bias)) * sx, &h1, &h2);
+              *reinterpret_cast<__half*>(a1 + i * 16) = h1;
+              *reinterpret_cast<__half*>(a1 + S::PLANE + i * 16) = h2;
+            }
+            tc::fence_async_smem();
+          } else {
+            // FP32, over the planes
+            float* pr = prod + o * (NE + 1) + half * 64;
+#pragma unroll
+            for (int i = 0; i < 64; i++) pr[i] = fmaf(acc[i], inv, bias);
+          }
+        }
+        if (fail) break;
+        const int tile_cur = cur;
+        node_lo = s_src[cnt - 1];
+        for (int i = tid; i <= NE; i += WORK_THREADS) s_rowwin[i] = P.row_ptr[min(node_lo + i, n_end)];   // for the next tile
+        sync_workers();
+        // ---- messages of channel mc, edges [EPT mg, EPT mg + EPT): the sum for the group's first node is its head, for its
+        // last node (when different) its tail; nodes strictly inside are complete and written at once -------------------
+        float head[4], sum[4];
+        bool first = true;
+        {
+          const int r_lo = mg * EPT, r_hi = min(r_lo + EPT, cnt);
+#pragma unroll
+          for (int k = 0; k < 4; k++) head[k] = sum[k] = 0.f;
+          if (r_lo < r_hi) {
+            int c_node = s_src[r_lo];
+            const float* pc = prod + mc * (NE + 1);
+            for (int eb = r_lo; eb < r_hi; eb += 4) {
+              // what four edges take from their neighbours: 28 loads in flight
+              float x[4][3], a[4][4];
+#pragma unroll
+              for (int i = 0; i < 4; i++) {
+                const size_t j = s_dst[eb + i];   // slots past cnt hold node 0
+                const float* xp = P.x_v + (j * n + mc) * 3;
+                const float* ap = P.actv + j * N + mc;
+#pragma unroll
+                for (int k = 0; k < 3; k++) x[i][k] = __ldg(xp + k);
+#pragma unroll
+                for (int k = 0; k < 4; k++) a[i][k] = __ldg(ap + k * n);
+              }
+#pragma unroll
+              for (int i = 0; i < 4; i++) {
+                const int e = eb + i;
+                if (e < r_hi) {
+                  const int s = s_src[e];
+                  if (s != c_node) {
+                    if (first) {
+#pragma unroll
+                      for (int k = 0; k < 4; k++) head[k] = sum[k];
+                      first = false;
+                    } else {
+#pragma unroll
+                      for (int k = 0; k < 4; k++) write_out(c_node, mc, k, sum[k]);
+                    }
+                    for (int z = c_node + 1; z < s; z++)   // nodes without edges
+#pragma unroll
+                      for (int k = 0; k < 4; k++) write_out(z, mc, k, 0.f);
+#pragma unroll
+                    for (int k = 0; k < 4; k++) sum[k] = 0.f;
+                    c_node = s;
+                  }
+                  const float p0 = pc[e] * a[i][0], p1 = pc[n * (NE + 1) + e] * a[i][1], p2 = pc[2 * n * (NE + 1) + e] * a[i][2];
+                  const float d0 = s_dir[e][0], d1 = s_dir[e][1], d2 = s_dir[e][2];
+                  sum[0] += x[i][0] * p0 + (x[i][1] * d2 - x[i][2] * d1) * p1 + d0 * p2;
+                  sum[1] += x[i][1] * p0 + (x[i][2] * d0 - x[i][0] * d2) * p1 + d1 * p2;
+                  sum[2] += x[i][2] * p0 + (x[i][0] * d1 - x[i][1] * d0) * p1 + d2 * p2;
+                  sum[3] += pc[3 * n * (NE + 1) + e] * a[i][3];
+                }
+              }
+            }
+          }
+        }
+        sync_workers();   // the products have been read: their place takes the heads and tails
+        float* s_head = prod;
+        float* s_tail = prod + 4 * WORK_THREADS;
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          s_head[(mg * 4 + k) * n + mc] = first ? sum[k] : head[k];
+          s_tail[(mg * 4 + k) * n + mc] = first ? 0.f : sum[k];
+        }
+        sync_workers();
+        // ---- the groups in edge order, with the sum carried over from earlier tiles: thread = (component, channel) --------
+        if (tid < 4 * n) {
+          int c_node = tile_cur;
+          float a = carry;
+          for (int g = 0; g < S::G && g * EPT < cnt; g++) {
+            const int f = s_src[g * EPT], l = s_src[min(g * EPT + EPT, cnt) - 1];
+            if (f != c_node) { flush_until(c_node, f, a); a = 0.f; c_node = f; }
+            a += s_head[g * 4 * n + tid];
+            if (l != f) {
+              flush_until(f, f + 1, a);   // node f alone: the gaps after it were filled by the group's thread
+              a = s_tail[g * 4 * n + tid];
+              c_node = l;
+            }
+          }
+          carry = a;
+        }
+        cur = node_lo;
+        sync_workers();   // geometry and planes are rewritten by the next tile
+      }
+      if (!fail && n_begin < n_end) {
+        flush_until(cur, n_end, carry);
+        edges_done += br.e_end - br.e_begin;
+      }
+    }
+    if (!fail && P.edge_counter != nullptr && tid == 0 && edges_done > 0)
+      atomicAdd((unsigned long long*)P.edge_counter, (unsigned long long)edges_done);
+  }
+  if (fail && lane == 0 && P.status != nullptr) atomicOr(P.status, LD_FLAG_TIMEOUT);
+  __syncthreads();
+  if (warp == 0) tc::tmem_dealloc(tmem_base, 512);
+}
+
+// scales of the three layers of an MLP (k0 -> N -> N -> N) whose inputs are at most 1 in size and whose activation does
+// not enlarge them: |input of layer l + 1| <= max over outputs of sum |W_l| * bound_l + |b_l|. Wt: [in][out].
+__global__ void __launch_bounds__(512) split_scales_kernel(const float* W1t, const float* b1, const float* W2t, const float* b2,
+                                                           const float* W3t, int k0, int N, float* __restrict__ scales) {
+  __shared__ float s_b[512], s_m[512];
+  float bound = 1.0f;
+  for (int layer = 0; layer < 3; layer++) {
+    const float* W = layer == 0 ? W1t : (layer == 1 ? W2t : W3t);
+    const float* b = layer == 0 ? b1 : b2;
+    const int K = layer == 0 ? k0 : N, o = threadIdx.x;
+    float sum = 0.f, mx = 0.f;
+    if (o < N)
+      for (int k = 0; k < K; k++) { const float a = fabsf(W[(size_t)k * N + o]); sum += a; mx = fmaxf(mx, a); }
+    s_b[o] = o < N ? fmaf(sum, bound, layer < 2 ? fabsf(b[o]) : 0.f) * 1.001f : 0.f;   // (rounding of the sum)
+    s_m[o] = mx;
+    __syncthreads();
+    for (int d = 256; d > 0; d >>= 1) {
+      if (o < d) { s_b[o] = fmaxf(s_b[o], s_b[o + d]); s_m[o] = fmaxf(s_m[o], s_m[o + d]); }
+      __syncthreads();
+    }
+    if (o == 0) {
+      const float sx = layer == 0 ? 16384.f : sf::scale_for(bound), sw = sf::scale_for(s_m[0]);
+      scales[layer] = sx; scales[3 + layer] = sw; scales[6 + layer] = 1.0f / (sx * sw);
+    }
+    bound = s_b[0];
+    __syncthreads();
+  }
+}
+
+// Wt [in][out] -> slabs [K chunk of 32][block of 128 outputs][plane][K/8][128][8], K padded with zeros to a multiple of 16
+__global__ void split_pack_kernel(const float* __restrict__ Wt, int K, int N, const float* __restrict__ scale, __half* __restrict__ out) {
+  const int kp = (K + 15) / 16 * 16;
+  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
+  if (idx >= kp * N) return;
+  const int o = idx % N, k = idx / N;
+  const float v = k < K ? Wt[(size_t)k * N + o] * scale[0] : 0.f;
+  const int ch = k / sf::SLAB_K, kw = min(sf::SLAB_K, kp - ch * sf::SLAB_K), kl = k - ch * sf::SLAB_K;
+  __half* slab = out + (size_t)ch * sf::SLAB_K * N * 2 + (size_t)(o / 128) * kw * 128 * 2;
+  __half* at = slab + (size_t)(kl / 8) * 128 * 8 + (o % 128) * 8 + kl % 8;
+  sf::split(v, at, at + (size_t)kw * 128);
+}
+
+template <int MB>
+int launch(const SplitParams& P, cudaStream_t st) {
+  LD_CUDA_TRY(cudaFuncSetAttribute(painn_message_split_kernel<MB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Shape<MB>::SMEM));
+  int dev = 0, sms = 148;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  painn_message_split_kernel<MB><<<sms, THREADS, Shape<MB>::SMEM, st>>>(P);
+  LD_LAUNCH_CHECK();
+  return LD_OK;
+}
+
+}  // namespace
+
+static bool split_form(int n, int n_rbf) { return (n == 32 || n == 64 || n == 128) && n_rbf > 0 && n_rbf <= 4 * n; }
+
+// FP16 elements of the three packed layers of a distance MLP n_rbf -> 4n -> 4n -> 4n (0: these widths have no split form)
+extern "C" int ld_painn_split_elems(int n, int n_rbf, long long* elems) {
+  if (n <= 0 || n_rbf <= 0) return LD_ERR_SHAPE;
+  *elems = split_form(n, n_rbf) ? 2LL * 4 * n * ((n_rbf + 15) / 16 * 16 + 8 * n) : 0;
+  return LD_OK;
+}
+
+// packed: as many FP16 values as ld_painn_split_elems says, 16-byte aligned; scales: nine floats. Weights [in][out], FP32.
+extern "C" int ld_painn_split_pack(const float* W1t, const float* b1, const float* W2t, const float* b2, const float* W3t, int n,
+                                   int n_rbf, void* packed, float* scales, void* stream) {
+  if (!split_form(n, n_rbf)) { ld_set_last_message("painn split pack: n must be 32, 64 or 128, n_rbf at most 4n"); return LD_ERR_UNSUPPORTED; }
+  if (b1 == nullptr || b2 == nullptr) return LD_ERR_SHAPE;
+  const int N = 4 * n, k0p = (n_rbf + 15) / 16 * 16;
+  cudaStream_t st = (cudaStream_t)stream;
+  split_scales_kernel<<<1, 512, 0, st>>>(W1t, b1, W2t, b2, W3t, n_rbf, N, scales);
+  LD_LAUNCH_CHECK();
+  __half* out = (__half*)packed;
+  const float* W[3] = {W1t, W2t, W3t};
+  for (int l = 0; l < 3; l++) {
+    const int K = l == 0 ? n_rbf : N, kp = l == 0 ? k0p : N;
+    split_pack_kernel<<<ld_cdiv((long long)kp * N, 256), 256, 0, st>>>(W[l], K, N, scales + 3 + l, out);
+    LD_LAUNCH_CHECK();
+    out += (size_t)2 * N * kp;
+  }
+  return LD_OK;
+}
+
+// ld_painn_message_f32 with the distance MLP as packed by ld_painn_split_pack (n = 32, 64 or 128). status_dev receives
+// LD_FLAG_TIMEOUT if a bounded wait ran out.
+extern "C" int ld_painn_message_f32_split(const int* row_ptr, const int* dst, const float* rij, int Nt, int n, int n_rbf,
+                                          int radial_kind, float rmax, float eps, const void* packed, const float* scales,
+                                          const float* b1, const float* b2, const float* b3, const float* actv, const float* x_v,
+                                          const float* res_a, const float* res_v, float* out_a, float* out_v,
+                                          long long* edge_counter, int* status_dev, void* stream) {
+  if (Nt < 0 || n <= 0 || n_rbf <= 0) return LD_ERR_SHAPE;
+  if (!split_form(n, n_rbf)) { ld_set_last_message("painn message (split path): n must be 32, 64 or 128, n_rbf at most 4n"); return LD_ERR_UNSUPPORTED; }
+  if (b1 == nullptr || b2 == nullptr || b3 == nullptr) { ld_set_last_message("painn message: biases are required"); return LD_ERR_SHAPE; }
+  if (((uintptr_t)packed % 16) != 0) return LD_ERR_SHAPE;
+  if (Nt == 0) return LD_OK;
+  SplitParams P;
+  const int N = 4 * n, k0p = (n_rbf + 15) / 16 * 16;
+  P.row_ptr = row_ptr; P.dst = dst; P.rij = rij; P.Nt = Nt; P.n_rbf = n_rbf; P.k0p = k0p; P.radial_kind = radial_kind;
+  // blocks walk the node range in segments whose gathered rows (28 n bytes a node) stay in L2
+  P.seg_nodes = ld_even_segments(Nt, (40LL << 20) / (28LL * n));
+  P.rmax = rmax; P.pi_over_rmax = (float)(3.14159265358979323846 / (double)rmax); P.eps = eps;
+  P.w[0] = (const __half*)packed; P.w[1] = P.w[0] + (size_t)2 * N * k0p; P.w[2] = P.w[1] + (size_t)2 * N * N;
+  P.b[0] = b1; P.b[1] = b2; P.b[2] = b3; P.scales = scales; P.actv = actv; P.x_v = x_v; P.res_a = res_a; P.res_v = res_v;
+  P.out_a = out_a; P.out_v = out_v; P.edge_counter = edge_counter; P.status = status_dev;
+  if (n == 128) return launch<4>(P, (cudaStream_t)stream);
+  if (n == 64) return launch<2>(P, (cudaStream_t)stream);
+  return launch<1>(P, (cudaStream_t)stream);
+}

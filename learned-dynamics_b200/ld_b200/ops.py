@@ -248,6 +248,7 @@ class PackedMLP:
         l1, l2, l3 = linears
         self._linears = (l1, l2, l3)
         self._bf16 = None
+        self._split = None
         self.Wt = [l.weight.detach().t().contiguous().float() for l in (l1, l2, l3)]
         self.b = [None if l.bias is None else l.bias.detach().contiguous().float() for l in (l1, l2, l3)]
         self.dims = (l1.weight.shape[1], l1.weight.shape[0], l2.weight.shape[0], l3.weight.shape[0])
@@ -258,6 +259,24 @@ def _packed_bf16(mlp):
     if mlp._bf16 is None:
         mlp._bf16 = [pack_weights_bf16(l.weight.detach().float()) for l in mlp._linears]
     return mlp._bf16
+
+
+def _packed_split(mlp, n):
+    """(FP16 planes, scales) of a distance MLP n_rbf -> 4n -> 4n -> 4n for the split-precision message kernel, built on first
+    use; None for widths without that form."""
+    if mlp._split is None:
+        elems = ctypes.c_longlong(0)
+        check(lib().ld_painn_split_elems(n, mlp.dims[0], ctypes.byref(elems)))
+        if elems.value == 0 or any(b is None for b in mlp.b):
+            mlp._split = ()
+        else:
+            dev = mlp.Wt[0].device
+            packed = torch.empty(elems.value, dtype=torch.float16, device=dev)
+            scales = torch.empty(9, dtype=torch.float32, device=dev)
+            check(lib().ld_painn_split_pack(ptr(mlp.Wt[0]), ptr(mlp.b[0]), ptr(mlp.Wt[1]), ptr(mlp.b[1]), ptr(mlp.Wt[2]), n, mlp.dims[0],
+                                            ptr(packed), ptr(scales), stream_ptr(dev)))
+            mlp._split = (packed, scales)
+    return mlp._split or None
 
 
 def mlp3_rows(x, mlp, act=ACT_SILU):
@@ -289,6 +308,14 @@ def painn_message_f32(row_ptr, dst, rij, mlp_dist, actv, x_v, rmax, eps=0.1, rad
         raise RuntimeError("painn_message: row_ptr and dst must be int32")
     out_a = torch.empty(Nt, n, dtype=torch.float32, device=x_v.device)
     out_v = torch.empty(Nt, n, 3, dtype=torch.float32, device=x_v.device)
+    split = _packed_split(mlp_dist, n)
+    if split is not None:   # n = 32, 64, 128: the distance MLP on the tensor cores, operands as sums of two FP16 values
+        with KERNEL_TIMER.region("painn_message"):
+            check(lib().ld_painn_message_f32_split(ptr(row_ptr), ptr(dst), ptr(rij), Nt, n, n_rbf, radial_kind, float(rmax), float(eps),
+                                                   ptr(split[0]), ptr(split[1]), ptr(mlp_dist.b[0]), ptr(mlp_dist.b[1]),
+                                                   ptr(mlp_dist.b[2]), ptr(actv), ptr(x_v), ptr(res_a), ptr(res_v), ptr(out_a),
+                                                   ptr(out_v), ptr(edge_counter), ptr(tc_status(x_v.device)), stream_ptr(x_v.device)))
+        return out_a, out_v
     with KERNEL_TIMER.region("painn_message"):
         check(lib().ld_painn_message_f32(ptr(row_ptr), ptr(dst), ptr(rij), Nt, n, n_rbf, radial_kind, float(rmax), float(eps),
                                          ptr(mlp_dist.Wt[0]), ptr(mlp_dist.b[0]), ptr(mlp_dist.Wt[1]), ptr(mlp_dist.b[1]),

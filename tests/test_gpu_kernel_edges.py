@@ -49,3 +49,59 @@ def test_bee_products_tails(rows, chan):
             m = b.abs() + 2 * (t[1] if k == 11 else t[2]).double().abs().amax(-1, keepdim=True) * t[4].double().abs().amax(-1).reshape(
                 rows, chan, *[1] * (k - 10))
         assert bool(((a.cpu().double() - b).abs() <= 10 * U * m).all()), k
+
+
+def _message64(row_ptr, dst, rij, weights, actv, x_v, radial, n_rbf, rmax):
+    from oracle import reference_math as R
+    (W1, b1), (W2, b2), (W3, b3) = [(W.double(), b.double()) for W, b in weights]
+    n = x_v.shape[1]
+    r = rij.double()
+    h = (R.radial_encode_painn if radial == 0 else R.radial_encode_gaussian)(r, n_rbf, rmax)
+    silu = torch.nn.functional.silu
+    P = (silu(silu(h @ W1.t() + b1) @ W2.t() + b2) @ W3.t() + b3) * actv.double()[dst.long()]
+    u = (r / torch.sqrt(0.1 + (r ** 2).sum(-1, keepdim=True)))[:, None]
+    xe = x_v.double()[dst.long()]
+    m = xe * P[:, :n, None] + torch.linalg.cross(xe, u.expand_as(xe)) * P[:, n:2 * n, None] + u * P[:, 2 * n:3 * n, None]
+    src = torch.repeat_interleave(torch.arange(len(row_ptr) - 1), (row_ptr[1:] - row_ptr[:-1]).long())
+    zeros = torch.zeros(x_v.shape, dtype=torch.float64)
+    return zeros[..., 0].index_add(0, src, P[:, 3 * n:]), zeros.index_add(0, src, m)
+
+
+# tiles hold 256, 128 or 64 edges (n = 32, 64, 128), slabs K = 32: nodes without edges, nodes that span tiles, a last tile
+# with one edge, input widths around the slab; weights far from 1 move the operands' scales
+@pytest.mark.parametrize("n,n_rbf,radial,degrees,wscale", [
+    (32, 1, 1, "one", 1.0), (32, 20, 1, "mixed", 1.0), (32, 128, 0, "long", 1.0), (64, 16, 1, "long", 30.0), (64, 64, 0, "mixed", 1.0),
+    (128, 8, 1, "mixed", 1.0), (128, 33, 0, "long", 1e-3), (128, 16, 1, "none", 1.0)])
+def test_split_message_is_as_exact_as_the_fma_kernel(n, n_rbf, radial, degrees, wscale):
+    """the two kernels against 64 bits: the split form may not be further off than the FP32 FMAs are (plus one rounding)"""
+    import ctypes
+    from ld_b200 import ops
+    from ld_b200._lib import lib, check, ptr, stream_ptr
+    g = torch.Generator().manual_seed(n + n_rbf)
+    deg = {"one": torch.tensor([0, 0, 1, 0]), "none": torch.zeros(5, dtype=torch.int64),
+           "mixed": torch.randint(0, 40, (61,), generator=g), "long": torch.tensor([3, 0, 700, 1, 0, 0, 64, 257, 129, 1])}[degrees]
+    Nt, E = len(deg), int(deg.sum())
+    row_ptr = torch.cat([torch.zeros(1, dtype=torch.int64), deg.cumsum(0)]).int()
+    dst = torch.randint(0, Nt, (E,), generator=g).int()
+    rmax = 4.0
+    rij = torch.randn(E, 3, generator=g) * 1.3
+    lin = [torch.nn.Linear(k, 4 * n) for k in (n_rbf, 4 * n, 4 * n)]
+    with torch.no_grad():
+        for l in lin:
+            l.weight.copy_((torch.rand(l.weight.shape, generator=g) * 2 - 1) * l.weight.shape[1] ** -0.5 * wscale)
+            l.bias.copy_((torch.rand(l.bias.shape, generator=g) * 2 - 1) * l.weight.shape[1] ** -0.5)
+    actv, x_v = torch.randn(Nt, 4 * n, generator=g), torch.randn(Nt, n, 3, generator=g)
+    want = _message64(row_ptr, dst, rij, [(l.weight.detach(), l.bias.detach()) for l in lin], actv, x_v, radial, n_rbf, rmax)
+    mlp = ops.PackedMLP([l.cuda() for l in lin])
+    args = [t.cuda() for t in (row_ptr, dst, rij)]
+    actv, x_v = actv.cuda(), x_v.cuda()
+    count = torch.zeros(1, dtype=torch.int64, device="cuda")
+    split = ops.painn_message_f32(*args, mlp, actv, x_v, rmax, radial_kind=radial, edge_counter=count)
+    assert mlp._split and int(count) == E and int(ops.tc_status(actv.device)) == 0
+    fma = torch.empty(Nt, n, device="cuda"), torch.empty(Nt, n, 3, device="cuda")
+    check(lib().ld_painn_message_f32(*[ptr(a) for a in args], Nt, n, n_rbf, radial, ctypes.c_float(rmax), ctypes.c_float(0.1), ptr(mlp.Wt[0]),
+                                     ptr(mlp.b[0]), ptr(mlp.Wt[1]), ptr(mlp.b[1]), ptr(mlp.Wt[2]), ptr(mlp.b[2]), ptr(actv), ptr(x_v), None,
+                                     None, ptr(fma[0]), ptr(fma[1]), None, stream_ptr()))
+    for w, a, b in zip(want, split, fma):
+        off = lambda t: float((t.cpu().double() - w).norm())  # noqa: E731
+        assert off(a) <= 1.2 * off(b) + U * float(w.norm()), (off(a) / float(w.norm()), off(b) / float(w.norm()))
