@@ -4,15 +4,15 @@
 // What bounds it: the shared-memory port. The two 4n x 4n layers are 3 x 2 x (4n)^2 flops an edge on the tensor cores; an MMA
 // of 128 x 64 x 16 (n = 128) takes 48 cycles, the time to read its 6 KB of operands, not the 32 of the tensor pipe, and the
 // weight slabs (2 MB per tile) come in through the same port: 433 cycles a slab of six MMAs measured, 416 by that count.
-// n = 128, 8 radial functions, 562 k edges: 3.04 ms, against 22.8 ms on the FMA pipe (painn_message.cu); n = 64, 11 k edges:
-// 61 us against 195. Error against 64 bits: 6.1e-7, against 7.5e-7.
+// n = 128, 8 radial functions, 562 k edges: 2.97 ms, against 22.8 ms on the FMA pipe (painn_message.cu); n = 64, 11 k edges:
+// 68 us against 195. Error against 64 bits: 6.1e-7, against 7.5e-7.
 //
 // A block owns a node-aligned, contiguous slice of the CSR and walks it 256 / (n / 32) edges at a time. Roles:
 //   * 16 working warps: geometry, radial features -> activation planes in shared memory; per layer each thread adds the
 //     partial sums of its channel (64 edges) from tensor memory into registers, then writes bias + SiLU back as the next
-//     layer's planes; after the last layer the product with the neighbour's activation goes to shared memory in FP32 and
-//     is turned into messages and per-node sums, 16 edges per thread, joined in edge order (no atomics, fixed order, every
-//     node written once).
+//     layer's planes; the last layer goes to shared memory in FP32, is turned into messages (16 edges of a channel per
+//     thread) and summed per node in edge order (no atomics; every node written once; the same bits wherever a node's
+//     edges fall in a tile).
 //   * 2 MMA warps and 1 producer warp (lane 0 of each): six MMAs per 16 KB weight slab; slabs stream through a ring.
 // Every wait is bounded (LD_FLAG_TIMEOUT): a failed wait is OR-ed into the next block barrier so that all threads leave
 // together.
@@ -22,14 +22,8 @@
 
 namespace {
 
-constexpr int WORK_WARPS = 16, WORK_THREADS = WORK_WARPS * 32;
-// Two issuing warps take the slabs in turn: a poll of a barrier costs about 220 cycles in the issuing thread even when the
-// barrier is ready, and no MMA of that thread is queued meanwhile (one 288-cycle slab per poll: 532 cycles a slab measured);
-// with two threads one polls while the other's MMAs run. A slab's accumulator belongs to one thread, so its order is fixed.
-constexpr int MMA_WARPS = 2, MMA_WARP = WORK_WARPS, PROD_WARP = WORK_WARPS + MMA_WARPS;
-constexpr int THREADS = (WORK_WARPS + MMA_WARPS + 1) * 32;
-constexpr int SYNC_THREADS = (WORK_WARPS + MMA_WARPS) * 32;   // working and MMA warps meet at barrier 1
-constexpr int STAGES = 5;                             // weight slabs in the ring
+using namespace sf;
+
 constexpr int EPT = 16;                               // edges per thread in the message phase
 
 // MB: blocks of 128 channels; n = 32 MB
@@ -59,45 +53,6 @@ struct SplitParams {
   long long* edge_counter;
   int* status;
 };
-
-__device__ __forceinline__ int work_lower_bound(const int* __restrict__ row_ptr, int lo, int hi, long long target) {
-  const long long base = (long long)row_ptr[lo] + lo;
-  while (lo < hi) {
-    const int mid = (lo + hi) >> 1;
-    if ((long long)row_ptr[mid] + mid - base < target) lo = mid + 1; else hi = mid;
-  }
-  return lo;
-}
-
-struct BlockRange { int n_begin, n_end; long long e_begin, e_end, ntiles; };
-
-// node-aligned share of segment [lo, hi) for this block, balanced over edges + nodes
-__device__ __forceinline__ BlockRange block_range(const int* __restrict__ row_ptr, int lo, int hi, int tile) {
-  BlockRange r;
-  const long long work = ((long long)row_ptr[hi] - row_ptr[lo]) + (hi - lo);
-  long long per = (work + gridDim.x - 1) / gridDim.x;
-  if (per < tile) per = tile;
-  r.n_begin = blockIdx.x == 0 ? lo : work_lower_bound(row_ptr, lo, hi, per * blockIdx.x);
-  r.n_end = blockIdx.x == gridDim.x - 1 ? hi : work_lower_bound(row_ptr, lo, hi, per * (blockIdx.x + 1));
-  r.e_begin = r.n_begin < r.n_end ? row_ptr[r.n_begin] : 0;
-  r.e_end = r.n_begin < r.n_end ? row_ptr[r.n_end] : 0;
-  r.ntiles = (r.e_end - r.e_begin + tile - 1) / tile;
-  return r;
-}
-
-// barrier 1: working warps + MMA warps; returns the OR of `flag` over its participants
-__device__ __forceinline__ int sync_or(int flag) {
-  int out;
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t"
-      "setp.ne.u32 q, %1, 0;\n\t"
-      "barrier.cta.red.or.pred p, 1, %2, q;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(out) : "r"(flag), "n"(SYNC_THREADS) : "memory");
-  return out;
-}
-// barrier 2: working warps only
-__device__ __forceinline__ void sync_workers() { asm volatile("barrier.cta.sync 2, %0;" ::"n"(WORK_THREADS) : "memory"); }
 
 // the two factors of a Gaussian radial feature (radial_feature, kind 1), the envelope once per edge
 __device__ __forceinline__ float radial_envelope(float d, float rmax) {
@@ -178,9 +133,9 @@ painn_message_split_kernel(const __grid_constant__ SplitParams P) {
     // reports both that the partial sum is complete and that the ring stage is free
     const uint32_t me = warp - MMA_WARP;
     uint32_t chunks = 0, st = me, full_phase = 0;
-    const uint64_t b1 = tc::smem_desc(tc::smem_u32(act), S::PANEL, 128), b2 = tc::smem_desc(tc::smem_u32(act + S::PLANE), S::PANEL, 128);
-    const uint64_t a0 = tc::smem_desc(tc::smem_u32(ring), 128 * 16, 128);
-    constexpr uint64_t b_step = (2 * S::PANEL) >> 4, st_step = sf::SLAB_BYTES >> 4;
+    const uint32_t b1 = desc_lo(act, S::PANEL), b2 = desc_lo(act + S::PLANE, S::PANEL);
+    const uint32_t a0 = desc_lo(ring, 128 * 16);
+    constexpr uint32_t b_step = (2 * S::PANEL) >> 4, st_step = sf::SLAB_BYTES >> 4;
     constexpr uint32_t idesc = sf::idesc_f16(128, NE);
     for (int seg_lo = 0; seg_lo < P.Nt && !fail; seg_lo += seg_nodes) {
       const long long ntiles = block_range(P.row_ptr, seg_lo, min(seg_lo + seg_nodes, P.Nt), NE).ntiles;
@@ -190,7 +145,7 @@ painn_message_split_kernel(const __grid_constant__ SplitParams P) {
           if (sync_or(fail)) { fail = 1; break; }    // [X] this layer's activations are written
           if (lane == 0) {
             const int K = layer == 0 ? P.k0p : N;
-            uint64_t x1 = b1, x2 = b2;
+            uint32_t x1 = b1, x2 = b2;
             for (int k0 = 0; k0 < K && !fail; k0 += sf::SLAB_K, chunks++, x1 += 2 * b_step, x2 += 2 * b_step) {
               const uint32_t ks = K - k0 > 16 ? 2 : 1;
               if (MB == 1 && (chunks & 1) != me) continue;
@@ -228,26 +183,25 @@ painn_message_split_kernel(const __grid_constant__ SplitParams P) {
     for (int seg_lo = 0; seg_lo < P.Nt && !fail; seg_lo += seg_nodes) {
       const BlockRange br = block_range(P.row_ptr, seg_lo, min(seg_lo + seg_nodes, P.Nt), NE);
       const int n_begin = br.n_begin, n_end = br.n_end;
-      float carry = 0.f;          // thread tid < 4n: sum of output (component tid / n, channel tid % n) of node `cur`
+      float carry = 0.f;          // thread tid < N: sum of output (component tid / n, channel tid % n) of node `cur`
       int cur = n_begin;
       int node_lo = n_begin;      // source node of the next tile's first edge (or an earlier one)
       sync_workers();             // the previous segment's last readers of s_rowwin are done
       for (int i = tid; i <= NE; i += WORK_THREADS) s_rowwin[i] = P.row_ptr[min(node_lo + i, n_end > n_begin ? n_end : n_begin)];
       sync_workers();
 
-      auto write_out = [&](int v, int c, int k, float val) {
-        if (k < 3) {
-          const size_t off = ((size_t)v * n + c) * 3 + k;
-          P.out_v[off] = P.res_v != nullptr ? val + P.res_v[off] : val;
-        } else {
-          const size_t off = (size_t)v * n + c;
-          P.out_a[off] = P.res_a != nullptr ? val + P.res_a[off] : val;
-        }
-      };
       // output of node `from`, zeros for the nodes (from, next)
       auto flush_until = [&](int from, int next, float val) {
-        if (tid < 4 * n)
-          for (int v = from; v < next; v++) write_out(v, mc, mg, v == from ? val : 0.f);
+        if (tid >= N) return;
+        for (int v = from; v < next; v++, val = 0.f) {
+          if (mg < 3) {
+            const size_t off = ((size_t)v * n + mc) * 3 + mg;
+            P.out_v[off] = P.res_v != nullptr ? val + P.res_v[off] : val;
+          } else {
+            const size_t off = (size_t)v * n + mc;
+            P.out_a[off] = P.res_a != nullptr ? val + P.res_a[off] : val;
+          }
+        }
       };
 
       for (long long e0 = br.e_begin; e0 < br.e_end; e0 += NE) {
@@ -340,90 +294,62 @@ painn_message_split_kernel(const __grid_constant__ SplitParams P) {
           }
         }
         if (fail) break;
-        const int tile_cur = cur;
         node_lo = s_src[cnt - 1];
         for (int i = tid; i <= NE; i += WORK_THREADS) s_rowwin[i] = P.row_ptr[min(node_lo + i, n_end)];   // for the next tile
         sync_workers();
-        // ---- messages of channel mc, edges [EPT mg, EPT mg + EPT): the sum for the group's first node is its head, for its
-        // last node (when different) its tail; nodes strictly inside are complete and written at once -------------------
-        float head[4], sum[4];
-        bool first = true;
+        // ---- messages of channel mc, edges [EPT mg, EPT mg + EPT), in the place of the products they are made of ------------
         {
           const int r_lo = mg * EPT, r_hi = min(r_lo + EPT, cnt);
+          float* pc = prod + mc * (NE + 1);
+          for (int eb = r_lo; eb < r_hi; eb += 4) {
+            // what four edges take from their neighbours: 28 loads in flight (slots past cnt hold node 0)
+            float x[4][3], a[4][4];
 #pragma unroll
-          for (int k = 0; k < 4; k++) head[k] = sum[k] = 0.f;
-          if (r_lo < r_hi) {
-            int c_node = s_src[r_lo];
-            const float* pc = prod + mc * (NE + 1);
-            for (int eb = r_lo; eb < r_hi; eb += 4) {
-              // what four edges take from their neighbours: 28 loads in flight
-              float x[4][3], a[4][4];
+            for (int i = 0; i < 4; i++) {
+              const size_t j = s_dst[eb + i];
+              const float* xp = P.x_v + (j * n + mc) * 3;
+              const float* ap = P.actv + j * N + mc;
 #pragma unroll
-              for (int i = 0; i < 4; i++) {
-                const size_t j = s_dst[eb + i];   // slots past cnt hold node 0
-                const float* xp = P.x_v + (j * n + mc) * 3;
-                const float* ap = P.actv + j * N + mc;
+              for (int k = 0; k < 3; k++) x[i][k] = __ldg(xp + k);
 #pragma unroll
-                for (int k = 0; k < 3; k++) x[i][k] = __ldg(xp + k);
+              for (int k = 0; k < 4; k++) a[i][k] = __ldg(ap + k * n);
+            }
 #pragma unroll
-                for (int k = 0; k < 4; k++) a[i][k] = __ldg(ap + k * n);
-              }
-#pragma unroll
-              for (int i = 0; i < 4; i++) {
-                const int e = eb + i;
-                if (e < r_hi) {
-                  const int s = s_src[e];
-                  if (s != c_node) {
-                    if (first) {
-#pragma unroll
-                      for (int k = 0; k < 4; k++) head[k] = sum[k];
-                      first = false;
-                    } else {
-#pragma unroll
-                      for (int k = 0; k < 4; k++) write_out(c_node, mc, k, sum[k]);
-                    }
-                    for (int z = c_node + 1; z < s; z++)   // nodes without edges
-#pragma unroll
-                      for (int k = 0; k < 4; k++) write_out(z, mc, k, 0.f);
-#pragma unroll
-                    for (int k = 0; k < 4; k++) sum[k] = 0.f;
-                    c_node = s;
-                  }
-                  const float p0 = pc[e] * a[i][0], p1 = pc[n * (NE + 1) + e] * a[i][1], p2 = pc[2 * n * (NE + 1) + e] * a[i][2];
-                  const float d0 = s_dir[e][0], d1 = s_dir[e][1], d2 = s_dir[e][2];
-                  sum[0] += x[i][0] * p0 + (x[i][1] * d2 - x[i][2] * d1) * p1 + d0 * p2;
-                  sum[1] += x[i][1] * p0 + (x[i][2] * d0 - x[i][0] * d2) * p1 + d1 * p2;
-                  sum[2] += x[i][2] * p0 + (x[i][0] * d1 - x[i][1] * d0) * p1 + d2 * p2;
-                  sum[3] += pc[3 * n * (NE + 1) + e] * a[i][3];
-                }
-              }
+            for (int i = 0; i < 4; i++) {
+              const int e = eb + i;
+              const float p0 = pc[e] * a[i][0], p1 = pc[n * (NE + 1) + e] * a[i][1], p2 = pc[2 * n * (NE + 1) + e] * a[i][2];
+              const float d0 = s_dir[e][0], d1 = s_dir[e][1], d2 = s_dir[e][2];
+              pc[e] = x[i][0] * p0 + (x[i][1] * d2 - x[i][2] * d1) * p1 + d0 * p2;
+              pc[n * (NE + 1) + e] = x[i][1] * p0 + (x[i][2] * d0 - x[i][0] * d2) * p1 + d1 * p2;
+              pc[2 * n * (NE + 1) + e] = x[i][2] * p0 + (x[i][0] * d1 - x[i][1] * d0) * p1 + d2 * p2;
+              pc[3 * n * (NE + 1) + e] *= a[i][3];
             }
           }
-        }
-        sync_workers();   // the products have been read: their place takes the heads and tails
-        float* s_head = prod;
-        float* s_tail = prod + 4 * WORK_THREADS;
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-          s_head[(mg * 4 + k) * n + mc] = first ? sum[k] : head[k];
-          s_tail[(mg * 4 + k) * n + mc] = first ? 0.f : sum[k];
         }
         sync_workers();
-        // ---- the groups in edge order, with the sum carried over from earlier tiles: thread = (component, channel) --------
-        if (tid < 4 * n) {
-          int c_node = tile_cur;
-          float a = carry;
-          for (int g = 0; g < S::G && g * EPT < cnt; g++) {
-            const int f = s_src[g * EPT], l = s_src[min(g * EPT + EPT, cnt) - 1];
-            if (f != c_node) { flush_until(c_node, f, a); a = 0.f; c_node = f; }
-            a += s_head[g * 4 * n + tid];
-            if (l != f) {
-              flush_until(f, f + 1, a);   // node f alone: the gaps after it were filled by the group's thread
-              a = s_tail[g * 4 * n + tid];
-              c_node = l;
+        // ---- per-node sums, thread = (component, channel): one edge after the other, so that a node's sum does not depend on
+        // where its edges fall in a tile or a block ----------------------------------------------------------------------
+        if (tid < N) {
+          const float* m = prod + tid * (NE + 1);
+          int c_node = cur;
+          for (int eb = 0; eb < cnt; eb += 8) {
+            float v[8];
+#pragma unroll
+            for (int i = 0; i < 8; i++) v[i] = m[eb + i];
+            const int last = min(eb + 8, cnt) - 1;
+            if (s_src[last] == c_node && last == eb + 7) {
+#pragma unroll
+              for (int i = 0; i < 8; i++) carry += v[i];
+            } else {
+#pragma unroll
+              for (int i = 0; i < 8; i++)
+                if (eb + i < cnt) {
+                  const int s = s_src[eb + i];
+                  if (s != c_node) { flush_until(c_node, s, carry); carry = 0.f; c_node = s; }
+                  carry += v[i];
+                }
             }
           }
-          carry = a;
         }
         cur = node_lo;
         sync_workers();   // geometry and planes are rewritten by the next tile
