@@ -249,6 +249,19 @@ int ld_bee_messages_scalar_f32(const int* row_ptr, const int* dst, const float* 
                                const float* jacobi, const float* Yt, const float* W1t, const float* b1, const float* W2t,
                                const float* b2, const float* W3t, const float* b3, const float* Wdt, float scale,
                                float* out_a, void* stream);
+/* The same at the same accuracy for chan and dim_a 64 or 128, with the per-edge linear maps on the FP16 tensor cores, every
+ * operand the sum of two FP16 values. ld_bee_split_elems: FP16 values that ld_bee_split_pack writes (0: no such form);
+ * scales: ten floats, written by it as well. ld_bee_rows13_f32: the neighbour rows [rows][13][chan] that it reads
+ * (ld_bee_messages_vd_f32 takes them with feat_bf16 = 3). */
+int ld_bee_split_elems(int chan, int dim_a, long long* elems);
+int ld_bee_split_pack(const float* Yt, const float* W1t, const float* b1, const float* W2t, const float* b2, const float* W3t,
+                      const float* Wdt, int chan, int dim_a, void* packed_f16, float* scales, void* stream);
+int ld_bee_rows13_f32(const float* l0, const float* l1, const float* l2, long long rows, int chan, float* rows13, void* stream);
+int ld_bee_messages_scalar_f32_split(const int* row_ptr, const int* dst, const float* rij, int Nt, int chan, int dim_a, float r0,
+                                     const float* rows13, const float* enc_w, const float* enc_b, const float* jacobi,
+                                     const void* packed_f16, const float* scales, const float* b1, const float* b2, const float* b3,
+                                     float scale, float* out_a, int* status_dev, void* stream);
+
 
 /* Tensor-core variant of ld_bee_messages_scalar_f32 (tcgen05, BF16 operands, 2e-2 relative); weights
  * packed by ld_pack_weights_bf16: Yp [a][3*chan], W1p [2a][a], W2p [2a][2a], W3p [a][3a] = (W3 | W_direct + I). */

@@ -18,6 +18,7 @@
 #include "common.cuh"
 #include "mlp_tile.cuh"
 #include "tp_math.h"
+#include "bee_edge.cuh"
 #include <cuda_bf16.h>
 #include "tc05.cuh"
 
@@ -60,22 +61,6 @@ __device__ __forceinline__ void bm_block_range(const int* __restrict__ row_ptr, 
   *n_end = blockIdx.x == gridDim.x - 1 ? hi : bm_work_lower_bound(row_ptr, lo, hi, per * (blockIdx.x + 1));
 }
 
-// per-edge geometry shared by all channels: rhat[3] and the eight radial features
-struct __align__(16) EdgeGeom { float enc[8]; float rhat[3]; float pad; };   // 48 bytes: three 16-byte shared-memory loads
-
-__device__ __forceinline__ void edge_geometry(const float* __restrict__ rij, long long e, float r0,
-                                              const float* __restrict__ jac, EdgeGeom* g) {
-  const float x = rij[e * 3], y = rij[e * 3 + 1], z = rij[e * 3 + 2];
-  const float d = sqrtf(x * x + y * y + z * z);
-  const float zz = d / r0;
-  const float env = fmaxf(1.f - zz, 0.f);
-  ld_radial_cheb8(zz, env, jac, g->enc);
-  const float s = 7.f / r0;
-  const float ux = x * s, uy = y * s, uz = z * s;
-  const float inv = 1.0f / sqrtf(1.f + ux * ux + uy * uy + uz * uz);
-  g->rhat[0] = ux * inv; g->rhat[1] = uy * inv; g->rhat[2] = uz * inv;
-}
-
 // the right-hand operands of one channel: phi_a scalar, phi_v = phi_a rhat, phi_d = phi_a rhat rhat^T
 __device__ __forceinline__ void edge_phi(const EdgeGeom& g, const float* w8, float bias, float* pa, float* pv, float* pd) {
   float a = bias;
@@ -95,11 +80,13 @@ __device__ __forceinline__ void edge_phi(const EdgeGeom& g, const float* w8, flo
 // S_v[node][k][c][3], k over (011,101,121,211,111); S_d[node][k][c][9], k over (022,202,112,222,212):
 // the layouts a channel mixing with 5*chan inputs expects. Thread = channel; a block walks its nodes
 // and stages the geometry of up to 32 edges at a time in shared memory.
-// CC: the channel count as a compile-time constant (0: taken from the parameters)
-template <typename FT, bool PACKED, int CC>
+// CC: the channel count as a compile-time constant (0: taken from the parameters). PACKED: BF16 rows [node][chan][16].
+// ROWS13: FP32 rows [node][13][chan], so that a warp's loads are consecutive addresses (219 k edges, 128 channels: 180 us
+// with the strided loads of the separate rank-1 and rank-2 features, 152 us so).
+template <typename FT, bool PACKED, int CC, bool ROWS13 = false>
 __global__ void __launch_bounds__(128, 4)   // four blocks per SM: at most 128 registers
 bee_vd_kernel(BeeEdgeParams P, float* __restrict__ S_v, float* __restrict__ S_d, float scale, int out_bf16_) {
-  const int out_bf16 = CC > 0 ? 1 : out_bf16_;   // the instance with a constant width is the tensor-core path's: BF16 sums
+  const int out_bf16 = ROWS13 ? 0 : CC > 0 ? 1 : out_bf16_;   // the BF16 instance with a constant width is the tensor-core path's: BF16 sums
   const FT* __restrict__ F0 = reinterpret_cast<const FT*>(P.L0);
   const FT* __restrict__ F1 = reinterpret_cast<const FT*>(P.L1);
   const FT* __restrict__ F2 = reinterpret_cast<const FT*>(P.L2);
@@ -151,7 +138,7 @@ bee_vd_kernel(BeeEdgeParams P, float* __restrict__ S_v, float* __restrict__ S_d,
       for (int eb = e_lo; eb < e_hi; eb += BV_TILE) {
         const int cnt = min(BV_TILE, e_hi - eb);
         __syncthreads();  // previous tile's readers are done
-        constexpr int UNR = 4;  // neighbour rows in flight per thread
+        constexpr int UNR = ROWS13 ? 2 : 4;  // neighbour rows in flight per thread
         // the edge list of the step is padded to whole batches with edges of weight zero (they read the row of the
         // step's first neighbour), so that the batches below need neither bounds checks nor clamped indices
         const int cnt_pad = (cnt + UNR - 1) & ~(UNR - 1);
@@ -171,6 +158,15 @@ bee_vd_kernel(BeeEdgeParams P, float* __restrict__ S_v, float* __restrict__ S_d,
         if (cok) {
           for (int tb = 0; tb < cnt_pad; tb += UNR) {
             uint32_t raw[UNR][8];
+            float row[UNR][13];
+            if (ROWS13) {
+#pragma unroll
+              for (int u = 0; u < UNR; u++) {
+                const FT* f = F0 + (size_t)s_dst[tb + u] * 13 * C + c;
+#pragma unroll
+                for (int k = 0; k < 13; k++) row[u][k] = bm_ld(f, k * C);
+              }
+            }
             if (PACKED) {
 #pragma unroll
               for (int u = 0; u < UNR; u++)
@@ -188,6 +184,12 @@ bee_vd_kernel(BeeEdgeParams P, float* __restrict__ S_v, float* __restrict__ S_d,
                 for (int k = 0; k < 3; k++) l1[k] = tc::bf16_at(raw[u], 1 + k);
 #pragma unroll
                 for (int k = 0; k < 9; k++) l2[k] = tc::bf16_at(raw[u], 4 + k);
+              } else if (ROWS13) {
+                l0 = row[u][0];
+#pragma unroll
+                for (int k = 0; k < 3; k++) l1[k] = row[u][1 + k];
+#pragma unroll
+                for (int k = 0; k < 9; k++) l2[k] = row[u][4 + k];
               } else {
                 l0 = bm_ld(F0, j);
 #pragma unroll
@@ -393,7 +395,8 @@ bee_scalar_kernel(BeeScalarParams P) {
 // Per-node sums of the ten rank-1 / rank-2 Bee products of a Messages layer, times `scale`.
 // S_v: [Nt, 5*chan, 3] (product order 011,101,121,211,111), S_d: [Nt, 5*chan, 3, 3] (022,202,112,222,212).
 // L0/L1/L2 are the node-level left operands: FP32 (feat_bf16 = 0), BF16 (1), or with feat_bf16 = 2
-// L0 alone points to the interleaved BF16 form [node][chan][16] = (l0, l1[3], l2[9], 3 unused); enc_w [chan,8] / enc_b [chan] the radial read-in,
+// L0 alone points to the interleaved BF16 form [node][chan][16] = (l0, l1[3], l2[9], 3 unused), with 3 to the FP32 rows
+// [node][13][chan] of ld_bee_rows13_f32; enc_w [chan,8] / enc_b [chan] the radial read-in,
 // jacobi the 8x9 coefficient matrix of the radial basis. Graph in CSR form sorted by source.
 // out_bf16: S_v / S_d are stored as BF16, component-major ([Nt][3][5*chan] and [Nt][9][5*chan]), the input form of
 // ld_linear_bf16_tc_in16.
@@ -413,7 +416,9 @@ extern "C" int ld_bee_messages_vd_f32(const int* row_ptr, const int* dst, const 
   BeeEdgeParams P{row_ptr, dst, rij, Nt, chan, r0, L0, L1, L2, enc_w, enc_b, jacobi, 0, next_node};
   int dev = 0, sms = 148;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (feat_bf16 == 2 && chan == 128 && out_bf16) bee_vd_kernel<__nv_bfloat16, true, 128><<<sms * 4, 128, 0, (cudaStream_t)stream>>>(P, S_v, S_d, scale, 1);
+  if (feat_bf16 == 3 && chan == 128) bee_vd_kernel<float, false, 128, true><<<sms * 4, 128, 0, (cudaStream_t)stream>>>(P, S_v, S_d, scale, 0);
+  else if (feat_bf16 == 3) bee_vd_kernel<float, false, 0, true><<<sms * 4, 128, 0, (cudaStream_t)stream>>>(P, S_v, S_d, scale, 0);
+  else if (feat_bf16 == 2 && chan == 128 && out_bf16) bee_vd_kernel<__nv_bfloat16, true, 128><<<sms * 4, 128, 0, (cudaStream_t)stream>>>(P, S_v, S_d, scale, 1);
   else if (feat_bf16 == 2) bee_vd_kernel<__nv_bfloat16, true, 0><<<sms * 4, 128, 0, (cudaStream_t)stream>>>(P, S_v, S_d, scale, out_bf16);
   else if (feat_bf16) bee_vd_kernel<__nv_bfloat16, false, 0><<<sms * 4, 128, 0, (cudaStream_t)stream>>>(P, S_v, S_d, scale, out_bf16);
   else bee_vd_kernel<float, false, 0><<<sms * 4, 128, 0, (cudaStream_t)stream>>>(P, S_v, S_d, scale, out_bf16);

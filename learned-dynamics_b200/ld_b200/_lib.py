@@ -67,6 +67,10 @@ SIGNATURES = {
     "ld_bee_left_rows_bf16_tc": [P, P, P, LL, I, I, I, I, P, P, P, P, P, P],
     "ld_bee_messages_vd_bf16_tc": [P, P, P, I, I, F, P, P, P, P, F, P, P, P, P],
     "ld_bee_messages_scalar_f32": [P, P, P, I, I, I, F, P, P, P, P, P, P, P, P, P, P, P, P, P, P, F, P, P],
+    "ld_bee_split_elems": [I, I, P],
+    "ld_bee_split_pack": [P, P, P, P, P, P, P, I, I, P, P, P],
+    "ld_bee_rows13_f32": [P, P, P, LL, I, P, P],
+    "ld_bee_messages_scalar_f32_split": [P, P, P, I, I, I, F, P, P, P, P, P, P, P, P, P, F, P, P, P],
     "ld_painn_split_elems": [I, I, P],
     "ld_painn_split_pack": [P, P, P, P, P, I, I, P, P, P],
     "ld_painn_message_f32_split": [P, P, P, I, I, I, I, F, F, P, P, P, P, P, P, P, P, P, P, P, P, P, P],

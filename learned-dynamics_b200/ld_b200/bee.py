@@ -7,6 +7,7 @@ runs as: three node-level channel mixings (L0, L1, L2), one pass over the edges 
 products summed per node, one pass for the scalar channel (per-edge Y maps + mlp_a), and two
 node-level channel mixings for the hoisted Y maps. With autograd it runs the reference's op
 sequence on this library's Bee / TensLinear / gather / segment-sum functions."""
+import ctypes
 from math import comb
 
 import torch
@@ -125,6 +126,16 @@ class Messages(nn.Module):
                 "W1t": f(lay[0].weight.t()), "b1": f(lay[0].bias), "W2t": f(lay[2].weight.t()), "b2": f(lay[2].bias),
                 "W3t": f(lay[4].weight.t()), "b3": f(lay[4].bias), "Wdt": f(self.mlp_a.lin_direct.weight.t()),
             }
+            if self.precision != "bf16":
+                # the scalar channel's per-edge maps as sums of two FP16 values (widths 64 and 128)
+                p, elems = self._packed, ctypes.c_longlong(0)
+                check(lib().ld_bee_split_elems(self.chan, self.dim_a, ctypes.byref(elems)))
+                if elems.value > 0 and dev.type == "cuda":
+                    p["split"] = torch.empty(elems.value, dtype=torch.float16, device=dev)
+                    p["split_scales"] = torch.empty(10, dtype=torch.float32, device=dev)
+                    check(lib().ld_bee_split_pack(ptr(p["Yt"]), ptr(p["W1t"]), ptr(p["b1"]), ptr(p["W2t"]), ptr(p["b2"]), ptr(p["W3t"]),
+                                                  ptr(p["Wdt"]), self.chan, self.dim_a, ptr(p["split"]), ptr(p["split_scales"]),
+                                                  stream_ptr(dev)))
             if self.precision == "bf16":
                 eye = torch.eye(self.dim_a, device=dev)
                 p = self._packed
@@ -238,6 +249,11 @@ class Messages(nn.Module):
             l0 = self.L0(x_a.reshape(Nt, -1))
             l1 = self.L1(x_v.reshape(Nt, -1, 3))
             l2 = self.L2(x_d.reshape(Nt, -1, 3, 3))
+            if "split" in w:
+                # both edge kernels read the neighbours' rows component-major, [node][13][chan]
+                rows13 = torch.empty(Nt, 13, C, dtype=torch.float32, device=dev)
+                check(lib().ld_bee_rows13_f32(ptr(l0), ptr(l1), ptr(l2), Nt, C, ptr(rows13), stream_ptr(dev)))
+                l0 = l1 = l2 = rows13
         rij = r_ij.contiguous()
         # the per-node product sums feed tensor-core channel mixings on the bf16 path, which round them to BF16 anyway
         sums16 = self.precision == "bf16" and self.dim_v % 32 == 0 and self.dim_d % 32 == 0
@@ -256,7 +272,7 @@ class Messages(nn.Module):
             with KERNEL_TIMER.region("bee_messages_vd"):
                 check(lib().ld_bee_messages_vd_f32(ptr(graph.row_ptr), ptr(graph.dst32), ptr(rij), Nt, C, float(self.r0), ptr(l0),
                                                    ptr(l1), ptr(l2), ptr(w["enc_w"]), ptr(w["enc_b"]), ptr(w["jac"]), 0.1,
-                                                   ptr(S_v), ptr(S_d), 2 if feat16 else 0, 1 if sums16 else 0, st))
+                                                   ptr(S_v), ptr(S_d), 2 if feat16 else 3 if "split" in w else 0, 1 if sums16 else 0, st))
         # the residual form: the rank-1 and rank-2 adds happen in the epilogues of the two Y maps (the scalar edge kernel
         # writes a node's row on its critical path, where a load of the residual cost more than the separate add)
         fuse_add = (add_input and self.precision == "bf16" and sums16 and all(t.dtype == torch.float32 for t in (x_a, x_v, x_d)))
@@ -269,6 +285,12 @@ class Messages(nn.Module):
                                                            2 if feat16 else 0, ptr(ops.tc_status(dev)), st))
             if fuse_add:
                 B_a += x_a.reshape(Nt, -1)
+        elif "split" in w:
+            with KERNEL_TIMER.region("bee_messages_scalar"):
+                check(lib().ld_bee_messages_scalar_f32_split(ptr(graph.row_ptr), ptr(graph.dst32), ptr(rij), Nt, C, self.dim_a,
+                                                             float(self.r0), ptr(l0), ptr(w["enc_w"]), ptr(w["enc_b"]), ptr(w["jac"]),
+                                                             ptr(w["split"]), ptr(w["split_scales"]), ptr(w["b1"]), ptr(w["b2"]),
+                                                             ptr(w["b3"]), 0.1, ptr(B_a), ptr(ops.tc_status(dev)), st))
         else:
             with KERNEL_TIMER.region("bee_messages_scalar"):
                 check(lib().ld_bee_messages_scalar_f32(ptr(graph.row_ptr), ptr(graph.dst32), ptr(rij), Nt, C, self.dim_a,

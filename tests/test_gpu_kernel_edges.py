@@ -105,3 +105,86 @@ def test_split_message_is_as_exact_as_the_fma_kernel(n, n_rbf, radial, degrees, 
     for w, a, b in zip(want, split, fma):
         off = lambda t: float((t.cpu().double() - w).norm())  # noqa: E731
         assert off(a) <= 1.2 * off(b) + U * float(w.norm()), (off(a) / float(w.norm()), off(b) / float(w.norm()))
+
+
+# tiles of 64 edges, groups of 16: nodes without edges, nodes that span tiles, one edge in the last tile; both widths of
+# either kind of channel; sizes of the features that move the scales of the operands, one edge far above the others
+@pytest.mark.parametrize("chan,dim_a,degrees,size", [(128, 128, "mixed", 1.0), (128, 64, "long", 1.0), (64, 128, "mixed", 1e6),
+                                                     (64, 64, "long", 1e-5), (128, 128, "one", 1.0), (64, 64, "none", 1.0), (128, 128, "long", "spread")])
+def test_split_scalar_channel_is_as_exact_as_the_fma_kernel(chan, dim_a, degrees, size):
+    from ld_b200 import bee
+    from ld_b200.graph_layers import Graph
+    from ld_b200._lib import lib, check, ptr, stream_ptr
+    from ld_b200 import ops
+    g = torch.Generator().manual_seed(chan + dim_a)
+    deg = {"one": torch.tensor([0, 0, 1, 0]), "none": torch.zeros(5, dtype=torch.int64),
+           "mixed": torch.randint(0, 40, (61,), generator=g), "long": torch.tensor([3, 0, 300, 1, 0, 0, 64, 17, 129, 16])}[degrees]
+    Nt, E = len(deg), int(deg.sum())
+    src = torch.repeat_interleave(torch.arange(Nt), deg)
+    dst = torch.randint(0, Nt, (E,), generator=g)
+    rij = torch.randn(E, 3, generator=g) * 1.5
+    torch.manual_seed(3)
+    m = bee.Messages(5.0, dim_a, 32, 32, chan).cuda()
+    rows = torch.randn(Nt, 13, chan, generator=g)
+    if size == "spread":
+        rows *= 10.0 ** torch.randint(-8, 8, (Nt, 1, 1), generator=g)
+    else:
+        rows *= size
+    graph = Graph(src.cuda(), dst.cuda(), None, 1, Nt)
+    with torch.no_grad():
+        w = m._pack()
+    r13, rc = rows.cuda(), rij.cuda()
+    l = [r13[:, 0].contiguous(), r13[:, 1:4].transpose(1, 2).contiguous(), r13[:, 4:].transpose(1, 2).contiguous()]
+    again = torch.empty_like(r13)
+    check(lib().ld_bee_rows13_f32(ptr(l[0]), ptr(l[1]), ptr(l[2]), Nt, chan, ptr(again), stream_ptr()))
+    assert torch.equal(again, r13)
+    split, fma = torch.full((Nt, dim_a), 7.0, device="cuda"), torch.full((Nt, dim_a), 7.0, device="cuda")
+    geo = (ptr(graph.row_ptr), ptr(graph.dst32), ptr(rc), Nt, chan, dim_a, 5.0)
+    enc = (ptr(w["enc_w"]), ptr(w["enc_b"]), ptr(w["jac"]))
+    check(lib().ld_bee_messages_scalar_f32_split(*geo, ptr(r13), *enc, ptr(w["split"]), ptr(w["split_scales"]), ptr(w["b1"]), ptr(w["b2"]),
+                                                 ptr(w["b3"]), 0.1, ptr(split), ptr(ops.tc_status(r13.device)), stream_ptr()))
+    check(lib().ld_bee_messages_scalar_f32(*geo, *[ptr(t) for t in l], *enc, ptr(w["Yt"]), ptr(w["W1t"]), ptr(w["b1"]), ptr(w["W2t"]),
+                                           ptr(w["b2"]), ptr(w["W3t"]), ptr(w["b3"]), ptr(w["Wdt"]), 0.1, ptr(fma), stream_ptr()))
+    assert int(ops.tc_status(r13.device)) == 0
+    # the same layer in 64 bits
+    p = {k: v.detach().cpu().double() for k, v in m.state_dict().items()}
+    r = rij.double()
+    phi = bee.radial_encode_8(r, 5.0) @ p["lin_enc.weight"].t() + p["lin_enc.bias"]
+    u = r * 1.4
+    u = u / torch.sqrt(1 + (u ** 2).sum(-1, keepdim=True))
+    f = rows.double()[dst]
+    y = [f[:, 0] * phi, torch.einsum("ekc,ek->ec", f[:, 1:4], u) * phi,
+         torch.einsum("exyc,ex,ey->ec", f[:, 4:].reshape(E, 3, 3, chan), u, u) * phi]
+    psi = sum(t @ p[f"Y_{k}.W"].t() for t, k in zip(y, ("000", "110", "220")))
+    h = psi
+    for k in (0, 2, 4):
+        h = h @ p[f"mlp_a.layers.{k}.weight"].t() + p[f"mlp_a.layers.{k}.bias"]
+        h = torch.nn.functional.leaky_relu(h, 0.1) if k < 4 else h
+    want = torch.zeros(Nt, dim_a, dtype=torch.float64).index_add(0, src, 0.1 * (psi + psi @ p["mlp_a.lin_direct.weight"].t() + h))
+    # per node (the sizes differ by orders of magnitude): not further off than the FMAs, plus a rounding of the largest edge
+    edge = (0.1 * (psi.abs() + h.abs())).amax(-1)
+    biggest = torch.zeros(Nt, dtype=torch.float64).index_reduce(0, src, edge, "amax")
+    a, b = ((t.cpu().double() - want).norm(dim=-1) for t in (split, fma))
+    assert bool((a <= 1.5 * b + 4 * U * biggest * dim_a ** 0.5 + 1e-30).all()), (a / (b + 1e-300)).max()
+
+
+def test_split_kernels_give_a_node_the_same_bits_in_any_partition():
+    """the outputs of a system do not depend on which systems are computed beside it"""
+    from ld_b200 import bee, painn
+    from ld_b200.graph_layers import Graph
+    g = torch.Generator().manual_seed(5)
+    B, N = 5, 37
+    pos = torch.cumsum(torch.randn(B, N, 3, generator=g) / 3 ** 0.5, dim=1).cuda()
+    feats = [torch.randn(B, N, *s, generator=g).cuda() for s in ((64,), (64, 3), (32, 3, 3))]
+    torch.manual_seed(2)
+    layer, message = bee.Messages(4.0, 64, 64, 32, 64).cuda(), painn.Message(4.0, 64).cuda()
+
+    def run(lo, hi):
+        graph = Graph.radius_graph(4.0, None, pos[lo:hi])
+        x = [f[lo:hi] for f in feats]
+        return (*layer(graph, graph.rij, *x), *message(graph, x[0], x[1], graph.rij, residual=True))
+
+    with torch.no_grad():
+        whole, parts = run(0, B), [run(0, 2), run(2, 3), run(3, B)]
+    for k, w in enumerate(whole):
+        assert torch.equal(w, torch.cat([p[k] for p in parts])), k
