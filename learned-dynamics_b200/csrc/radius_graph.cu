@@ -59,10 +59,10 @@ __device__ __forceinline__ int open_cell(float x, float origin, float scale, int
   return min(max(c, 0), ndiv - 1);
 }
 
-// One block per system. Open boundary: bounding box -> cell grid with edge >= cutoff*(1+1e-5).
-__global__ void grid_setup_kernel(const float* __restrict__ pos, GraphParams P, GridDesc* __restrict__ desc,
+// One block per system. Open boundary: bounding box -> cell grid with edge >= cutoff*(1+1e-5). The description is valid in
+// the first thread, which also stores it.
+__device__ GridDesc describe_grid(const float* __restrict__ pos, const GraphParams& P, int b, GridDesc* __restrict__ desc,
                                   int* __restrict__ status) {
-  const int b = blockIdx.x;
   __shared__ float red[6][32];
   __shared__ int bad;
   if (threadIdx.x == 0) bad = 0;
@@ -91,9 +91,9 @@ __global__ void grid_setup_kernel(const float* __restrict__ pos, GraphParams P, 
     if (lane == 0) { red[a][w] = lo[a]; red[3 + a][w] = hi[a]; }
   }
   __syncthreads();
+  GridDesc g;
   if (threadIdx.x == 0) {
     if (bad) atomicOr(status, LD_FLAG_NONFINITE);
-    GridDesc g;
     g.pad0 = g.pad1 = g.pad2 = 0;
     if (P.periodic) {
       g.ox = g.oy = g.oz = 0.f;
@@ -133,6 +133,11 @@ __global__ void grid_setup_kernel(const float* __restrict__ pos, GraphParams P, 
     }
     desc[b] = g;
   }
+  return g;
+}
+
+__global__ void grid_setup_kernel(const float* __restrict__ pos, GraphParams P, GridDesc* __restrict__ desc, int* __restrict__ status) {
+  describe_grid(pos, P, blockIdx.x, desc, status);
 }
 
 __device__ __forceinline__ int cell_of(const GraphParams& P, const GridDesc& g, float x, float y, float z,
@@ -202,24 +207,88 @@ __global__ void cell_sort_kernel(const float4* __restrict__ binned, const int* _
   sorted_cell[lo + rank] = c;
 }
 
-__device__ __forceinline__ float torch_mod_wrap(float d, float box) {
-  // ((d + 0.5*box) % box) - 0.5*box with torch's floor-mod for floats
-  float h = __fmul_rn(0.5f, box);
-  float t = __fadd_rn(d, h);
-  float m = fmodf(t, box);
-  if (m != 0.f && m < 0.f) m = __fadd_rn(m, box);
-  return __fsub_rn(m, h);
+// grid, counts, starts and the sorted particles of a whole system in one block (everything above in one launch instead of
+// eight). A system's particles start at b * nodes, so no scan over the systems is needed.
+// Shared memory: counts [cells_cap + 1], starts [cells_cap + 1], cell of each particle [nodes], particles by cell [nodes].
+constexpr int CELL_MAX_NODES = 8192, CELL_MAX_CELLS = 8192;   // 128 KB of shared memory; a block walks at most 8 particles a thread
+
+template <int CELL_THREADS>   // 1024, or 256 for up to 512 particles
+__global__ void __launch_bounds__(CELL_THREADS)
+build_cells_kernel(const float* __restrict__ pos, GraphParams P, GridDesc* __restrict__ desc, int* __restrict__ cell_start,
+                   float4* __restrict__ sorted, int* __restrict__ sorted_cell, int* __restrict__ status) {
+  extern __shared__ int s_cells[];
+  int* s_count = s_cells;
+  int* s_start = s_count + P.cells_cap + 1;
+  int* s_cell = s_start + P.cells_cap + 1;
+  int* s_order = s_cell + P.nodes;
+  __shared__ GridDesc s_grid;
+  __shared__ int s_warp[CELL_THREADS / 32], s_carry;
+  const int b = blockIdx.x, tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  {
+    const GridDesc g = describe_grid(pos, P, b, desc, status);
+    if (tid == 0) { s_grid = g; s_carry = 0; }
+  }
+  for (int c = tid; c <= P.cells_cap; c += CELL_THREADS) s_count[c] = 0;
+  __syncthreads();
+  const GridDesc g = s_grid;
+  const float* bp = pos + (size_t)b * P.nodes * 3;
+  float x, y, z;
+  for (int i = tid; i < P.nodes; i += CELL_THREADS) {
+    const int c = cell_of(P, g, bp[3 * i], bp[3 * i + 1], bp[3 * i + 2], &x, &y, &z);
+    s_cell[i] = c;
+    atomicAdd(&s_count[c], 1);
+  }
+  __syncthreads();
+  // exclusive prefix of the counts, CELL_THREADS cells at a time; the counts become cursors
+  for (int base = 0; base <= P.cells_cap; base += CELL_THREADS) {
+    const int c = base + tid;
+    const int v = c <= P.cells_cap ? s_count[c] : 0;
+    int inc = v;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) { const int t = __shfl_up_sync(0xffffffffu, inc, d); if (lane >= d) inc += t; }
+    if (lane == 31) s_warp[w] = inc;
+    __syncthreads();
+    if (w == 0) {
+      const int t = lane < CELL_THREADS / 32 ? s_warp[lane] : 0;
+      int ti = t;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) { const int u = __shfl_up_sync(0xffffffffu, ti, d); if (lane >= d) ti += u; }
+      if (lane < CELL_THREADS / 32) s_warp[lane] = ti - t;
+    }
+    __syncthreads();
+    const int start = s_carry + s_warp[w] + inc - v;
+    if (c <= P.cells_cap) {
+      s_start[c] = start;
+      s_count[c] = start;
+      if (c < P.cells_cap) cell_start[(size_t)b * P.cells_cap + c] = b * P.nodes + start;
+    }
+    __syncthreads();
+    if (tid == CELL_THREADS - 1) s_carry = start + v;
+    __syncthreads();
+  }
+  if (b == P.batch - 1 && tid == 0) cell_start[(size_t)P.batch * P.cells_cap] = P.batch * P.nodes;
+  for (int i = tid; i < P.nodes; i += CELL_THREADS) s_order[atomicAdd(&s_count[s_cell[i]], 1)] = i;
+  __syncthreads();
+  // ascending particle index inside every cell (rank by counting)
+  for (int s = tid; s < P.nodes; s += CELL_THREADS) {
+    const int i = s_order[s], c = s_cell[i], lo = s_start[c], hi = s_start[c + 1];
+    int rank = 0;
+    for (int k = lo; k < hi; k++) rank += s_order[k] < i ? 1 : 0;
+    cell_of(P, g, bp[3 * i], bp[3 * i + 1], bp[3 * i + 2], &x, &y, &z);
+    const size_t at = (size_t)b * P.nodes + lo + rank;
+    sorted[at] = make_float4(x, y, z, __int_as_float(i));
+    sorted_cell[at] = b * P.cells_cap + c;
+  }
 }
 
 constexpr int NB_WARPS = 8;
 
-// minimum image of a difference of two wrapped coordinates, d in [-box, box]. Bit-identical to
-// remainderf(d, box) there: the quotient is -1, 0 or +1 (ties at +-box/2 go to the even quotient 0)
-// and d -+ box is exact (Sterbenz), so two compares replace the library routine.
-__device__ __forceinline__ float min_image(float d, float box, float half) {
-  if (d > half) return __fsub_rn(d, box);
-  if (d < -half) return __fadd_rn(d, box);
-  return d;
+// size of the minimum image of a difference of two wrapped coordinates, d in [-box, box]: |remainderf(d, box)| bit for
+// bit. There the quotient is -1, 0 or +1 (ties at +-box/2 go to the even quotient 0), d -+ box is exact (Sterbenz), and box -
+// |d| is the smaller of the two sizes exactly when |d| > box/2.
+__device__ __forceinline__ float min_image_size(float d, float box) {
+  const float a = fabsf(d);
+  return fminf(a, __fsub_rn(box, a));
 }
 
 // ((d + 0.5*box) % box) - 0.5*box with torch's floor-mod; fast exact paths for |d + box/2| < 2*box
@@ -236,133 +305,230 @@ __device__ __forceinline__ float torch_mod_wrap_fast(float d, float box, float h
   return __fsub_rn(m, half);
 }
 
-// One warp per particle (in cell order). FILL=false: degree per node. FILL=true: write the edges.
+// One warp per `group` consecutive particles of the cell-sorted order. FILL=false: degree per node. FILL=true: write the edges.
 // Candidates: the 3x3 neighbouring cell columns in (x, y); along z the cells cz-1, cz, cz+1 are
 // consecutive in the cell-sorted particle array, so each column is one contiguous run (two when it
-// wraps around the box): at most 18 runs, walked 32 candidates at a time.
-template <bool FILL>
+// wraps around the box): at most 18 runs, walked 32 candidates at a time, each batch against all particles of the group that
+// share the cell.
+// Bound by the instructions per (particle, candidate), of which one in eight is an edge: the test is kept to a dozen, the cell
+// arithmetic and the loads are shared by the group, and what an edge needs (displacement, lattice shift, stores) is done for
+// 32 edges of a particle at a time, the accepted candidates waiting in a queue in shared memory. 32 boxes of 4096 nodes,
+// 8.6 M edges: count 122 us, fill 244 us (one warp per particle, selects and adds for the image, the edges of a batch
+// written at once, four on average: 190 and 453).
+constexpr int NB_GROUP = 8;
+
+// particles per warp: up to NB_GROUP, but at least 32 warps for every SM
+inline int nb_group(int total) {
+  int g = total / (148 * 32);
+  return g < 1 ? 1 : (g > NB_GROUP ? NB_GROUP : g);
+}
+
+template <bool FILL, bool PERIODIC>
 __global__ void __launch_bounds__(NB_WARPS * 32)
 neighbour_kernel(const float* __restrict__ pos, GraphParams P, const GridDesc* __restrict__ desc,
                  const int* __restrict__ cell_start, const float4* __restrict__ sorted,
-                 const int* __restrict__ sorted_cell, int* __restrict__ degree, const int* __restrict__ row_ptr,
+                 const int* __restrict__ sorted_cell, int group, int* __restrict__ degree, const int* __restrict__ row_ptr,
                  long long capacity, int* __restrict__ src, int* __restrict__ dst, int* __restrict__ shift,
                  float* __restrict__ rij, int* __restrict__ status) {
+  __shared__ float4 s_me[NB_WARPS][NB_GROUP];
+  __shared__ int s_queue[FILL ? NB_WARPS : 1][NB_GROUP][64];
+  __shared__ float s_rij[FILL ? NB_WARPS : 1][96];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int s = blockIdx.x * NB_WARPS + w;
   const int total = P.batch * P.nodes;
-  if (s >= total) return;
-  const float4 me = sorted[s];
-  const int idx = __float_as_int(me.w);
-  const int gcell = sorted_cell[s];
-  const int b = gcell / P.cells_cap;
-  const int lc = gcell - b * P.cells_cap;
-  const GridDesc g = desc[b];
-  const int cz = lc % g.nz;
-  const int cy = (lc / g.nz) % g.ny;
-  const int cx = lc / (g.nz * g.ny);
+  const int s0 = (blockIdx.x * NB_WARPS + w) * group;
+  if (s0 >= total) return;
+  const int members = min(group, total - s0);
   const float hx = __fmul_rn(0.5f, P.bx), hy = __fmul_rn(0.5f, P.by), hz = __fmul_rn(0.5f, P.bz);
+  // lane p < members: the group's p-th particle
+  int my_cell = -1, my_idx = 0;
+  if (lane < members) {
+    const float4 me = sorted[s0 + lane];
+    my_cell = sorted_cell[s0 + lane];
+    my_idx = __float_as_int(me.w);
+    s_me[w][lane] = me;
+  }
+  __syncwarp();
+  float* wrij = s_rij[FILL ? w : 0];
+  constexpr int UNROLL = FILL ? 1 : 4;   // of the loop over the particles (4: count 131 -> 122 us, but fill 244 -> 443)
 
-  // lanes 0..8: (dx, dy) column, first run; lanes 16..24: same column, second run (z wrap-around)
-  int run_start = 0, run_len = 0;
-  {
-    const int col = lane & 15;
-    const bool second = lane >= 16;
-    if (col < 9) {
-      const int dx = col / 3 - 1, dy = col % 3 - 1;
-      int ncx = cx + dx, ncy = cy + dy;
-      bool ok = true;
-      int z_lo, z_hi;  // inclusive range of cz offsets handled by this run, in unwrapped cell units
-      if (P.periodic) {
-        // with fewer than 3 cells on an axis the offsets {-1,0,1} would visit a cell twice
-        if (g.nx < 3) ok = ok && (dx >= 0) && (dx < g.nx);
-        if (g.ny < 3) ok = ok && (dy >= 0) && (dy < g.ny);
-        ncx = (ncx + g.nx) % g.nx; ncy = (ncy + g.ny) % g.ny;
-        if (g.nz < 3) { z_lo = 0; z_hi = g.nz - 1; ok = ok && !second; }   // the whole column, once
-        else {
-          const int lo = cz - 1, hi = cz + 1;
-          if (lo >= 0 && hi < g.nz) { z_lo = lo; z_hi = hi; ok = ok && !second; }
-          else if (lo < 0) { if (!second) { z_lo = 0; z_hi = hi; } else { z_lo = g.nz - 1; z_hi = g.nz - 1; } }
-          else { if (!second) { z_lo = lo; z_hi = g.nz - 1; } else { z_lo = 0; z_hi = 0; } }
+  for (int g0 = 0; g0 < members;) {
+    const int gcell = __shfl_sync(0xffffffffu, my_cell, g0);
+    const int g1 = g0 + __popc(__ballot_sync(0xffffffffu, lane >= g0 && my_cell == gcell));   // equal cells are neighbours in the order
+    const int b = gcell / P.cells_cap;
+    const int lc = gcell - b * P.cells_cap;
+    const GridDesc g = desc[b];
+    const int cz = lc % g.nz;
+    const int cy = (lc / g.nz) % g.ny;
+    const int cx = lc / (g.nz * g.ny);
+
+    // lanes 0..8: (dx, dy) column, first run; lanes 16..24: same column, second run (z wrap-around)
+    int run_start = 0, run_len = 0;
+    {
+      const int col = lane & 15;
+      const bool second = lane >= 16;
+      if (col < 9) {
+        const int dx = col / 3 - 1, dy = col % 3 - 1;
+        int ncx = cx + dx, ncy = cy + dy;
+        bool ok = true;
+        int z_lo, z_hi;  // inclusive range of cz offsets handled by this run, in unwrapped cell units
+        if (PERIODIC) {
+          // with fewer than 3 cells on an axis the offsets {-1,0,1} would visit a cell twice
+          if (g.nx < 3) ok = ok && (dx >= 0) && (dx < g.nx);
+          if (g.ny < 3) ok = ok && (dy >= 0) && (dy < g.ny);
+          ncx = (ncx + g.nx) % g.nx; ncy = (ncy + g.ny) % g.ny;
+          if (g.nz < 3) { z_lo = 0; z_hi = g.nz - 1; ok = ok && !second; }   // the whole column, once
+          else {
+            const int lo = cz - 1, hi = cz + 1;
+            if (lo >= 0 && hi < g.nz) { z_lo = lo; z_hi = hi; ok = ok && !second; }
+            else if (lo < 0) { if (!second) { z_lo = 0; z_hi = hi; } else { z_lo = g.nz - 1; z_hi = g.nz - 1; } }
+            else { if (!second) { z_lo = lo; z_hi = g.nz - 1; } else { z_lo = 0; z_hi = 0; } }
+          }
+        } else {
+          ok = ncx >= 0 && ncx < g.nx && ncy >= 0 && ncy < g.ny && !second;
+          z_lo = max(cz - 1, 0); z_hi = min(cz + 1, g.nz - 1);
         }
-      } else {
-        ok = ncx >= 0 && ncx < g.nx && ncy >= 0 && ncy < g.ny && !second;
-        z_lo = max(cz - 1, 0); z_hi = min(cz + 1, g.nz - 1);
-      }
-      if (ok) {
-        const int base_cell = b * P.cells_cap + (ncx * g.ny + ncy) * g.nz;
-        run_start = cell_start[base_cell + z_lo];
-        run_len = cell_start[base_cell + z_hi + 1] - run_start;
+        if (ok) {
+          const int base_cell = b * P.cells_cap + (ncx * g.ny + ncy) * g.nz;
+          run_start = cell_start[base_cell + z_lo];
+          run_len = cell_start[base_cell + z_hi + 1] - run_start;
+        }
       }
     }
-  }
 
-  const int node = b * P.nodes + idx;
-  long long base = 0;
-  float xi = 0.f, yi = 0.f, zi = 0.f;
-  if (FILL) {
-    base = row_ptr[node];
-    const float* p = pos + (size_t)node * 3;
-    xi = p[0]; yi = p[1]; zi = p[2];
-  }
-  int found = 0;
-  unsigned live = __ballot_sync(0xffffffffu, run_len > 0);
-  while (live) {
-    const int r = __ffs(live) - 1;
-    live &= live - 1;
-    const int rs = __shfl_sync(0xffffffffu, run_start, r);
-    const int rl = __shfl_sync(0xffffffffu, run_len, r);
-    for (int k0 = 0; k0 < rl; k0 += 32) {
-      const int k = k0 + lane;
-      bool hit = false;
-      int jdx = 0;
-      if (k < rl) {
-        const float4 q = __ldg(&sorted[rs + k]);
-        jdx = __float_as_int(q.w);
-        float dx = __fsub_rn(me.x, q.x), dy = __fsub_rn(me.y, q.y), dz = __fsub_rn(me.z, q.z);
-        if (P.periodic) { dx = min_image(dx, P.bx, hx); dy = min_image(dy, P.by, hy); dz = min_image(dz, P.bz, hz); }
-        const float d2 = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx)));
-        hit = (jdx != idx) && (d2 <= P.rc2);
-      }
-      const unsigned bal = __ballot_sync(0xffffffffu, hit);
-      if (FILL) {
-        if (hit) {
-          const long long e = base + found + __popc(bal & ((1u << lane) - 1));
-          if (e < capacity) {
-            const int nj = b * P.nodes + jdx;
-            src[e] = node;
-            dst[e] = nj;
-            if (rij != nullptr || shift != nullptr) {
-              const float* pj = pos + (size_t)nj * 3;
-              float ddx = __fsub_rn(__ldg(pj), xi), ddy = __fsub_rn(__ldg(pj + 1), yi), ddz = __fsub_rn(__ldg(pj + 2), zi);
-              if (shift != nullptr) {
-                int sx = 0, sy = 0, sz = 0;
-                if (P.periodic) {
-                  sx = -(int)floorf(__fdiv_rn(__fadd_rn(ddx, hx), P.bx));
-                  sy = -(int)floorf(__fdiv_rn(__fadd_rn(ddy, hy), P.by));
-                  sz = -(int)floorf(__fdiv_rn(__fadd_rn(ddz, hz), P.bz));
-                }
-                shift[e] = (sx & 0xff) | ((sy & 0xff) << 8) | ((sz & 0xff) << 16);
-                // three signed bytes: positions more than 127 box lengths apart do not fit
-                if ((abs(sx) > 127 || abs(sy) > 127 || abs(sz) > 127) && status != nullptr) atomicOr(status, LD_FLAG_OVERFLOW);
-              }
-              if (rij != nullptr) {
-                if (P.periodic) {
-                  ddx = torch_mod_wrap_fast(ddx, P.bx, hx); ddy = torch_mod_wrap_fast(ddy, P.by, hy);
-                  ddz = torch_mod_wrap_fast(ddz, P.bz, hz);
-                }
-                rij[e * 3 + 0] = ddx; rij[e * 3 + 1] = ddy; rij[e * 3 + 2] = ddz;
-              }
+    // lane p of the group: edges counted (FILL: written), edges waiting in its queue, first edge
+    int found = 0, queued = 0;
+    const bool mine = lane >= g0 && lane < g1;
+    const int my_node = b * P.nodes + my_idx;
+    int my_base = 0;
+    if (FILL && mine) my_base = row_ptr[my_node];
+    // writes the first `n` queued edges of particle p
+    auto emit = [&](int p, int n) {
+      const int node = __shfl_sync(0xffffffffu, my_node, p);
+      const long long first = (long long)__shfl_sync(0xffffffffu, my_base, p) + __shfl_sync(0xffffffffu, found, p);
+      const long long e = first + lane;
+      float ddx = 0.f, ddy = 0.f, ddz = 0.f;
+      if (lane < n) {
+        const int nj = b * P.nodes + s_queue[FILL ? w : 0][p][lane];
+        if (rij != nullptr || shift != nullptr) {
+          const float* pi = pos + (size_t)node * 3;
+          const float* pj = pos + (size_t)nj * 3;
+          ddx = __fsub_rn(__ldg(pj), __ldg(pi)); ddy = __fsub_rn(__ldg(pj + 1), __ldg(pi + 1)); ddz = __fsub_rn(__ldg(pj + 2), __ldg(pi + 2));
+        }
+        if (e < capacity) {
+          src[e] = node;
+          dst[e] = nj;
+          if (shift != nullptr) {
+            int sx = 0, sy = 0, sz = 0;
+            if (PERIODIC) {
+              sx = -(int)floorf(__fdiv_rn(__fadd_rn(ddx, hx), P.bx));
+              sy = -(int)floorf(__fdiv_rn(__fadd_rn(ddy, hy), P.by));
+              sz = -(int)floorf(__fdiv_rn(__fadd_rn(ddz, hz), P.bz));
             }
+            shift[e] = (sx & 0xff) | ((sy & 0xff) << 8) | ((sz & 0xff) << 16);
+            // three signed bytes: positions more than 127 box lengths apart do not fit
+            if ((abs(sx) > 127 || abs(sy) > 127 || abs(sz) > 127) && status != nullptr) atomicOr(status, LD_FLAG_OVERFLOW);
           }
         }
       }
-      found += __popc(bal);
+      if (rij != nullptr) {
+        if (PERIODIC) {
+          ddx = torch_mod_wrap_fast(ddx, P.bx, hx); ddy = torch_mod_wrap_fast(ddy, P.by, hy); ddz = torch_mod_wrap_fast(ddz, P.bz, hz);
+        }
+        wrij[3 * lane] = ddx; wrij[3 * lane + 1] = ddy; wrij[3 * lane + 2] = ddz;   // (stride 3: no bank conflicts)
+        __syncwarp();
+        const long long room = capacity - first;
+        const int live = 3 * (int)(room < n ? (room > 0 ? room : 0) : n);
+        float* out = rij + first * 3;
+#pragma unroll
+        for (int q = 0; q < 3; q++)
+          if (lane + 32 * q < live) out[lane + 32 * q] = wrij[lane + 32 * q];
+      }
+      __syncwarp();
+      if (lane == p) found += n;
+    };
+
+    unsigned live = __ballot_sync(0xffffffffu, run_len > 0);
+    while (live) {
+      const int r = __ffs(live) - 1;
+      live &= live - 1;
+      const int rs = __shfl_sync(0xffffffffu, run_start, r);
+      const int rl = __shfl_sync(0xffffffffu, run_len, r);
+      for (int k0 = 0; k0 < rl; k0 += 32) {
+        float4 q = make_float4(0.f, 0.f, 0.f, __int_as_float(-1));
+        const bool there = k0 + lane < rl;
+        if (there) q = __ldg(&sorted[rs + k0 + lane]);
+        const int jdx = __float_as_int(q.w);
+#pragma unroll UNROLL
+        for (int p = g0; p < g1; p++) {
+          const float4 me = s_me[w][p];
+          float dx = __fsub_rn(me.x, q.x), dy = __fsub_rn(me.y, q.y), dz = __fsub_rn(me.z, q.z);
+          if (PERIODIC) { dx = min_image_size(dx, P.bx); dy = min_image_size(dy, P.by); dz = min_image_size(dz, P.bz); }
+          const float d2 = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx)));
+          const bool hit = there && jdx != __float_as_int(me.w) && d2 <= P.rc2;
+          const unsigned bal = __ballot_sync(0xffffffffu, hit);
+          if (!FILL) {
+            if (lane == p) found += __popc(bal);
+          } else if (bal != 0u) {
+            int* queue = s_queue[FILL ? w : 0][p];
+            const int have = __shfl_sync(0xffffffffu, queued, p);
+            if (hit) queue[have + __popc(bal & ((1u << lane) - 1))] = jdx;
+            int now = have + __popc(bal);
+            if (now >= 32) {
+              __syncwarp();
+              emit(p, 32);
+              now -= 32;
+              const int rest = lane < now ? queue[32 + lane] : 0;
+              __syncwarp();
+              if (lane < now) queue[lane] = rest;
+            }
+            if (lane == p) queued = now;
+          }
+        }
+      }
     }
+    if (!FILL) {
+      if (mine) degree[my_node] = found;
+    } else {
+      __syncwarp();
+      for (int p = g0; p < g1; p++) {
+        const int n = __shfl_sync(0xffffffffu, queued, p);
+        if (n > 0) emit(p, n);
+      }
+      if (mine && (long long)my_base + found > capacity) atomicOr(status, LD_FLAG_CAPACITY);
+    }
+    g0 = g1;
   }
-  if (!FILL) {
-    if (lane == 0) degree[node] = found;
-  } else {
-    if (lane == 0 && base + found > capacity) atomicOr(status, LD_FLAG_CAPACITY);
+}
+
+// exclusive prefix of the degrees and the cumulative edge counts of the systems, in one block
+constexpr int ONE_SCAN_THREADS = 1024, ONE_SCAN_MAX = 16384;
+__global__ void __launch_bounds__(ONE_SCAN_THREADS)
+degree_scan_kernel(const int* __restrict__ degree, int Nt, int nodes, int* __restrict__ row_ptr, int* __restrict__ edge_counts) {
+  __shared__ int s_warp[32];
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const int items = (Nt + ONE_SCAN_THREADS - 1) / ONE_SCAN_THREADS, i0 = tid * items;
+  int sum = 0;
+  for (int q = 0; q < items; q++) sum += i0 + q < Nt ? degree[i0 + q] : 0;
+  int inc = sum;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) { const int t = __shfl_up_sync(0xffffffffu, inc, d); if (lane >= d) inc += t; }
+  if (lane == 31) s_warp[w] = inc;
+  __syncthreads();
+  if (w == 0) {
+    const int t = s_warp[lane];
+    int ti = t;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) { const int u = __shfl_up_sync(0xffffffffu, ti, d); if (lane >= d) ti += u; }
+    s_warp[lane] = ti - t;
+  }
+  __syncthreads();
+  int at = s_warp[w] + inc - sum;
+  for (int q = 0; q < items && i0 + q < Nt; q++) {
+    const int i = i0 + q;
+    row_ptr[i] = at;
+    at += degree[i];
+    if (i == Nt - 1) row_ptr[Nt] = at;
+    if (edge_counts != nullptr && (i + 1) % nodes == 0) edge_counts[i / nodes] = at;
   }
 }
 
@@ -500,32 +666,52 @@ extern "C" int ld_radius_graph_count(const float* pos, int batch, int nodes, int
     LD_CUDA_TRY(cudaMemsetAsync(row_ptr, 0, 4, stream));
     return LD_OK;
   }
-  const size_t nc = (size_t)batch * P.cells_cap;
-  LD_CUDA_TRY(cudaMemsetAsync(w.cell_count, 0, 4 * (nc + 1), stream));
-  LD_CUDA_TRY(cudaMemsetAsync(w.cell_cursor, 0, 4 * nc, stream));
-  grid_setup_kernel<<<batch, 256, 0, stream>>>(pos, P, w.desc, status_dev);
+  if (nodes <= CELL_MAX_NODES && P.cells_cap <= CELL_MAX_CELLS) {
+    const size_t smem = 4 * ((size_t)2 * (P.cells_cap + 1) + 2 * (size_t)nodes);
+    auto kern = nodes <= 512 ? build_cells_kernel<256> : build_cells_kernel<1024>;
+    if (smem > 48 * 1024) LD_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kern<<<batch, nodes <= 512 ? 256 : 1024, smem, stream>>>(pos, P, w.desc, w.cell_start, w.sorted, w.sorted_cell, status_dev);
+    LD_LAUNCH_CHECK();
+  } else {
+    // a system that one block cannot hold: counts, scan and placement over all particles
+    const size_t nc = (size_t)batch * P.cells_cap;
+    LD_CUDA_TRY(cudaMemsetAsync(w.cell_count, 0, 4 * (nc + 1), stream));
+    LD_CUDA_TRY(cudaMemsetAsync(w.cell_cursor, 0, 4 * nc, stream));
+    grid_setup_kernel<<<batch, 256, 0, stream>>>(pos, P, w.desc, status_dev);
+    LD_LAUNCH_CHECK();
+    const int nb = ld_cdiv(Nt, 256);
+    bin_kernel<false><<<nb, 256, 0, stream>>>(pos, P, w.desc, w.cell_count, nullptr, nullptr, nullptr, nullptr);
+    LD_LAUNCH_CHECK();
+    rc = ld_scan_exclusive(w.cell_count, w.cell_start, (long long)nc, w.scan, stream);
+    if (rc != LD_OK) return rc;
+    bin_kernel<true><<<nb, 256, 0, stream>>>(pos, P, w.desc, nullptr, w.cell_start, w.cell_cursor, w.binned, w.binned_cell);
+    LD_LAUNCH_CHECK();
+    cell_sort_kernel<<<nb, 256, 0, stream>>>(w.binned, w.binned_cell, w.cell_start, Nt, w.sorted, w.sorted_cell);
+    LD_LAUNCH_CHECK();
+  }
+  const int group = nb_group(Nt), nblk = ld_cdiv(Nt, NB_WARPS * group);
+  if (P.periodic)
+    neighbour_kernel<false, true><<<nblk, NB_WARPS * 32, 0, stream>>>(pos, P, w.desc, w.cell_start, w.sorted, w.sorted_cell, group, w.degree, nullptr,
+                                                                      0, nullptr, nullptr, nullptr, nullptr, status_dev);
+  else
+    neighbour_kernel<false, false><<<nblk, NB_WARPS * 32, 0, stream>>>(pos, P, w.desc, w.cell_start, w.sorted, w.sorted_cell, group, w.degree, nullptr,
+                                                                       0, nullptr, nullptr, nullptr, nullptr, status_dev);
   LD_LAUNCH_CHECK();
-  const int nb = ld_cdiv(Nt, 256);
-  bin_kernel<false><<<nb, 256, 0, stream>>>(pos, P, w.desc, w.cell_count, nullptr, nullptr, nullptr, nullptr);
-  LD_LAUNCH_CHECK();
-  rc = ld_scan_exclusive(w.cell_count, w.cell_start, (long long)nc, w.scan, stream);
-  if (rc != LD_OK) return rc;
-  bin_kernel<true><<<nb, 256, 0, stream>>>(pos, P, w.desc, nullptr, w.cell_start, w.cell_cursor, w.binned, w.binned_cell);
-  LD_LAUNCH_CHECK();
-  cell_sort_kernel<<<nb, 256, 0, stream>>>(w.binned, w.binned_cell, w.cell_start, Nt, w.sorted, w.sorted_cell);
-  LD_LAUNCH_CHECK();
-  neighbour_kernel<false><<<ld_cdiv(Nt, NB_WARPS), NB_WARPS * 32, 0, stream>>>(
-      pos, P, w.desc, w.cell_start, w.sorted, w.sorted_cell, w.degree, nullptr, 0, nullptr, nullptr, nullptr, nullptr,
-      status_dev);
-  LD_LAUNCH_CHECK();
-  rc = ld_scan_exclusive(w.degree, row_ptr, (long long)Nt, w.scan, stream);
-  if (rc != LD_OK) return rc;
+  // up to 16384 nodes the prefix sum is one launch of a few us instead of four (its serial part grows with the count)
+  const bool one_scan = Nt <= ONE_SCAN_MAX;
+  if (one_scan) {
+    degree_scan_kernel<<<1, ONE_SCAN_THREADS, 0, stream>>>(w.degree, Nt, nodes, row_ptr, edge_counts);
+    LD_LAUNCH_CHECK();
+  } else {
+    rc = ld_scan_exclusive(w.degree, row_ptr, (long long)Nt, w.scan, stream);
+    if (rc != LD_OK) return rc;
+  }
   // row_ptr is int32: only problems whose edge count could pass 2^31-1 pay for the 64-bit check of the degree sum
   if ((long long)Nt * (nodes - 1) > 0x7fffffffLL) {
     degree_overflow_kernel<<<1, 256, 0, stream>>>(w.degree, Nt, status_dev);
     LD_LAUNCH_CHECK();
   }
-  if (edge_counts != nullptr) {
+  if (edge_counts != nullptr && !one_scan) {
     edge_counts_kernel<<<ld_cdiv(batch, 256), 256, 0, stream>>>(row_ptr, batch, nodes, edge_counts);
     LD_LAUNCH_CHECK();
   }
@@ -555,8 +741,13 @@ extern "C" int ld_radius_graph_fill(const float* pos, int batch, int nodes, int 
     LD_LAUNCH_CHECK();
     return LD_OK;
   }
-  neighbour_kernel<true><<<ld_cdiv(Nt, NB_WARPS), NB_WARPS * 32, 0, stream>>>(
-      pos, P, w.desc, w.cell_start, w.sorted, w.sorted_cell, nullptr, row_ptr, capacity, src, dst, shift, rij, status_dev);
+  const int group = nb_group(Nt), nblk = ld_cdiv(Nt, NB_WARPS * group);
+  if (P.periodic)
+    neighbour_kernel<true, true><<<nblk, NB_WARPS * 32, 0, stream>>>(
+        pos, P, w.desc, w.cell_start, w.sorted, w.sorted_cell, group, nullptr, row_ptr, capacity, src, dst, shift, rij, status_dev);
+  else
+    neighbour_kernel<true, false><<<nblk, NB_WARPS * 32, 0, stream>>>(
+        pos, P, w.desc, w.cell_start, w.sorted, w.sorted_cell, group, nullptr, row_ptr, capacity, src, dst, shift, rij, status_dev);
   LD_LAUNCH_CHECK();
   return LD_OK;
 }

@@ -188,3 +188,40 @@ def test_split_kernels_give_a_node_the_same_bits_in_any_partition():
         whole, parts = run(0, B), [run(0, 2), run(2, 3), run(3, B)]
     for k, w in enumerate(whole):
         assert torch.equal(w, torch.cat([p[k] for p in parts])), k
+
+
+# one block per system up to 8192 nodes and cells (256 threads to 512 nodes), all particles together beyond; the degrees in one
+# block up to 16384 nodes; boxes with two to many cells per axis, coordinates on the boundary and in other images
+@pytest.mark.parametrize("batch,nodes,box,cutoff", [
+    (3, 512, None, 3.0), (2, 513, (9.0, 7.0, 11.0), 2.9), (2, 8192, (20.0, 21.0, 22.0), 1.5), (1, 8193, (18.0, 20.0, 19.0), 1.4),
+    (40, 410, (8.0, 8.0, 8.0), 1.1), (5, 37, (4.0, 4.1, 9.0), 1.9), (2, 300, (30.0, 60.0, 30.0), 1.0), (1, 1, None, 1.0)])
+def test_radius_graph_build_paths(batch, nodes, box, cutoff):
+    from ld_b200 import graph as G
+    g = torch.Generator().manual_seed(nodes)
+    if box is None:
+        pos = torch.cumsum(torch.randn(batch, nodes, 3, generator=g) / 3 ** 0.5, dim=1)
+    else:
+        L = torch.tensor(box)
+        pos = torch.rand(batch, nodes, 3, generator=g) * L
+        pos[:, :: 7] += L * torch.randint(-3, 4, pos[:, :: 7].shape, generator=g)
+        pos[:, 1 :: 11, 0] = L[0]
+        pos[:, 2 :: 11, 1] = 0.0
+        pos[:, 3 :: 13, 2] = torch.nextafter(L[2], torch.zeros(()))
+    b = G.RadiusGraphBuilder(batch, nodes, cutoff, box)
+    got = b.build(pos.cuda(), want_shift=True)
+    assert int(b.status) == 0
+    from oracle import reference_math as R
+    oracle = R.radius_graph(pos, cutoff, box)
+    src, dst = oracle["src"], oracle["dst"]
+    E = got["E"]
+    key = lambda s, d: torch.sort(s.cpu().long() * (batch * nodes) + d.cpu().long()).values  # noqa: E731
+    assert torch.equal(key(got["src"], got["dst"]), key(src, dst))
+    deg = torch.bincount(got["src"].cpu().long(), minlength=batch * nodes)
+    assert torch.equal(got["row_ptr"].cpu().long(), torch.cat([torch.zeros(1, dtype=torch.long), deg.cumsum(0)]))
+    assert torch.equal(got["edge_counts"].cpu().long(), deg.reshape(batch, nodes).sum(1).cumsum(0))
+    s, d = got["src"].cpu().long(), got["dst"].cpu().long()
+    # displacements and shifts of the same pairs (the two lists order a node's neighbours differently)
+    mine, ref = torch.argsort(s * (batch * nodes) + d), torch.argsort(src.long() * (batch * nodes) + dst.long())
+    assert torch.equal(got["rij"].cpu()[mine], oracle["rij"][ref])
+    assert torch.equal(G.unpack_shift(got["shift"]).cpu()[mine], oracle["shift"][ref].int())
+    assert bool((s[1:] >= s[:-1]).all()) and E == len(src)
