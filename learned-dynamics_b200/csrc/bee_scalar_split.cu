@@ -63,7 +63,7 @@ bee_scalar_split_kernel(const __grid_constant__ BeeSplitParams P) {
   using S = BeeShape<C, A>;
   constexpr int HB = S::HB;
   extern __shared__ __align__(1024) unsigned char smem[];
-  __shared__ __align__(8) uint64_t bar_full[STAGES], bar_done[4], bar_taken[2];
+  __shared__ __align__(8) uint64_t bar_full[STAGES], bar_empty[STAGES], bar_done[4], bar_taken[2];
   __shared__ uint32_t tmem_slot;
   __shared__ EdgeGeom s_geom[NE];
   __shared__ EdgeScales s_sc[NE];
@@ -79,7 +79,7 @@ bee_scalar_split_kernel(const __grid_constant__ BeeSplitParams P) {
 
   if (tid < 8) ld_poly8_to_chebyshev(P.jacobi + tid * 9, s_jac + tid * 9);   // Chebyshev form of the radial polynomials
   if (tid == 0) {
-    for (int s = 0; s < STAGES; s++) tc::mbar_init(&bar_full[s], 1);
+    for (int s = 0; s < STAGES; s++) { tc::mbar_init(&bar_full[s], 1); tc::mbar_init(&bar_empty[s], 1); }
     for (int s = 0; s < 4; s++) tc::mbar_init(&bar_done[s], 1);            // MMAs of slab q: accumulator q % 4
     for (int s = 0; s < 2; s++) tc::mbar_init(&bar_taken[s], WORK_WARPS);  // partial sums of a step are in registers
     tc::mbar_init_fence();
@@ -101,8 +101,8 @@ bee_scalar_split_kernel(const __grid_constant__ BeeSplitParams P) {
         for (long long t = 0; t < ntiles && !fail; t++) {
           const unsigned char* src = reinterpret_cast<const unsigned char*>(P.w);
           for (int q = 0; q < S::SLABS; q++, loads++, src += SLAB_BYTES) {
-            const uint32_t st = loads % STAGES, old = loads - STAGES;   // the slab that held this stage
-            if (loads >= STAGES && !tc::mbar_wait(&bar_done[old & 3], (old >> 2) & 1)) { fail = 1; break; }
+            const uint32_t st = loads % STAGES, use = loads / STAGES;
+            if (use >= 1 && !tc::mbar_wait(&bar_empty[st], (use - 1) & 1)) { fail = 1; break; }   // MMAs that read it are done
             tc::mbar_expect_tx(&bar_full[st], SLAB_BYTES);
             tc::bulk_g2s(ring + (size_t)st * SLAB_BYTES, src, SLAB_BYTES, &bar_full[st]);
           }
@@ -130,8 +130,10 @@ bee_scalar_split_kernel(const __grid_constant__ BeeSplitParams P) {
         if (steps >= 2 && !tc::mbar_wait(&bar_taken[steps & 1], ((steps >> 1) - 1) & 1)) { fail = 1; break; }
         tc::fence_after_sync();
         if (!tc::mbar_wait(&bar_full[st], full_phase)) { fail = 1; break; }
+        tc::fence_after_sync();
         const uint32_t slot = (steps & 1) * 2 + me;
         slab_mmas(tmem_base + slot * NE, a0 + st * st_step, 2, x1, x2, b_step, idesc);
+        tc::mma_commit(&bar_empty[st]);
         tc::mma_commit(&bar_done[slot]);
         st += MMA_WARPS;
         if (st >= STAGES) { st -= STAGES; full_phase ^= 1; }

@@ -72,7 +72,7 @@ painn_message_split_kernel(const __grid_constant__ SplitParams P) {
   using S = Shape<MB>;
   constexpr int N = S::N, n = S::n, NE = S::NE, SLOTS = S::SLOTS;
   extern __shared__ __align__(1024) unsigned char smem[];
-  __shared__ __align__(8) uint64_t bar_full[STAGES], bar_done[SLOTS], bar_taken[2];
+  __shared__ __align__(8) uint64_t bar_full[STAGES], bar_empty[STAGES], bar_done[SLOTS], bar_taken[2];
   __shared__ uint32_t tmem_slot;
   __shared__ float s_dir[NE][3];
   __shared__ float s_dist[NE], s_env[NE];
@@ -87,7 +87,7 @@ painn_message_split_kernel(const __grid_constant__ SplitParams P) {
 
   for (int i = tid; i < 3 * N; i += THREADS) s_bias[i] = P.b[i / N][i % N];
   if (tid == 0) {
-    for (int s = 0; s < STAGES; s++) tc::mbar_init(&bar_full[s], 1);
+    for (int s = 0; s < STAGES; s++) { tc::mbar_init(&bar_full[s], 1); tc::mbar_init(&bar_empty[s], 1); }
     for (int s = 0; s < SLOTS; s++) tc::mbar_init(&bar_done[s], 1);      // MMAs of slab q: slot q % SLOTS
     for (int s = 0; s < 2; s++) tc::mbar_init(&bar_taken[s], WORK_WARPS);   // partial sums of a chunk are in registers
     tc::mbar_init_fence();
@@ -113,8 +113,8 @@ painn_message_split_kernel(const __grid_constant__ SplitParams P) {
             for (int k0 = 0; k0 < K && !fail; k0 += sf::SLAB_K) {
               const uint32_t bytes = 2u * 128u * 2u * (uint32_t)min(sf::SLAB_K, K - k0);
               for (int m = 0; m < MB; m++, loads++, src += bytes) {
-                const uint32_t st = loads % STAGES, old = loads - STAGES;   // the slab that held this stage
-                if (loads >= STAGES && !tc::mbar_wait(&bar_done[old % SLOTS], (old / SLOTS) & 1)) { fail = 1; break; }
+                const uint32_t st = loads % STAGES, use = loads / STAGES;
+                if (use >= 1 && !tc::mbar_wait(&bar_empty[st], (use - 1) & 1)) { fail = 1; break; }   // MMAs that read it are done
                 tc::mbar_expect_tx(&bar_full[st], bytes);
                 tc::bulk_g2s(ring + (size_t)st * sf::SLAB_BYTES, src, bytes, &bar_full[st]);
               }
@@ -129,8 +129,7 @@ painn_message_split_kernel(const __grid_constant__ SplitParams P) {
   } else if (warp >= MMA_WARP) {
     // ===== MMA issue ==============================================================================================
     // the issuing thread runs alone in its warp, so every instruction between two MMAs is exposed: descriptors and ring
-    // positions advance by additions, accumulators are waited for once per chunk of MB slabs, and one commit per slab
-    // reports both that the partial sum is complete and that the ring stage is free
+    // positions advance by additions, and accumulators are waited for once per chunk of MB slabs
     const uint32_t me = warp - MMA_WARP;
     uint32_t chunks = 0, st = me, full_phase = 0;
     const uint32_t b1 = desc_lo(act, S::PANEL), b2 = desc_lo(act + S::PLANE, S::PANEL);
@@ -156,7 +155,9 @@ painn_message_split_kernel(const __grid_constant__ SplitParams P) {
               for (int h = 0; h < (MB + 1) / 2; h++) {
                 const uint32_t slot = (chunks & 1) * MB + (MB == 1 ? 0 : 2 * h + me);   // slabs are numbered chunk * MB + block
                 if (!tc::mbar_wait(&bar_full[st], full_phase)) { fail = 1; break; }
+                tc::fence_after_sync();
                 sf::slab_mmas(tmem_base + slot * NE, a0 + st * st_step, ks, x1, x2, b_step, idesc);
+                tc::mma_commit(&bar_empty[st]);
                 tc::mma_commit(&bar_done[slot]);
                 st += MMA_WARPS;
                 if (st >= STAGES) { st -= STAGES; full_phase ^= 1; }
