@@ -49,49 +49,6 @@ __device__ __forceinline__ void run_mlp3(const MlpWeights& m, int act, float* bu
   mt_tile_linear<NCOL, true>(buf0, m.n2, m.W3t, m.b3, m.n3, LD_ACT_NONE, buf1, ldo, wstage);
 }
 
-// out[r, :] = W3 act(W2 act(W1 x[r] + b1) + b2) + b3 (+ Wd x[r] when Wdt != nullptr)
-template <int NCOL>
-__global__ void __launch_bounds__(MT_THREADS, 1)
-mlp3_rows_kernel(const float* __restrict__ x, long long rows, MlpWeights m, int act, const float* __restrict__ Wdt,
-                 float* __restrict__ out) {
-  extern __shared__ __align__(16) float smem[];
-  const SmemPlan plan(m);
-  float* buf0 = smem;
-  float* buf1 = buf0 + plan.buf_floats;
-  float* wstage = buf1 + plan.buf_floats;
-  const int tid = threadIdx.x;
-  const long long ntiles = (rows + MT_ROWS - 1) / MT_ROWS;
-  for (long long t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    const long long r0 = t * MT_ROWS;
-    for (int idx = tid; idx < MT_ROWS * m.k0; idx += MT_THREADS) {
-      const int r = idx & (MT_ROWS - 1), k = idx >> 5;
-      buf0[k * MT_ROWS + r] = (r0 + r < rows) ? x[(r0 + r) * m.k0 + k] : 0.f;
-    }
-    __syncthreads();
-    run_mlp3<NCOL>(m, act, buf0, buf1, plan.ldo, wstage);
-    if (Wdt != nullptr) {
-      // direct linear term: reload x (buf0 was overwritten by layer 2) and accumulate
-      for (int idx = tid; idx < MT_ROWS * m.k0; idx += MT_THREADS) {
-        const int r = idx & (MT_ROWS - 1), k = idx >> 5;
-        buf0[k * MT_ROWS + r] = (r0 + r < rows) ? x[(r0 + r) * m.k0 + k] : 0.f;
-      }
-      __syncthreads();
-      for (int idx = tid; idx < MT_ROWS * m.n3; idx += MT_THREADS) {
-        const int r = idx / m.n3, c = idx - r * m.n3;
-        float a = 0.f;
-        for (int k = 0; k < m.k0; k++) a = fmaf(buf0[k * MT_ROWS + r], Wdt[(size_t)k * m.n3 + c], a);
-        buf1[(size_t)r * plan.ldo + c] += a;
-      }
-      __syncthreads();
-    }
-    for (int idx = tid; idx < MT_ROWS * m.n3; idx += MT_THREADS) {
-      const int r = idx / m.n3, c = idx - r * m.n3;
-      if (r0 + r < rows) out[(r0 + r) * m.n3 + c] = buf1[(size_t)r * plan.ldo + c];
-    }
-    __syncthreads();
-  }
-}
-
 struct MessageParams {
   const int* row_ptr;   // [Nt+1]
   const int* dst;       // [E]
@@ -274,33 +231,6 @@ int sm_count() {
 }
 
 }  // namespace
-
-// Three dense layers on `rows` rows. Weights are passed transposed ("packed"): Wkt is [in][out]
-// contiguous, i.e. nn.Linear.weight.t().contiguous(). act: 0 none, 1 SiLU, 2 LeakyReLU(0.1),
-// applied after layers 1 and 2. Wdt (optional, [k0][n3]) adds a direct linear term x*Wd.
-extern "C" int ld_mlp3_rows(const float* x, long long rows, int k0, const float* W1t, const float* b1, int n1,
-                            const float* W2t, const float* b2, int n2, const float* W3t, const float* b3, int n3, int act,
-                            const float* Wdt, float* out, void* stream) {
-  if (rows < 0) return LD_ERR_SHAPE;
-  MlpWeights m{W1t, b1, W2t, b2, W3t, b3, k0, n1, n2, n3};
-  int ncol = 1;
-  int rc = check_mlp(m, &ncol);
-  if (rc != LD_OK) return rc;
-  if (rows == 0) return LD_OK;
-  const SmemPlan plan(m);
-  const size_t smem = plan.bytes();
-  const long long ntiles = (rows + MT_ROWS - 1) / MT_ROWS;
-  const int grid = (int)(ntiles < sm_count() ? ntiles : sm_count());
-  if (ncol == 1) {
-    rc = set_smem(mlp3_rows_kernel<1>, smem); if (rc != LD_OK) return rc;
-    mlp3_rows_kernel<1><<<grid, MT_THREADS, smem, (cudaStream_t)stream>>>(x, rows, m, act, Wdt, out);
-  } else {
-    rc = set_smem(mlp3_rows_kernel<2>, smem); if (rc != LD_OK) return rc;
-    mlp3_rows_kernel<2><<<grid, MT_THREADS, smem, (cudaStream_t)stream>>>(x, rows, m, act, Wdt, out);
-  }
-  LD_LAUNCH_CHECK();
-  return LD_OK;
-}
 
 // Fused PaiNN message (FP32). Graph in CSR form sorted by source (row_ptr[Nt+1], dst[E], rij[E,3]).
 // Distance MLP: n_rbf -> 4n -> 4n -> 4n, SiLU, packed weights. actv = mlp_actv(x_a) [Nt,4n].

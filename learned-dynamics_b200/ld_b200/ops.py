@@ -294,6 +294,26 @@ def mlp3_rows(x, mlp, act=ACT_SILU):
     return out
 
 
+def painn_update_front(y, x_a, rows, n):
+    """y [rows, 3n, 3] = the stacked mixings of x_v: (inner [rows, n], cat [rows, 2n]) of PaiNN's Update"""
+    inner = torch.empty(rows, n, dtype=torch.float32, device=y.device)
+    cat = torch.empty(rows, 2 * n, dtype=torch.float32, device=y.device)
+    with KERNEL_TIMER.region("painn_update"):
+        check(lib().ld_painn_update_front(ptr(y), ptr(x_a), rows, n, ptr(inner), ptr(cat), stream_ptr(y.device)))
+    return inner, cat
+
+
+def painn_update_back(y, m, inner, x_a, x_v, rows, n):
+    """(scaled, base [rows, n]; the new x_v, shaped as x_v): the group norm of `scaled` plus `base` is the new x_a"""
+    require_cuda_f32(m, "m")
+    scaled, base = torch.empty_like(inner), torch.empty_like(inner)
+    out_v = torch.empty_like(x_v)
+    with KERNEL_TIMER.region("painn_update"):
+        check(lib().ld_painn_update_back(ptr(y), ptr(m), ptr(inner), ptr(x_a), ptr(x_v), rows, n, ptr(scaled), ptr(base), ptr(out_v),
+                                         stream_ptr(y.device)))
+    return scaled, base, out_v
+
+
 def painn_message_f32(row_ptr, dst, rij, mlp_dist, actv, x_v, rmax, eps=0.1, radial_kind=RADIAL_PAINN, res_a=None,
                       res_v=None, edge_counter=None):
     """Fused PaiNN message; returns (out_a [Nt,n], out_v [Nt,n,3]). actv = mlp_actv(x_a) as [Nt,4n]."""

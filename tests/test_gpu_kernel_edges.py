@@ -225,3 +225,56 @@ def test_radius_graph_build_paths(batch, nodes, box, cutoff):
     assert torch.equal(got["rij"].cpu()[mine], oracle["rij"][ref])
     assert torch.equal(G.unpack_shift(got["shift"]).cpu()[mine], oracle["shift"][ref].int())
     assert bool((s[1:] >= s[:-1]).all()) and E == len(src)
+
+
+# 4, 8 or 16 rows per block with the line at 592 and 1184 rows; widths that leave threads over (192, 40) and the widest
+@pytest.mark.parametrize("rows", [1, 5, 593, 1185, 2371])
+@pytest.mark.parametrize("k0,n1,n2,n3,direct", [(64, 256, 256, 256, False), (128, 192, 192, 192, False), (7, 40, 8, 24, True), (512, 512, 512, 512, True)])
+def test_mlp_rows_tiles(rows, k0, n1, n2, n3, direct):
+    from ld_b200 import ops
+    torch.manual_seed(rows + k0)
+    lin = [torch.nn.Linear(a, b) for a, b in ((k0, n1), (n1, n2), (n2, n3))]
+    d = torch.nn.Linear(k0, n3, bias=False) if direct else None
+    x = torch.randn(rows, k0)
+    y = ops.mlp3_rows(x.cuda(), ops.PackedMLP([l.cuda() for l in lin], None if d is None else d.cuda())).cpu().double()
+    W = [(l.weight.detach().cpu().double(), l.bias.detach().cpu().double()) for l in lin]
+    silu = torch.nn.functional.silu
+    # first-order propagation of |error| <= (terms + 4) u (sum of sizes) through each layer (SiLU's slope is at most 1.1)
+    h, e = x.double(), torch.zeros(rows, k0, dtype=torch.float64)
+    for i, (w, b) in enumerate(W):
+        size = h.abs() @ w.abs().t() + b.abs()
+        e = e @ w.abs().t() + (w.shape[1] + 4) * U * size
+        h = h @ w.t() + b
+        if i < 2:
+            h, e = silu(h), 1.1 * e + 4 * U * h.abs()
+    if d is not None:
+        wd = d.weight.detach().cpu().double()
+        h, e = h + x.double() @ wd.t(), e + (k0 + w.shape[1] + 4) * U * (x.double().abs() @ wd.abs().t() + size)
+    assert bool(((y - h).abs() <= e).all())
+
+
+@pytest.mark.parametrize("n,batch,nodes", [(32, 1, 3), (64, 8, 64), (24, 2, 35)])
+def test_painn_update_in_its_residual_form(n, batch, nodes):
+    """the fused form against the module's own formula in 64 bits"""
+    from ld_b200 import painn
+    torch.manual_seed(n)
+    m = painn.Update(n).cuda()
+    x_a, x_v = torch.randn(batch, nodes, n).cuda(), torch.randn(batch, nodes, n, 3).cuda()
+    p = {k: v.detach().double() for k, v in m.state_dict().items()}
+    mix = lambda k: torch.einsum("oi,bnix->bnox", p[k], x_v.double())  # noqa: E731
+    left, right = mix("lin_l.W"), mix("lin_r.W")
+    y = torch.cat([x_a.double(), right.norm(dim=-1)], dim=-1)
+    for k in (0, 2, 4):
+        y = y @ p[f"mlp.layers.{k}.weight"].t() + p[f"mlp.layers.{k}.bias"]
+        y = torch.nn.functional.silu(y) if k < 4 else y
+    d_v = mix("lin_v.W") * y[..., :n, None]
+    h = ((left * right).sum(-1) * y[..., n:2 * n]).reshape(batch, nodes, 4, n // 4)
+    h = h - h.mean([1, 3], keepdim=True)
+    h = (h / torch.sqrt(1 + (h ** 2).mean([1, 3], keepdim=True))).reshape(batch, nodes, n)
+    want = x_a.double() + p["gn.beta"] + p["gn.gamma"] * h + y[..., 2 * n:], x_v.double() + d_v / torch.sqrt(1 + (d_v ** 2).sum(-1, keepdim=True))
+    with torch.no_grad():
+        got = m.residual(x_a, x_v)
+        parts = m(x_a, x_v)
+    for g, w, d, x in zip(got, want, parts, (x_a, x_v)):
+        off = float((g.double() - w).norm() / w.norm())
+        assert off <= 1.5 * float(((x + d).double() - w).norm() / w.norm()) + 2 * U, off   # not further off than the separate operations
