@@ -35,6 +35,10 @@ struct Shape {
   static constexpr int PLANE = (N / 8) * PANEL;
   static constexpr int ACT = 2 * PLANE;               // also the FP32 products [N][NE + 1]
   static constexpr int SLOTS = 2 * MB;                // accumulators of NE columns in tensor memory
+  // weight slabs in the ring. A warp that waits for a slab has to know that the one before it in the same stage has landed, or
+  // the parity it waits for means nothing: with four blocks the stages are even in number, so that both are its own; with
+  // fewer, the wait for the accumulators says so.
+  static constexpr int STAGES = MB == 4 ? 4 : 5;
   static constexpr int G = WORK_THREADS / n;          // threads per channel in the message phase
   static_assert(N * (NE + 1) * 4 <= ACT, "the products reuse the activation planes");
   static_assert(G * EPT == NE, "the message phase covers the tile");
@@ -70,7 +74,7 @@ template <int MB>
 __global__ void __launch_bounds__(THREADS, 1)
 painn_message_split_kernel(const __grid_constant__ SplitParams P) {
   using S = Shape<MB>;
-  constexpr int N = S::N, n = S::n, NE = S::NE, SLOTS = S::SLOTS;
+  constexpr int N = S::N, n = S::n, NE = S::NE, SLOTS = S::SLOTS, STAGES = S::STAGES;
   extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ __align__(8) uint64_t bar_full[STAGES], bar_empty[STAGES], bar_done[SLOTS], bar_taken[2];
   __shared__ uint32_t tmem_slot;
