@@ -228,6 +228,15 @@ int ld_painn_message_bf16_tc(const int* row_ptr, const int* dst, const float* ri
                              const void* w3p, const float* b3, const float* actv, const float* x_v, const void* gather16,
                              const float* res_a, const float* res_v, float* out_a, float* out_v, long long* edge_counter,
                              int* status_dev, void* stream);
+/* ld_painn_message_bf16_slabs: the same for n = 32, 64, 128 with the weights as slabs in streaming order (ld_painn_pack_slabs_bf16,
+ * N * (K rounded up to 16) BF16 values each) and the neighbours' features read in FP32. */
+int ld_painn_pack_slabs_bf16(const float* W, long long sw0, long long sw1, int N, int K, void* out, void* stream);
+int ld_painn_message_bf16_slabs(const int* row_ptr, const int* dst, const float* rij, int Nt, int n, int n_rbf, int radial_kind,
+                                float rmax, float eps, const void* w1s, const float* b1, const void* w2s, const float* b2,
+                                const void* w3s, const float* b3, const float* actv, const float* x_v, const float* res_a,
+                                const float* res_v, float* out_a, float* out_v, long long* edge_counter, int* status_dev,
+                                void* stream);
+
 
 /* ---- fused l<=2 message layer ------------------------------------------------------------------------
  * Messages.forward (archs/diffuser_atoms15.py:227-253) without edge-sized tensors: the radial

@@ -4,7 +4,7 @@
 // What bounds it: the shared-memory port. The two 4n x 4n layers are 3 x 2 x (4n)^2 flops an edge on the tensor cores; an MMA
 // of 128 x 64 x 16 (n = 128) takes 48 cycles, the time to read its 6 KB of operands, not the 32 of the tensor pipe, and the
 // weight slabs (2 MB per tile) come in through the same port: 433 cycles a slab of six MMAs measured, 416 by that count.
-// n = 128, 8 radial functions, 562 k edges: 2.97 ms, against 22.8 ms on the FMA pipe (painn_message.cu); n = 64, 11 k edges:
+// n = 128, 8 radial functions, 562 k edges: 3.06 ms, against 22.8 ms on the FMA pipe (painn_message.cu); n = 64, 11 k edges:
 // 68 us against 195. Error against 64 bits: 6.1e-7, against 7.5e-7.
 //
 // A block owns a node-aligned, contiguous slice of the CSR and walks it 256 / (n / 32) edges at a time. Roles:

@@ -71,6 +71,8 @@ SIGNATURES = {
     "ld_bee_split_pack": [P, P, P, P, P, P, P, I, I, P, P, P],
     "ld_bee_rows13_f32": [P, P, P, LL, I, P, P],
     "ld_bee_messages_scalar_f32_split": [P, P, P, I, I, I, F, P, P, P, P, P, P, P, P, P, F, P, P, P],
+    "ld_painn_pack_slabs_bf16": [P, LL, LL, I, I, P, P],
+    "ld_painn_message_bf16_slabs": [P, P, P, I, I, I, I, F, F, P, P, P, P, P, P, P, P, P, P, P, P, P, P, P],
     "ld_painn_update_front": [P, P, LL, I, P, P, P],
     "ld_painn_update_back": [P, P, P, P, P, LL, I, P, P, P, P],
     "ld_painn_split_elems": [I, I, P],

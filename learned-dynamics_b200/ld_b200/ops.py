@@ -249,6 +249,7 @@ class PackedMLP:
         self._linears = (l1, l2, l3)
         self._bf16 = None
         self._split = None
+        self._slabs = None
         self.Wt = [l.weight.detach().t().contiguous().float() for l in (l1, l2, l3)]
         self.b = [None if l.bias is None else l.bias.detach().contiguous().float() for l in (l1, l2, l3)]
         self.dims = (l1.weight.shape[1], l1.weight.shape[0], l2.weight.shape[0], l3.weight.shape[0])
@@ -277,6 +278,20 @@ def _packed_split(mlp, n):
                                             ptr(packed), ptr(scales), stream_ptr(dev)))
             mlp._split = (packed, scales)
     return mlp._split or None
+
+
+def _packed_slabs(mlp):
+    """BF16 weights of a distance MLP in the slab order of ld_painn_message_bf16_slabs (built on first use)"""
+    if mlp._slabs is None:
+        slabs = []
+        for l in mlp._linears:
+            W = l.weight.detach().float()
+            N, K = W.shape
+            out = torch.empty(N * ((K + 15) // 16 * 16), dtype=torch.bfloat16, device=W.device)
+            check(lib().ld_painn_pack_slabs_bf16(ptr(W), W.stride(0), W.stride(1), N, K, ptr(out), stream_ptr(W.device)))
+            slabs.append(out)
+        mlp._slabs = slabs
+    return mlp._slabs
 
 
 def mlp3_rows(x, mlp, act=ACT_SILU):
@@ -495,6 +510,16 @@ def painn_message_bf16_tc(row_ptr, dst, rij, mlp_dist, actv, x_v, rmax, eps=0.1,
         raise RuntimeError("painn_message: widths must be n_rbf -> 4n -> 4n -> 4n and actv [Nt,4n]")
     if dst.dtype != torch.int32 or row_ptr.dtype != torch.int32:
         raise RuntimeError("painn_message: row_ptr and dst must be int32")
+    if n in (32, 64, 128) and n_rbf <= 4 * n and all(b is not None for b in mlp_dist.b):
+        w = _packed_slabs(mlp_dist)
+        out_a = torch.empty(Nt, n, dtype=torch.float32, device=x_v.device)
+        out_v = torch.empty(Nt, n, 3, dtype=torch.float32, device=x_v.device)
+        with KERNEL_TIMER.region("painn_message_tc"):
+            check(lib().ld_painn_message_bf16_slabs(ptr(row_ptr), ptr(dst), ptr(rij), Nt, n, n_rbf, radial_kind, float(rmax), float(eps),
+                                                    ptr(w[0]), ptr(mlp_dist.b[0]), ptr(w[1]), ptr(mlp_dist.b[1]), ptr(w[2]),
+                                                    ptr(mlp_dist.b[2]), ptr(actv), ptr(x_v), ptr(res_a), ptr(res_v), ptr(out_a), ptr(out_v),
+                                                    ptr(edge_counter), ptr(tc_status(x_v.device)), stream_ptr(x_v.device)))
+        return out_a, out_v
     w = _packed_bf16(mlp_dist)
     out_a = torch.empty(Nt, n, dtype=torch.float32, device=x_v.device)
     out_v = torch.empty(Nt, n, 3, dtype=torch.float32, device=x_v.device)

@@ -106,6 +106,45 @@ def test_split_message_is_as_exact_as_the_fma_kernel(n, n_rbf, radial, degrees, 
         off = lambda t: float((t.cpu().double() - w).norm())  # noqa: E731
         assert off(a) <= 1.2 * off(b) + U * float(w.norm()), (off(a) / float(w.norm()), off(b) / float(w.norm()))
 
+# tiles of 128 edges, at n = 128 taken in two passes of 64; slabs K = 64: input widths around them, nodes without edges and
+# nodes that span tiles, one edge in the last tile
+@pytest.mark.parametrize("n,n_rbf,radial,degrees", [(32, 1, 1, "one"), (32, 128, 0, "long"), (64, 65, 0, "mixed"), (64, 16, 1, "long"),
+                                                    (128, 8, 1, "mixed"), (128, 80, 0, "long"), (128, 16, 1, "none")])
+def test_bf16_slab_message_against_the_edge_major_kernel(n, n_rbf, radial, degrees):
+    """both BF16 kernels against 64 bits: the slab kernel (which reads the features in FP32) may not be further off, plus one
+    rounding to BF16 of what is summed"""
+    import ctypes
+    from ld_b200 import ops
+    from ld_b200._lib import lib, check, ptr, stream_ptr
+    g = torch.Generator().manual_seed(n + n_rbf)
+    deg = {"one": torch.tensor([0, 0, 1, 0]), "none": torch.zeros(5, dtype=torch.int64),
+           "mixed": torch.randint(0, 40, (61,), generator=g), "long": torch.tensor([3, 0, 700, 1, 0, 0, 64, 257, 129, 1])}[degrees]
+    Nt, E = len(deg), int(deg.sum())
+    row_ptr = torch.cat([torch.zeros(1, dtype=torch.int64), deg.cumsum(0)]).int()
+    dst = torch.randint(0, Nt, (E,), generator=g).int()
+    rij = torch.randn(E, 3, generator=g) * 1.3
+    torch.manual_seed(n)
+    lin = [torch.nn.Linear(k, 4 * n) for k in (n_rbf, 4 * n, 4 * n)]
+    actv, x_v = torch.randn(Nt, 4 * n, generator=g), torch.randn(Nt, n, 3, generator=g)
+    want = _message64(row_ptr, dst, rij, [(l.weight.detach(), l.bias.detach()) for l in lin], actv, x_v, radial, n_rbf, 4.0)
+    mlp = ops.PackedMLP([l.cuda() for l in lin])
+    args = [t.cuda() for t in (row_ptr, dst, rij)]
+    actv, x_v = actv.cuda(), x_v.cuda()
+    count = torch.zeros(1, dtype=torch.int64, device="cuda")
+    res = torch.randn(Nt, n, generator=g).cuda(), torch.randn(Nt, n, 3, generator=g).cuda()
+    slabs = ops.painn_message_bf16_tc(*args, mlp, actv, x_v, 4.0, radial_kind=radial, edge_counter=count)
+    added = ops.painn_message_bf16_tc(*args, mlp, actv, x_v, 4.0, radial_kind=radial, res_a=res[0], res_v=res[1])
+    assert mlp._slabs and int(count) == E and int(ops.tc_status(actv.device)) == 0
+    w = ops._packed_bf16(mlp)
+    old = torch.empty(Nt, n, device="cuda"), torch.empty(Nt, n, 3, device="cuda")
+    check(lib().ld_painn_message_bf16_tc(*[ptr(a) for a in args], Nt, n, n_rbf, radial, ctypes.c_float(4.0), ctypes.c_float(0.1), ptr(w[0]),
+                                         ptr(mlp.b[0]), ptr(w[1]), ptr(mlp.b[1]), ptr(w[2]), ptr(mlp.b[2]), ptr(actv), ptr(x_v), None, None,
+                                         None, ptr(old[0]), ptr(old[1]), None, ptr(ops.tc_status(actv.device)), stream_ptr()))
+    for w64, a, b, r, ar in zip(want, slabs, old, res, added):
+        off = lambda t: float((t.cpu().double() - w64).norm())  # noqa: E731
+        assert off(a) <= 1.2 * off(b) + 2.0 ** -9 * float(w64.norm()), (off(a) / float(w64.norm()), off(b) / float(w64.norm()))
+        assert torch.equal(ar, a + r)
+
 
 # tiles of 64 edges, groups of 16: nodes without edges, nodes that span tiles, one edge in the last tile; both widths of
 # either kind of channel; sizes of the features that move the scales of the operands, one edge far above the others
