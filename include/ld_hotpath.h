@@ -135,9 +135,11 @@ int ld_cow_o1_bw(int left, const float* o0, const float* o1, const float* g011, 
 int ld_mlp3_rows(const float* x, long long rows, int k0, const float* W1t, const float* b1, int n1, const float* W2t,
                  const float* b2, int n2, const float* W3t, const float* b3, int n3, int act, const float* Wdt,
                  float* out, void* stream);
-/* The pointwise halves of PaiNN's Update (archs/meanflow_painn8.py:53-75) around its MLP, on rows of n channels; y [rows][3n][3]
- * = (lin_l | lin_r | lin_v) of x_v. Front: inner = l . r, cat = (x_a | |r|). Back, with m [rows][3n] the MLP's output: out_v =
+/* PaiNN's Update (archs/meanflow_painn8.py:53-75) on rows of n channels. Mix: y [rows][3n][3] = (lin_l | lin_r | lin_v) of x_v, from
+ * three contiguous [n][n] weights. The pointwise halves around the update's MLP follow. Front: inner = l . r, cat = (x_a | |r|). Back, with m [rows][3n] the MLP's output: out_v =
  * x_v + u / sqrt(1 + |u|^2), u = v m[:n]; scaled = inner m[n:2n] (to be normalised), base = x_a + m[2n:]. */
+int ld_painn_update_mix(const float* W_l, const float* W_r, const float* W_v, const float* x_v, long long rows, int n, float* y,
+                        void* stream);
 int ld_painn_update_front(const float* y, const float* x_a, long long rows, int n, float* inner, float* cat, void* stream);
 int ld_painn_update_back(const float* y, const float* m, const float* inner, const float* x_a, const float* x_v, long long rows,
                          int n, float* scaled, float* base, float* out_v, void* stream);

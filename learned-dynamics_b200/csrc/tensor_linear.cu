@@ -63,10 +63,12 @@ struct TlTile {
   static constexpr size_t BYTES = TL_STAGES * sizeof(float) * STAGE;
 };
 
-template <int S, int TY, int OU, int NR, int VEC>
+// W[o, i] at w[0] + o * sw0 + i * sw1; a stack of three matrices (PARTS = 3) has `part` outputs in each of w[0], w[1], w[2]
+struct TlWeights { const float* w[3]; long long sw0, sw1; int part; };
+
+template <int S, int TY, int OU, int NR, int VEC, int PARTS>
 __global__ void __launch_bounds__(TL_THREADS, 2)
-tensor_linear_kernel(const float* __restrict__ W, long long sw0, long long sw1, const float* __restrict__ x,
-                     float* __restrict__ y, long long rows, int I, int O) {
+tensor_linear_kernel(const TlWeights W, const float* __restrict__ x, float* __restrict__ y, long long rows, int I, int O) {
   using T = TlTile<S, TY, OU, NR>;
   constexpr int KC = T::KC, PITCH = T::PITCH, TX = T::TX, TO = T::TO, TR = T::TR, WP = T::WP;
   extern __shared__ __align__(16) float smem[];
@@ -86,9 +88,15 @@ tensor_linear_kernel(const float* __restrict__ W, long long sw0, long long sw1, 
     tl_rows<VEC, TR, KC * S, PITCH>(xs, x + (r0 * I + i0) * S, (long long)I * S, rcnt, min(KC, I - i0) * S);
     for (int idx = tid; idx < KC * TO; idx += TL_THREADS) {
       // lanes run along whichever index of W is the contiguous one
-      const int kc = sw1 == 1 ? idx % KC : idx / TO, o = sw1 == 1 ? idx / KC : idx % TO;
+      const int kc = W.sw1 == 1 ? idx % KC : idx / TO, o = W.sw1 == 1 ? idx / KC : idx % TO;
       const bool ok = i0 + kc < I && o0 + o < O;
-      tl_cp<1>(ws + kc * WP + o, ok ? W + (long long)(o0 + o) * sw0 + (long long)(i0 + kc) * sw1 : W, ok);
+      const float* w = W.w[0];
+      int row = o0 + o;
+      if (PARTS == 3) {
+        if (row >= 2 * W.part) { w = W.w[2]; row -= 2 * W.part; }
+        else if (row >= W.part) { w = W.w[1]; row -= W.part; }
+      }
+      tl_cp<1>(ws + kc * WP + o, ok ? w + row * W.sw0 + (i0 + kc) * W.sw1 : w, ok);
     }
     tl_commit();
   };
@@ -288,35 +296,35 @@ int dw_splits(int inds, long long rows, int I, int O) {
   return (int)want;
 }
 
-template <int S, int TY, int OU, int NR, int VEC>
-int tl_run(const float* W, long long sw0, long long sw1, const float* x, float* y, long long rows, int I, int O, cudaStream_t st) {
+template <int S, int TY, int OU, int NR, int VEC, int PARTS>
+int tl_run(const TlWeights& W, const float* x, float* y, long long rows, int I, int O, cudaStream_t st) {
   using T = TlTile<S, TY, OU, NR>;
   if (T::BYTES > 48 * 1024)
-    LD_CUDA_TRY(cudaFuncSetAttribute(tensor_linear_kernel<S, TY, OU, NR, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::BYTES));
+    LD_CUDA_TRY(cudaFuncSetAttribute(tensor_linear_kernel<S, TY, OU, NR, VEC, PARTS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::BYTES));
   const dim3 g((unsigned)((rows + T::TR - 1) / T::TR), ld_cdiv(O, T::TO));
-  tensor_linear_kernel<S, TY, OU, NR, VEC><<<g, TL_THREADS, T::BYTES, st>>>(W, sw0, sw1, x, y, rows, I, O);
+  tensor_linear_kernel<S, TY, OU, NR, VEC, PARTS><<<g, TL_THREADS, T::BYTES, st>>>(W, x, y, rows, I, O);
   LD_LAUNCH_CHECK();
   return LD_OK;
 }
 
-template <int S, int TY, int OU, int NR>
-int tl_launch(const float* W, long long sw0, long long sw1, const float* x, float* y, long long rows, int I, int O, cudaStream_t st) {
+template <int S, int TY, int OU, int NR, int PARTS>
+int tl_launch(const TlWeights& W, const float* x, float* y, long long rows, int I, int O, cudaStream_t st) {
   // 8-byte copies need even rows of x on an 8-byte boundary
-  if (I % 2 == 0 && ((uintptr_t)x & 7) == 0) return tl_run<S, TY, OU, NR, 2>(W, sw0, sw1, x, y, rows, I, O, st);
-  return tl_run<S, TY, OU, NR, 1>(W, sw0, sw1, x, y, rows, I, O, st);
+  if (I % 2 == 0 && ((uintptr_t)x & 7) == 0) return tl_run<S, TY, OU, NR, 2, PARTS>(W, x, y, rows, I, O, st);
+  return tl_run<S, TY, OU, NR, 1, PARTS>(W, x, y, rows, I, O, st);
 }
 
 // Which tile: 8 outputs x 6 to 9 columns per thread, as many outputs per block as there are (32, 64 or 128) and the rest of
 // the threads along the rows, so that x is read once. Where that leaves SMs without a block, tiles of 32 outputs and a
 // quarter of the columns (twice the shared loads per FMA, but up to sixteen times the blocks).
-template <int S, int NR, int NR_SMALL>
-int tl_pick(const float* W, long long sw0, long long sw1, const float* x, float* y, long long rows, int I, int O, cudaStream_t st) {
+template <int S, int NR, int NR_SMALL, int PARTS = 1>
+int tl_pick(const TlWeights& W, const float* x, float* y, long long rows, int I, int O, cudaStream_t st) {
   const int tr = O <= 32 ? TlTile<S, 4, 8, NR>::TR : (O <= 64 ? TlTile<S, 8, 8, NR>::TR : TlTile<S, 16, 8, NR>::TR);
   const long long blocks = (rows + tr - 1) / tr * (O <= 128 ? 1 : ld_cdiv(O, 128));
-  if (blocks < 148) return tl_launch<S, 16, 2, NR_SMALL>(W, sw0, sw1, x, y, rows, I, O, st);
-  if (O <= 32) return tl_launch<S, 4, 8, NR>(W, sw0, sw1, x, y, rows, I, O, st);
-  if (O <= 64) return tl_launch<S, 8, 8, NR>(W, sw0, sw1, x, y, rows, I, O, st);
-  return tl_launch<S, 16, 8, NR>(W, sw0, sw1, x, y, rows, I, O, st);
+  if (blocks < 148) return tl_launch<S, 16, 2, NR_SMALL, PARTS>(W, x, y, rows, I, O, st);
+  if (O <= 32) return tl_launch<S, 4, 8, NR, PARTS>(W, x, y, rows, I, O, st);
+  if (O <= 64) return tl_launch<S, 8, 8, NR, PARTS>(W, x, y, rows, I, O, st);
+  return tl_launch<S, 16, 8, NR, PARTS>(W, x, y, rows, I, O, st);
 }
 
 template <int S, int TO, int TI, int VEC>
@@ -359,9 +367,19 @@ extern "C" int ld_tensor_linear(int inds, const float* W, long long sw0, long lo
   if (rows < 0 || dim_in < 0 || dim_out < 0) return LD_ERR_SHAPE;
   if (rows == 0 || dim_out == 0) return LD_OK;
   cudaStream_t st = (cudaStream_t)stream;
-  if (inds == 0) return tl_pick<1, 8, 2>(W, sw0, sw1, x, y, rows, dim_in, dim_out, st);
-  if (inds == 1) return tl_pick<3, 2, 1>(W, sw0, sw1, x, y, rows, dim_in, dim_out, st);
-  return tl_pick<9, 1, 1>(W, sw0, sw1, x, y, rows, dim_in, dim_out, st);
+  const TlWeights Ws{{W, W, W}, sw0, sw1, dim_out};
+  if (inds == 0) return tl_pick<1, 8, 2>(Ws, x, y, rows, dim_in, dim_out, st);
+  if (inds == 1) return tl_pick<3, 2, 1>(Ws, x, y, rows, dim_in, dim_out, st);
+  return tl_pick<9, 1, 1>(Ws, x, y, rows, dim_in, dim_out, st);
+}
+
+// The three channel mixings of PaiNN's Update in one launch, the weights read where they lie: y [rows][3n][3] = (W_l x | W_r x |
+// W_v x) for x_v [rows][n][3] and contiguous [n][n] weights.
+extern "C" int ld_painn_update_mix(const float* W_l, const float* W_r, const float* W_v, const float* x_v, long long rows, int n, float* y,
+                                   void* stream) {
+  if (rows < 0 || n <= 0 || n > 0x7fffffff / 3) return LD_ERR_SHAPE;
+  if (rows == 0) return LD_OK;
+  return tl_pick<3, 2, 1, 3>(TlWeights{{W_l, W_r, W_v}, n, 1, n}, x_v, y, rows, n, 3 * n, (cudaStream_t)stream);
 }
 
 extern "C" int ld_tensor_linear_dw_workspace(int inds, long long rows, int dim_in, int dim_out, size_t* bytes) {

@@ -73,6 +73,7 @@ SIGNATURES = {
     "ld_bee_messages_scalar_f32_split": [P, P, P, I, I, I, F, P, P, P, P, P, P, P, P, P, F, P, P, P],
     "ld_painn_pack_slabs_bf16": [P, LL, LL, I, I, P, P],
     "ld_painn_message_bf16_slabs": [P, P, P, I, I, I, I, F, F, P, P, P, P, P, P, P, P, P, P, P, P, P, P, P],
+    "ld_painn_update_mix": [P, P, P, P, LL, I, P, P],
     "ld_painn_update_front": [P, P, LL, I, P, P, P],
     "ld_painn_update_back": [P, P, P, P, P, LL, I, P, P, P, P],
     "ld_painn_split_elems": [I, I, P],

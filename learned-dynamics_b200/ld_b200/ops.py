@@ -309,6 +309,19 @@ def mlp3_rows(x, mlp, act=ACT_SILU):
     return out
 
 
+def painn_update_mix(W_l, W_r, W_v, x_v, rows, n):
+    """y [rows, 3n, 3] = the three channel mixings of x_v, stacked; the weights (contiguous float32 [n, n]) are read in place"""
+    require_cuda_f32(x_v, "x_v")
+    for W in (W_l, W_r, W_v):
+        require_cuda_f32(W, "W")
+        if tuple(W.shape) != (n, n):
+            raise RuntimeError("painn_update_mix: weights must be [n, n]")
+    y = torch.empty(rows, 3 * n, 3, dtype=torch.float32, device=x_v.device)
+    with KERNEL_TIMER.region("tensor_linear"):
+        check(lib().ld_painn_update_mix(ptr(W_l), ptr(W_r), ptr(W_v), ptr(x_v), rows, n, ptr(y), stream_ptr(x_v.device)))
+    return y
+
+
 def painn_update_front(y, x_a, rows, n):
     """y [rows, 3n, 3] = the stacked mixings of x_v: (inner [rows, n], cat [rows, 2n]) of PaiNN's Update"""
     inner = torch.empty(rows, n, dtype=torch.float32, device=y.device)

@@ -92,22 +92,18 @@ class Update(nn.Module):
         self.mlp = MLP(2 * n, 3 * n)
         assert n % 4 == 0
         self.gn = ScalGroupNorm(n, 4, epsilon=1.)
-        self._cat, self._cat_key = None, None
 
     def residual(self, x_a, x_v):
-        """x_a + dx_a, x_v + dx_v. Without autograd: the three channel mixings as one, and what is pointwise around the MLP
-        and the norm as two kernels instead of some twenty."""
+        """x_a + dx_a, x_v + dx_v. Without autograd: the three channel mixings as one launch on the weights as they are, and
+        what is pointwise around the MLP and the norm as two kernels instead of some twenty."""
         lins = (self.lin_l, self.lin_r, self.lin_v)
         if (torch.is_grad_enabled() or not x_a.is_cuda or x_a.dim() != 3 or x_a.dtype != torch.float32 or x_v.dtype != torch.float32
-                or any(l.precision != "fp32" for l in lins)):
+                or any(l.precision != "fp32" or l.W.dtype != torch.float32 or not l.W.is_contiguous() for l in lins)):
             dx_a, dx_v = self.forward(x_a, x_v)
             return x_a + dx_a, x_v + dx_v
-        key = tuple((l.W.data_ptr(), l.W._version) for l in lins)
-        if self._cat_key != key:
-            self._cat, self._cat_key = torch.cat([l.W.detach() for l in lins], dim=0).float().contiguous(), key
         n, rows = self.n, x_a.shape[0] * x_a.shape[1]
         x_a, x_v = x_a.contiguous(), x_v.contiguous()
-        y = ops.tensor_linear_fwd(1, self._cat, x_v.reshape(rows, n, 3))
+        y = ops.painn_update_mix(self.lin_l.W, self.lin_r.W, self.lin_v.W, x_v, rows, n)
         inner, cat = ops.painn_update_front(y, x_a, rows, n)
         scaled, base, out_v = ops.painn_update_back(y, self.mlp(cat), inner, x_a, x_v, rows, n)
         return self.gn(scaled.reshape(x_a.shape), residual=base.reshape(x_a.shape)), out_v

@@ -317,3 +317,19 @@ def test_painn_update_in_its_residual_form(n, batch, nodes):
     for g, w, d, x in zip(got, want, parts, (x_a, x_v)):
         off = float((g.double() - w).norm() / w.norm())
         assert off <= 1.5 * float(((x + d).double() - w).norm() / w.norm()) + 2 * U, off   # not further off than the separate operations
+
+
+def test_painn_update_reads_its_mixing_weights_in_every_call():
+    """writes that autograd's version counter does not see (.data, another tensor at the same place) take effect at once"""
+    from ld_b200 import painn
+    torch.manual_seed(4)
+    m = painn.Update(32).cuda()
+    x_a, x_v = torch.randn(2, 17, 32).cuda(), torch.randn(2, 17, 32, 3).cuda()
+    with torch.no_grad():
+        m.residual(x_a, x_v)
+        for name in ("lin_l", "lin_r", "lin_v"):
+            getattr(m, name).W.data.mul_(-1.7)
+            fresh = painn.Update(32).cuda()
+            fresh.load_state_dict(m.state_dict())
+            for a, b in zip(m.residual(x_a, x_v), fresh.residual(x_a, x_v)):
+                assert torch.equal(a, b), name
