@@ -248,8 +248,10 @@ int ld_painn_message_bf16_slabs(const int* row_ptr, const int* dst, const float*
  * caller applies them per node with ld_tensor_linear over 5*chan inputs). _scalar: per-edge Y maps
  * and mlp_a, summed per node. `jacobi` = 8x9 coefficients of the shifted Jacobi(1,0) polynomials.
  * feat_bf16: 0 = L0/L1/L2 FP32; 1 = BF16; 2 = L0 alone points to the interleaved BF16 form
- * [node][chan][16] = (l0, l1[3], l2[9], 3 unused) written by ld_linear_bf16_tc_out16.
- * out_bf16 (vd): S_v / S_d are stored as BF16 (same shapes), the input form of ld_linear_bf16_tc_in16. */
+ * [node][chan][16] = (l0, l1[3], l2[9], 3 unused) written by ld_linear_bf16_tc_out16;
+ * 3 (vd) = L0 alone points to the FP32 rows [node][13][chan] of ld_bee_rows13_f32.
+ * out_bf16 (vd): S_v / S_d are stored as BF16 (same shapes), the input form of ld_linear_bf16_tc_in16. With feat_bf16 = 3
+ * the sums are FP32, and out_bf16 is refused (LD_ERR_UNSUPPORTED). */
 int ld_bee_messages_vd_f32(const int* row_ptr, const int* dst, const float* rij, int Nt, int chan, float r0, const float* L0,
                            const float* L1, const float* L2, const float* enc_w, const float* enc_b, const float* jacobi,
                            float scale, void* S_v, void* S_d, int feat_bf16, int out_bf16, void* stream);

@@ -399,7 +399,7 @@ bee_scalar_kernel(BeeScalarParams P) {
 // [node][13][chan] of ld_bee_rows13_f32; enc_w [chan,8] / enc_b [chan] the radial read-in,
 // jacobi the 8x9 coefficient matrix of the radial basis. Graph in CSR form sorted by source.
 // out_bf16: S_v / S_d are stored as BF16, component-major ([Nt][3][5*chan] and [Nt][9][5*chan]), the input form of
-// ld_linear_bf16_tc_in16.
+// ld_linear_bf16_tc_in16 (not with feat_bf16 = 3).
 extern "C" int ld_bee_messages_vd_f32(const int* row_ptr, const int* dst, const float* rij, int Nt, int chan, float r0,
                                       const float* L0, const float* L1, const float* L2, const float* enc_w,
                                       const float* enc_b, const float* jacobi, float scale, void* S_v_, void* S_d_,
@@ -407,6 +407,7 @@ extern "C" int ld_bee_messages_vd_f32(const int* row_ptr, const int* dst, const 
   float* S_v = (float*)S_v_;
   float* S_d = (float*)S_d_;
   if (Nt < 0 || chan <= 0 || !(r0 > 0.f)) return LD_ERR_SHAPE;
+  if (feat_bf16 == 3 && out_bf16) { ld_set_last_message("bee messages: the sums of FP32 rows [node][13][chan] are FP32"); return LD_ERR_UNSUPPORTED; }
   if (Nt == 0) return LD_OK;
   int* next_node = nullptr;
   {

@@ -46,3 +46,6 @@ def test_argument_errors_without_gpu():
     rc = L.ld_radius_graph_workspace_size(2, 10, 0, 1.0, None, 1, 0, C.byref(n))
     assert rc == _lib.LD_ERR_SHAPE  # reference-compatible grid is periodic only
     assert L.ld_tensor_linear(3, None, 1, 1, None, None, 4, 4, 4, None) == _lib.LD_ERR_UNSUPPORTED
+    # the sums of the FP32 neighbour rows are FP32: a buffer sized for BF16 is refused, not overrun
+    rc = L.ld_bee_messages_vd_f32(None, None, None, 4, 64, C.c_float(5.0), None, None, None, None, None, None, C.c_float(0.1), None, None, 3, 1, None)
+    assert rc == _lib.LD_ERR_UNSUPPORTED
