@@ -309,9 +309,15 @@ def mlp3_rows(x, mlp, act=ACT_SILU):
     return out
 
 
+def _require_numel(t, name, numel):
+    require_cuda_f32(t, name)
+    if t.numel() != numel:
+        raise RuntimeError(f"{name}: {numel} elements expected, got {tuple(t.shape)}")
+
+
 def painn_update_mix(W_l, W_r, W_v, x_v, rows, n):
     """y [rows, 3n, 3] = the three channel mixings of x_v, stacked; the weights (contiguous float32 [n, n]) are read in place"""
-    require_cuda_f32(x_v, "x_v")
+    _require_numel(x_v, "x_v", rows * n * 3)
     for W in (W_l, W_r, W_v):
         require_cuda_f32(W, "W")
         if tuple(W.shape) != (n, n):
@@ -324,6 +330,8 @@ def painn_update_mix(W_l, W_r, W_v, x_v, rows, n):
 
 def painn_update_front(y, x_a, rows, n):
     """y [rows, 3n, 3] = the stacked mixings of x_v: (inner [rows, n], cat [rows, 2n]) of PaiNN's Update"""
+    _require_numel(y, "y", rows * 9 * n)
+    _require_numel(x_a, "x_a", rows * n)
     inner = torch.empty(rows, n, dtype=torch.float32, device=y.device)
     cat = torch.empty(rows, 2 * n, dtype=torch.float32, device=y.device)
     with KERNEL_TIMER.region("painn_update"):
@@ -333,7 +341,8 @@ def painn_update_front(y, x_a, rows, n):
 
 def painn_update_back(y, m, inner, x_a, x_v, rows, n):
     """(scaled, base [rows, n]; the new x_v, shaped as x_v): the group norm of `scaled` plus `base` is the new x_a"""
-    require_cuda_f32(m, "m")
+    for t, name, width in ((y, "y", 9 * n), (m, "m", 3 * n), (inner, "inner", n), (x_a, "x_a", n), (x_v, "x_v", 3 * n)):
+        _require_numel(t, name, rows * width)
     scaled, base = torch.empty_like(inner), torch.empty_like(inner)
     out_v = torch.empty_like(x_v)
     with KERNEL_TIMER.region("painn_update"):

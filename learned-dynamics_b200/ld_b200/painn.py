@@ -98,6 +98,7 @@ class Update(nn.Module):
         what is pointwise around the MLP and the norm as two kernels instead of some twenty."""
         lins = (self.lin_l, self.lin_r, self.lin_v)
         if (torch.is_grad_enabled() or not x_a.is_cuda or x_a.dim() != 3 or x_a.dtype != torch.float32 or x_v.dtype != torch.float32
+                or x_a.shape[2] != self.n or x_v.shape != (*x_a.shape, 3) or x_v.device != x_a.device   # (what does not fit is refused there)
                 or any(l.precision != "fp32" or l.W.dtype != torch.float32 or not l.W.is_contiguous() for l in lins)):
             dx_a, dx_v = self.forward(x_a, x_v)
             return x_a + dx_a, x_v + dx_v

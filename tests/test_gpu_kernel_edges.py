@@ -333,3 +333,18 @@ def test_painn_update_reads_its_mixing_weights_in_every_call():
             fresh.load_state_dict(m.state_dict())
             for a, b in zip(m.residual(x_a, x_v), fresh.residual(x_a, x_v)):
                 assert torch.equal(a, b), name
+
+
+# too few channels or nodes for the layer, axes in another order: refused, as by the module's separate operations
+@pytest.mark.parametrize("a,v", [((2, 17, 16), (2, 17, 32, 3)), ((2, 17, 32), (2, 17, 16, 3)), ((2, 17, 32), (2, 16, 32, 3)),
+                                 ((2, 17, 32), (17, 2, 32, 3)), ((2, 17, 32), (2, 17, 3, 32))])
+def test_painn_update_refuses_what_does_not_fit(a, v):
+    from ld_b200 import ops, painn
+    m = painn.Update(32).cuda()
+    with torch.no_grad(), pytest.raises(RuntimeError):
+        m.residual(torch.zeros(a).cuda(), torch.zeros(v).cuda())
+    y, row = torch.zeros(34, 96, 3).cuda(), torch.zeros(34, 32).cuda()
+    with pytest.raises(RuntimeError):
+        ops.painn_update_front(y, row[:33], 34, 32)
+    with pytest.raises(RuntimeError):
+        ops.painn_update_back(y, row, row, row, y[:, :32].contiguous(), 34, 32)
