@@ -14,6 +14,7 @@ import math
 
 import torch
 import torch.nn as nn
+from torch.nn.modules import module as nn_module
 
 from . import ops
 from .graph_layers import Graph, edges_read, edges_read_dst, edges_reduce_src, boxwrap
@@ -82,6 +83,11 @@ class ScalGroupNorm(nn.Module):
         return ans if residual is None else residual + ans
 
 
+def _as_built(m, cls):
+    """m is a plain `cls`, with nothing registered or replaced that a call of it would run"""
+    return type(m) is cls and not m._forward_hooks and not m._forward_pre_hooks and "forward" not in vars(m)
+
+
 class Update(nn.Module):
     def __init__(self, n):
         super().__init__()
@@ -93,14 +99,19 @@ class Update(nn.Module):
         assert n % 4 == 0
         self.gn = ScalGroupNorm(n, 4, epsilon=1.)
 
+    def _fusable(self):
+        return (_as_built(self, Update) and all(_as_built(l, TensLinear) and l.inds == 1 for l in (self.lin_l, self.lin_r, self.lin_v))
+                and _as_built(self.mlp, MLP) and _as_built(self.gn, ScalGroupNorm)
+                and not nn_module._global_forward_hooks and not nn_module._global_forward_pre_hooks)
+
     def residual(self, x_a, x_v):
         """x_a + dx_a, x_v + dx_v. Without autograd: the three channel mixings as one launch on the weights as they are, and
-        what is pointwise around the MLP and the norm as two kernels instead of some twenty."""
+        what is pointwise around the MLP and the norm as two kernels instead of some twenty; not where hooks or replaced parts want to see the separate calls."""
         lins = (self.lin_l, self.lin_r, self.lin_v)
-        if (torch.is_grad_enabled() or not x_a.is_cuda or x_a.dim() != 3 or x_a.dtype != torch.float32 or x_v.dtype != torch.float32
+        if (torch.is_grad_enabled() or not x_a.is_cuda or not self._fusable() or x_a.dim() != 3 or x_a.dtype != torch.float32 or x_v.dtype != torch.float32
                 or x_a.shape[2] != self.n or x_v.shape != (*x_a.shape, 3) or x_v.device != x_a.device   # (what does not fit is refused there)
                 or any(l.precision != "fp32" or l.W.dtype != torch.float32 or not l.W.is_contiguous() for l in lins)):
-            dx_a, dx_v = self.forward(x_a, x_v)
+            dx_a, dx_v = self(x_a, x_v)
             return x_a + dx_a, x_v + dx_v
         n, rows = self.n, x_a.shape[0] * x_a.shape[1]
         x_a, x_v = x_a.contiguous(), x_v.contiguous()

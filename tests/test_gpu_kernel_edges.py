@@ -348,3 +348,35 @@ def test_painn_update_refuses_what_does_not_fit(a, v):
         ops.painn_update_front(y, row[:33], 34, 32)
     with pytest.raises(RuntimeError):
         ops.painn_update_back(y, row, row, row, y[:, :32].contiguous(), 34, 32)
+
+
+@pytest.mark.parametrize("grad", [False, True])
+def test_hooks_of_the_update_run_inside_a_block(grad):
+    """forward and pre-forward hooks of Update and of its parts see the calls that they saw, and what they return counts"""
+    from ld_b200 import painn
+    from ld_b200.graph_layers import Graph
+    torch.manual_seed(6)
+    block = painn.Block(3.0, 32).cuda()
+    pos = torch.cumsum(torch.randn(2, 20, 3) / 3 ** 0.5, dim=1).cuda()
+    graph, bonds = Graph.radius_graph(3.0, None, pos), painn.chain_bond_graph(2, 20, "cuda")
+    flat = pos.reshape(-1, 3)
+    x = torch.randn(2, 20, 32).cuda(), torch.randn(2, 20, 32, 3).cuda()
+
+    def run():
+        with torch.set_grad_enabled(grad):
+            return [t.detach() for t in block((pos, graph, graph.rij, bonds, flat[bonds.dst] - flat[bonds.src], *x, None))[5:7]]
+
+    plain = run()
+    for name in ("", "lin_l", "lin_r", "lin_v", "mlp", "gn"):
+        part = block.update.get_submodule(name)
+        calls = []
+        handles = [part.register_forward_pre_hook(lambda m, a: calls.append(a[0].shape)),
+                   part.register_forward_hook(lambda m, a, out: calls.append(type(out)))]
+        # the fused and the separate form differ by roundings
+        assert all(float((a - b).norm()) <= 1e-5 * float(b.norm()) for a, b in zip(run(), plain)) and len(calls) == 2, name
+        assert calls[0] == (x[1] if name.startswith("lin") else torch.empty(2, 20, 64) if name == "mlp" else x[0]).shape, name
+        handles.append(part.register_forward_hook(lambda m, a, out: tuple(2 * t for t in out) if isinstance(out, tuple) else 2 * out))
+        assert not all(float((a - b).norm()) <= 1e-2 * float(b.norm()) for a, b in zip(run(), plain)), name
+        for h in handles:
+            h.remove()
+        assert all(torch.equal(a, b) for a, b in zip(run(), plain)), name
