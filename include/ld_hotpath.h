@@ -129,7 +129,7 @@ int ld_cow_o1_bw(int left, const float* o0, const float* o1, const float* g011, 
 /* ---- dense layers and the fused PaiNN message ----------------------------------------------------
  * ld_mlp3_rows: the three-layer MLPs applied per node (archs/meanflow_painn8.py:38-51;
  * archs/diffuser_atoms15.py:98-110 with the direct term Wdt). Weights are "packed":
- * Wkt = nn.Linear.weight.t().contiguous(), [in][out].
+ * Wkt = nn.Linear.weight.t().contiguous(), [in][out], 16-byte aligned (Wdt: any alignment).
  * ld_painn_message_f32: Message.forward (archs/meanflow_painn8.py:77-100) fused with the edge
  * gather and edges_reduce_src; FP32 arithmetic throughout. */
 int ld_mlp3_rows(const float* x, long long rows, int k0, const float* W1t, const float* b1, int n1, const float* W2t,

@@ -19,12 +19,13 @@ struct MlpRows {
 // threads, so that a narrow layer still has 512 loads in flight), and the groups' sums are added up in shared memory.
 // Bound by the loads of the weights at few rows (64 -> 256 -> 256 -> 256 on 512 rows: 11.7 us; a tile of 32 rows per block, 16
 // blocks, took 68) and by the FMA pipe at many (2048 rows, 128 -> 512 -> 512 -> 512: 83 us against 206).
-template <int R>
+template <int R, bool ALIGNED = true>
 __device__ __forceinline__ void mr_accumulate(const float* __restrict__ in, int K, const float* __restrict__ W, int N, int g, int KG, int c4,
                                               float (&acc)[4][R]) {
 #pragma unroll 4
   for (int k = g; k < K; k += KG) {
-    const float4 w = __ldg(reinterpret_cast<const float4*>(W + (size_t)k * N + c4));
+    const float* wp = W + (size_t)k * N + c4;
+    const float4 w = ALIGNED ? __ldg(reinterpret_cast<const float4*>(wp)) : make_float4(__ldg(wp), __ldg(wp + 1), __ldg(wp + 2), __ldg(wp + 3));
 #pragma unroll
     for (int r = 0; r < R; r += 4) {
       const float4 h = *reinterpret_cast<const float4*>(in + k * R + r);
@@ -66,7 +67,10 @@ mlp3_rows_kernel(const float* __restrict__ x, long long rows, MlpRows m, int act
 #pragma unroll
         for (int r = 0; r < R; r++) acc[j][r] = 0.f;
       mr_accumulate<R>(in, K, m.W[layer], N, g, KG, c4, acc);
-      if (layer == 2 && m.Wd != nullptr) mr_accumulate<R>(xs, m.k0, m.Wd, N, g, KG, c4, acc);
+      if (layer == 2 && m.Wd != nullptr) {
+        if ((reinterpret_cast<uintptr_t>(m.Wd) & 15) == 0) mr_accumulate<R>(xs, m.k0, m.Wd, N, g, KG, c4, acc);
+        else mr_accumulate<R, false>(xs, m.k0, m.Wd, N, g, KG, c4, acc);
+      }
 #pragma unroll
       for (int r = 0; r < R; r++)
         *reinterpret_cast<float4*>(part + ((size_t)g * R + r) * N + c4) = make_float4(acc[0][r], acc[1][r], acc[2][r], acc[3][r]);
@@ -93,7 +97,7 @@ int check_widths(const MlpRows& m) {
     if (dims[i] > 512) { ld_set_last_message("mlp (FP32 path): widths above 512 are not supported"); return LD_ERR_UNSUPPORTED; }
   }
   if (m.k0 <= 0 || m.k0 > 512) { ld_set_last_message("mlp (FP32 path): widths above 512 are not supported"); return LD_ERR_UNSUPPORTED; }
-  if ((((uintptr_t)m.W[0] | (uintptr_t)m.W[1] | (uintptr_t)m.W[2] | (uintptr_t)m.Wd) % 16) != 0) {
+  if ((((uintptr_t)m.W[0] | (uintptr_t)m.W[1] | (uintptr_t)m.W[2]) % 16) != 0) {
     ld_set_last_message("mlp: packed weights must be 16-byte aligned");
     return LD_ERR_SHAPE;
   }
@@ -144,7 +148,7 @@ __global__ void __launch_bounds__(256) update_back_kernel(const float* __restric
 
 // Three dense layers on `rows` rows. Weights are passed transposed ("packed"): Wkt is [in][out]
 // contiguous, i.e. nn.Linear.weight.t().contiguous(). act: 0 none, 1 SiLU, 2 LeakyReLU(0.1),
-// applied after layers 1 and 2. Wdt (optional, [k0][n3]) adds a direct linear term x*Wd.
+// applied after layers 1 and 2. Wdt (optional, [k0][n3], of any alignment) adds a direct linear term x*Wd.
 extern "C" int ld_mlp3_rows(const float* x, long long rows, int k0, const float* W1t, const float* b1, int n1,
                             const float* W2t, const float* b2, int n2, const float* W3t, const float* b3, int n3, int act,
                             const float* Wdt, float* out, void* stream) {

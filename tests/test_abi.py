@@ -49,3 +49,6 @@ def test_argument_errors_without_gpu():
     # the sums of the FP32 neighbour rows are FP32: a buffer sized for BF16 is refused, not overrun
     rc = L.ld_bee_messages_vd_f32(None, None, None, 4, 64, C.c_float(5.0), None, None, None, None, None, None, C.c_float(0.1), None, None, 3, 1, None)
     assert rc == _lib.LD_ERR_UNSUPPORTED
+    # the direct weight of ld_mlp3_rows need not be aligned, the three layers' have to be
+    mlp = lambda w, wd: L.ld_mlp3_rows(None, 0, 8, w, None, 16, w, None, 16, w, None, 16, 1, wd, None, None)  # noqa: E731
+    assert mlp(16, 20) == 0 and mlp(20, 16) == _lib.LD_ERR_SHAPE

@@ -380,3 +380,16 @@ def test_hooks_of_the_update_run_inside_a_block(grad):
         for h in handles:
             h.remove()
         assert all(torch.equal(a, b) for a, b in zip(run(), plain)), name
+
+
+@pytest.mark.parametrize("rows", [3, 700, 1300])
+def test_mlp_rows_takes_a_direct_weight_of_any_alignment(rows):
+    from ld_b200 import ops
+    torch.manual_seed(rows)
+    mlp = ops.PackedMLP([torch.nn.Linear(a, 40).cuda() for a in (12, 40, 40)], torch.nn.Linear(12, 40, bias=False).cuda())
+    x = torch.randn(rows, 12).cuda()
+    want = ops.mlp3_rows(x, mlp)
+    shifted = torch.empty(12 * 40 + 1, device="cuda")[1:].reshape(12, 40)
+    mlp.Wdt = shifted.copy_(mlp.Wdt)
+    assert shifted.data_ptr() % 16 == 4
+    assert torch.equal(ops.mlp3_rows(x, mlp), want)
