@@ -149,7 +149,8 @@ int ld_painn_message_f32(const int* row_ptr, const int* dst, const float* rij, i
                          const float* res_v, float* out_a, float* out_v, long long* edge_counter, void* stream);
 /* ld_painn_message_f32_split: the same at the same accuracy for n = 32, 64, 128 and n_rbf <= 4n, with the distance MLP on
  * the FP16 tensor cores, every operand the sum of two FP16 values. ld_painn_split_elems: FP16 values that
- * ld_painn_split_pack writes (0: no such form for these widths); scales: nine floats, written by it as well. */
+ * ld_painn_split_pack writes, the channels' scales behind the weights (0: no such form for these widths); `scales` is not used
+ * (may be null). */
 int ld_painn_split_elems(int n, int n_rbf, long long* elems);
 int ld_painn_split_pack(const float* W1t, const float* b1, const float* W2t, const float* b2, const float* W3t, int n, int n_rbf,
                         void* packed_f16, float* scales, void* stream);

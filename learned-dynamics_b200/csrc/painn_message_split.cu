@@ -18,6 +18,7 @@
 // together.
 #include "common.cuh"
 #include "split_f16.cuh"
+#include "split_pack.cuh"
 #include "tp_math.h"
 
 namespace {
@@ -42,7 +43,7 @@ struct Shape {
   static constexpr int G = WORK_THREADS / n;          // threads per channel in the message phase
   static_assert(N * (NE + 1) * 4 <= ACT, "the products reuse the activation planes");
   static_assert(G * EPT == NE, "the message phase covers the tile");
-  static constexpr size_t SMEM = (size_t)ACT + STAGES * sf::SLAB_BYTES + 3 * N * 4;
+  static constexpr size_t SMEM = (size_t)ACT + STAGES * sf::SLAB_BYTES + 8 * N * 4;
 };
 
 struct SplitParams {
@@ -51,7 +52,7 @@ struct SplitParams {
   float rmax, pi_over_rmax, eps;
   const __half* w[3];      // packed slabs per layer
   const float* b[3];
-  const float* scales;     // [3] input scales, [3] weight scales, [3] their inverse products
+  const float* scales;     // [3][N] what takes an accumulator back, [2][N] scales of the hidden channels
   const float* actv; const float* x_v; const float* res_a; const float* res_v;
   float* out_a; float* out_v;
   long long* edge_counter;
@@ -88,8 +89,11 @@ painn_message_split_kernel(const __grid_constant__ SplitParams P) {
   float* prod = reinterpret_cast<float*>(smem);                           // [N][NE + 1], after the last layer
   unsigned char* ring = smem + S::ACT;
   float* s_bias = reinterpret_cast<float*>(ring + STAGES * sf::SLAB_BYTES);   // [3][N]
+  float* s_inv = s_bias + 3 * N;                                          // [3][N]
+  float* s_scale = s_inv + 3 * N;                                         // [2][N]
 
   for (int i = tid; i < 3 * N; i += THREADS) s_bias[i] = P.b[i / N][i % N];
+  for (int i = tid; i < 5 * N; i += THREADS) s_inv[i] = P.scales[i];
   if (tid == 0) {
     for (int s = 0; s < STAGES; s++) { tc::mbar_init(&bar_full[s], 1); tc::mbar_init(&bar_empty[s], 1); }
     for (int s = 0; s < SLOTS; s++) tc::mbar_init(&bar_done[s], 1);      // MMAs of slab q: slot q % SLOTS
@@ -179,8 +183,6 @@ painn_message_split_kernel(const __grid_constant__ SplitParams P) {
     const int mblk = (warp >> 2) % MB, half = (warp >> 2) / MB, quarter = warp & 3;
     const int o = mblk * 128 + quarter * 32 + lane;   // this thread's channel, and edges [64 half, 64 half + 64)
     const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + half * 64;
-    const float sx1 = P.scales[1], sx2 = P.scales[2];
-    const float inv0 = P.scales[6], inv1 = P.scales[7], inv2 = P.scales[8];
     uint32_t chunks = 0;                              // partial sums taken so far by this thread's channel block
     const int mc = tid % n, mg = tid / n;             // message phase: channel, group of EPT edges
     long long edges_done = 0;
@@ -279,9 +281,9 @@ painn_message_split_kernel(const __grid_constant__ SplitParams P) {
           }
           fail = __any_sync(0xffffffffu, fail);
           if (sync_or(fail)) { fail = 1; break; }                                            // [A] the planes may be overwritten
-          const float bias = s_bias[layer * N + o], inv = layer == 0 ? inv0 : (layer == 1 ? inv1 : inv2);
+          const float bias = s_bias[layer * N + o], inv = s_inv[layer * N + o];
           if (layer < 2) {
-            const float sx = layer == 0 ? sx1 : sx2;
+            const float sx = s_scale[layer * N + o];
             unsigned char* a1 = act + (o >> 3) * S::PANEL + (half * 64) * 16 + (o & 7) * 2;
 #pragma unroll
             for (int i = 0; i < 64; i++) {
@@ -372,48 +374,6 @@ painn_message_split_kernel(const __grid_constant__ SplitParams P) {
   if (warp == 0) tc::tmem_dealloc(tmem_base, 512);
 }
 
-// scales of the three layers of an MLP (k0 -> N -> N -> N) whose inputs are at most 1 in size and whose activation does
-// not enlarge them: |input of layer l + 1| <= max over outputs of sum |W_l| * bound_l + |b_l|. Wt: [in][out].
-__global__ void __launch_bounds__(512) split_scales_kernel(const float* W1t, const float* b1, const float* W2t, const float* b2,
-                                                           const float* W3t, int k0, int N, float* __restrict__ scales) {
-  __shared__ float s_b[512], s_m[512];
-  float bound = 1.0f;
-  for (int layer = 0; layer < 3; layer++) {
-    const float* W = layer == 0 ? W1t : (layer == 1 ? W2t : W3t);
-    const float* b = layer == 0 ? b1 : b2;
-    const int K = layer == 0 ? k0 : N, o = threadIdx.x;
-    float sum = 0.f, mx = 0.f;
-    if (o < N)
-      for (int k = 0; k < K; k++) { const float a = fabsf(W[(size_t)k * N + o]); sum += a; mx = fmaxf(mx, a); }
-    s_b[o] = o < N ? fmaf(sum, bound, layer < 2 ? fabsf(b[o]) : 0.f) * 1.001f : 0.f;   // (rounding of the sum)
-    s_m[o] = mx;
-    __syncthreads();
-    for (int d = 256; d > 0; d >>= 1) {
-      if (o < d) { s_b[o] = fmaxf(s_b[o], s_b[o + d]); s_m[o] = fmaxf(s_m[o], s_m[o + d]); }
-      __syncthreads();
-    }
-    if (o == 0) {
-      const float sx = layer == 0 ? 16384.f : sf::scale_for(bound), sw = sf::scale_for(s_m[0]);
-      scales[layer] = sx; scales[3 + layer] = sw; scales[6 + layer] = 1.0f / (sx * sw);
-    }
-    bound = s_b[0];
-    __syncthreads();
-  }
-}
-
-// Wt [in][out] -> slabs [K chunk of 32][block of 128 outputs][plane][K/8][128][8], K padded with zeros to a multiple of 16
-__global__ void split_pack_kernel(const float* __restrict__ Wt, int K, int N, const float* __restrict__ scale, __half* __restrict__ out) {
-  const int kp = (K + 15) / 16 * 16;
-  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= kp * N) return;
-  const int o = idx % N, k = idx / N;
-  const float v = k < K ? Wt[(size_t)k * N + o] * scale[0] : 0.f;
-  const int ch = k / sf::SLAB_K, kw = min(sf::SLAB_K, kp - ch * sf::SLAB_K), kl = k - ch * sf::SLAB_K;
-  __half* slab = out + (size_t)ch * sf::SLAB_K * N * 2 + (size_t)(o / 128) * kw * 128 * 2;
-  __half* at = slab + (size_t)(kl / 8) * 128 * 8 + (o % 128) * 8 + kl % 8;
-  sf::split(v, at, at + (size_t)kw * 128);
-}
-
 template <int MB>
 int launch(const SplitParams& P, cudaStream_t st) {
   LD_CUDA_TRY(cudaFuncSetAttribute(painn_message_split_kernel<MB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Shape<MB>::SMEM));
@@ -428,40 +388,44 @@ int launch(const SplitParams& P, cudaStream_t st) {
 
 static bool split_form(int n, int n_rbf) { return (n == 32 || n == 64 || n == 128) && n_rbf > 0 && n_rbf <= 4 * n; }
 
-// FP16 elements of the three packed layers of a distance MLP n_rbf -> 4n -> 4n -> 4n (0: these widths have no split form)
+// The packed layers are followed by floats, N = 4n of each: inverse scales of three layers, scales of two hidden ones, their bounds
+static long long packed_slabs(int n, int n_rbf) { return 2LL * 4 * n * ((n_rbf + 15) / 16 * 16 + 8 * n); }
+
+// FP16 elements of a packed distance MLP n_rbf -> 4n -> 4n -> 4n (0: these widths have no split form)
 extern "C" int ld_painn_split_elems(int n, int n_rbf, long long* elems) {
   if (n <= 0 || n_rbf <= 0) return LD_ERR_SHAPE;
-  *elems = split_form(n, n_rbf) ? 2LL * 4 * n * ((n_rbf + 15) / 16 * 16 + 8 * n) : 0;
+  *elems = split_form(n, n_rbf) ? packed_slabs(n, n_rbf) + 2LL * 7 * 4 * n : 0;
   return LD_OK;
 }
 
-// packed: as many FP16 values as ld_painn_split_elems says, 16-byte aligned; scales: nine floats. Weights [in][out], FP32.
+// packed: as many FP16 values as ld_painn_split_elems says, 16-byte aligned. Weights [in][out], FP32. scales: not used.
 extern "C" int ld_painn_split_pack(const float* W1t, const float* b1, const float* W2t, const float* b2, const float* W3t, int n,
                                    int n_rbf, void* packed, float* scales, void* stream) {
+  (void)scales;
   if (!split_form(n, n_rbf)) { ld_set_last_message("painn split pack: n must be 32, 64 or 128, n_rbf at most 4n"); return LD_ERR_UNSUPPORTED; }
-  if (b1 == nullptr || b2 == nullptr) return LD_ERR_SHAPE;
+  if (b1 == nullptr || b2 == nullptr || ((uintptr_t)packed % 16) != 0) return LD_ERR_SHAPE;
   const int N = 4 * n, k0p = (n_rbf + 15) / 16 * 16;
   cudaStream_t st = (cudaStream_t)stream;
-  split_scales_kernel<<<1, 512, 0, st>>>(W1t, b1, W2t, b2, W3t, n_rbf, N, scales);
-  LD_LAUNCH_CHECK();
-  __half* out = (__half*)packed;
-  const float* W[3] = {W1t, W2t, W3t};
-  for (int l = 0; l < 3; l++) {
-    const int K = l == 0 ? n_rbf : N, kp = l == 0 ? k0p : N;
-    split_pack_kernel<<<ld_cdiv((long long)kp * N, 256), 256, 0, st>>>(W[l], K, N, scales + 3 + l, out);
-    LD_LAUNCH_CHECK();
-    out += (size_t)2 * N * kp;
-  }
-  return LD_OK;
+  __half* w = (__half*)packed;
+  float* f = (float*)(w + packed_slabs(n, n_rbf));
+  float* inv = f; float* scale = f + 3 * N; float* bound = f + 5 * N;
+  int rc = split_layer<SPLIT_SILU>(SplitLayer{W1t, n_rbf, N, nullptr, nullptr, nullptr, b1, w, inv, scale, bound, nullptr, nullptr}, st);
+  if (rc != LD_OK) return rc;
+  w += (size_t)2 * N * k0p;
+  rc = split_layer<SPLIT_SILU>(SplitLayer{W2t, N, N, bound, nullptr, scale, b2, w, inv + N, scale + N, bound + N, nullptr, nullptr}, st);
+  if (rc != LD_OK) return rc;
+  w += (size_t)2 * N * N;
+  return split_layer<SPLIT_LAST>(SplitLayer{W3t, N, N, bound + N, nullptr, scale + N, nullptr, w, inv + 2 * N, nullptr, nullptr, nullptr, nullptr}, st);
 }
 
 // ld_painn_message_f32 with the distance MLP as packed by ld_painn_split_pack (n = 32, 64 or 128). status_dev receives
-// LD_FLAG_TIMEOUT if a bounded wait ran out.
+// LD_FLAG_TIMEOUT if a bounded wait ran out. scales: not used.
 extern "C" int ld_painn_message_f32_split(const int* row_ptr, const int* dst, const float* rij, int Nt, int n, int n_rbf,
                                           int radial_kind, float rmax, float eps, const void* packed, const float* scales,
                                           const float* b1, const float* b2, const float* b3, const float* actv, const float* x_v,
                                           const float* res_a, const float* res_v, float* out_a, float* out_v,
                                           long long* edge_counter, int* status_dev, void* stream) {
+  (void)scales;
   if (Nt < 0 || n <= 0 || n_rbf <= 0) return LD_ERR_SHAPE;
   if (!split_form(n, n_rbf)) { ld_set_last_message("painn message (split path): n must be 32, 64 or 128, n_rbf at most 4n"); return LD_ERR_UNSUPPORTED; }
   if (b1 == nullptr || b2 == nullptr || b3 == nullptr) { ld_set_last_message("painn message: biases are required"); return LD_ERR_SHAPE; }
@@ -474,7 +438,8 @@ extern "C" int ld_painn_message_f32_split(const int* row_ptr, const int* dst, co
   P.seg_nodes = ld_even_segments(Nt, (40LL << 20) / (28LL * n));
   P.rmax = rmax; P.pi_over_rmax = (float)(3.14159265358979323846 / (double)rmax); P.eps = eps;
   P.w[0] = (const __half*)packed; P.w[1] = P.w[0] + (size_t)2 * N * k0p; P.w[2] = P.w[1] + (size_t)2 * N * N;
-  P.b[0] = b1; P.b[1] = b2; P.b[2] = b3; P.scales = scales; P.actv = actv; P.x_v = x_v; P.res_a = res_a; P.res_v = res_v;
+  P.b[0] = b1; P.b[1] = b2; P.b[2] = b3; P.actv = actv; P.x_v = x_v; P.res_a = res_a; P.res_v = res_v;
+  P.scales = (const float*)(P.w[0] + packed_slabs(n, n_rbf));
   P.out_a = out_a; P.out_v = out_v; P.edge_counter = edge_counter; P.status = status_dev;
   if (n == 128) return launch<4>(P, (cudaStream_t)stream);
   if (n == 64) return launch<2>(P, (cudaStream_t)stream);

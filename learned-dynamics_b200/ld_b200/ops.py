@@ -263,8 +263,8 @@ def _packed_bf16(mlp):
 
 
 def _packed_split(mlp, n):
-    """(FP16 planes, scales) of a distance MLP n_rbf -> 4n -> 4n -> 4n for the split-precision message kernel, built on first
-    use; None for widths without that form."""
+    """A distance MLP n_rbf -> 4n -> 4n -> 4n as FP16 planes with their scales, for the split-precision message kernel, built on
+    first use; None for widths without that form."""
     if mlp._split is None:
         elems = ctypes.c_longlong(0)
         check(lib().ld_painn_split_elems(n, mlp.dims[0], ctypes.byref(elems)))
@@ -273,11 +273,10 @@ def _packed_split(mlp, n):
         else:
             dev = mlp.Wt[0].device
             packed = torch.empty(elems.value, dtype=torch.float16, device=dev)
-            scales = torch.empty(9, dtype=torch.float32, device=dev)
             check(lib().ld_painn_split_pack(ptr(mlp.Wt[0]), ptr(mlp.b[0]), ptr(mlp.Wt[1]), ptr(mlp.b[1]), ptr(mlp.Wt[2]), n, mlp.dims[0],
-                                            ptr(packed), ptr(scales), stream_ptr(dev)))
-            mlp._split = (packed, scales)
-    return mlp._split or None
+                                            ptr(packed), None, stream_ptr(dev)))
+            mlp._split = (packed,)
+    return mlp._split[0] if mlp._split else None
 
 
 def _packed_slabs(mlp):
@@ -369,7 +368,7 @@ def painn_message_f32(row_ptr, dst, rij, mlp_dist, actv, x_v, rmax, eps=0.1, rad
     if split is not None:   # n = 32, 64, 128: the distance MLP on the tensor cores, operands as sums of two FP16 values
         with KERNEL_TIMER.region("painn_message"):
             check(lib().ld_painn_message_f32_split(ptr(row_ptr), ptr(dst), ptr(rij), Nt, n, n_rbf, radial_kind, float(rmax), float(eps),
-                                                   ptr(split[0]), ptr(split[1]), ptr(mlp_dist.b[0]), ptr(mlp_dist.b[1]),
+                                                   ptr(split), None, ptr(mlp_dist.b[0]), ptr(mlp_dist.b[1]),
                                                    ptr(mlp_dist.b[2]), ptr(actv), ptr(x_v), ptr(res_a), ptr(res_v), ptr(out_a),
                                                    ptr(out_v), ptr(edge_counter), ptr(tc_status(x_v.device)), stream_ptr(x_v.device)))
         return out_a, out_v

@@ -393,3 +393,55 @@ def test_mlp_rows_takes_a_direct_weight_of_any_alignment(rows):
     mlp.Wdt = shifted.copy_(mlp.Wdt)
     assert shifted.data_ptr() % 16 == 4
     assert torch.equal(ops.mlp3_rows(x, mlp), want)
+
+
+def _uneven(lin, kind):
+    """hidden channels of layers lin[0] and lin[1] far larger or smaller than their neighbours, the same function of the inputs up
+    to the activation"""
+    g = torch.Generator().manual_seed(11)
+    with torch.no_grad():
+        for a, b in zip(lin, lin[1:]):
+            if kind == "spread":      # over six orders of magnitude
+                s = 10.0 ** (6 * torch.rand(a.weight.shape[0], generator=g) - 3)
+            elif kind == "unit":      # one channel 1e5 in, 1e-5 out
+                s = torch.ones(a.weight.shape[0])
+                s[3] = 1e5
+            elif kind == "off":       # one channel that its bias keeps off
+                a.bias[5] = -1e6
+                continue
+            else:
+                continue
+            a.weight *= s[:, None]
+            a.bias *= s
+            b.weight /= s
+
+
+@pytest.mark.parametrize("n,n_rbf", [(32, 9), (64, 64), (128, 8)])
+@pytest.mark.parametrize("kind", ["even", "spread", "unit", "off"])
+def test_split_message_with_uneven_channels(n, n_rbf, kind):
+    """every channel has scales of its own: no further from 64 bits than the FP32 FMA kernel, whatever its neighbours' sizes"""
+    import ctypes
+    from ld_b200 import ops
+    from ld_b200._lib import lib, check, ptr, stream_ptr
+    g = torch.Generator().manual_seed(n)
+    Nt, deg = 23, 17
+    E = Nt * deg
+    row_ptr = torch.arange(0, E + 1, deg).int()
+    dst, rij = torch.randint(0, Nt, (E,), generator=g).int(), torch.randn(E, 3, generator=g) * 1.3
+    torch.manual_seed(n)
+    lin = [torch.nn.Linear(k, 4 * n) for k in (n_rbf, 4 * n, 4 * n)]
+    _uneven(lin, kind)
+    actv, x_v = torch.randn(Nt, 4 * n, generator=g), torch.randn(Nt, n, 3, generator=g)
+    want = _message64(row_ptr, dst, rij, [(l.weight.detach(), l.bias.detach()) for l in lin], actv, x_v, 1, n_rbf, 4.0)
+    mlp = ops.PackedMLP([l.cuda() for l in lin])
+    args = [t.cuda() for t in (row_ptr, dst, rij)]
+    actv, x_v = actv.cuda(), x_v.cuda()
+    split = ops.painn_message_f32(*args, mlp, actv, x_v, 4.0, radial_kind=1)
+    assert mlp._split and int(ops.tc_status(actv.device)) == 0
+    fma = torch.empty(Nt, n, device="cuda"), torch.empty(Nt, n, 3, device="cuda")
+    check(lib().ld_painn_message_f32(*[ptr(a) for a in args], Nt, n, n_rbf, 1, ctypes.c_float(4.0), ctypes.c_float(0.1), ptr(mlp.Wt[0]),
+                                     ptr(mlp.b[0]), ptr(mlp.Wt[1]), ptr(mlp.b[1]), ptr(mlp.Wt[2]), ptr(mlp.b[2]), ptr(actv), ptr(x_v), None,
+                                     None, ptr(fma[0]), ptr(fma[1]), None, stream_ptr()))
+    for w, a, b in zip(want, split, fma):
+        off = lambda t: float((t.cpu().double() - w).norm())  # noqa: E731
+        assert off(a) <= 1.2 * off(b) + U * float(w.norm()), (off(a) / float(w.norm()), off(b) / float(w.norm()))
