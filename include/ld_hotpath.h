@@ -270,9 +270,9 @@ int ld_bee_messages_scalar_f32(const int* row_ptr, const int* dst, const float* 
                                const float* b2, const float* W3t, const float* b3, const float* Wdt, float scale,
                                float* out_a, void* stream);
 /* The same at the same accuracy for chan and dim_a 64 or 128, with the per-edge linear maps on the FP16 tensor cores, every
- * operand the sum of two FP16 values. ld_bee_split_elems: FP16 values that ld_bee_split_pack writes (0: no such form);
- * scales: ten floats, written by it as well. ld_bee_rows13_f32: the neighbour rows [rows][13][chan] that it reads
- * (ld_bee_messages_vd_f32 takes them with feat_bf16 = 3). */
+ * operand the sum of two FP16 values. ld_bee_split_elems: FP16 values that ld_bee_split_pack writes, the
+ * channels' scales behind the weights (0: no such form); `scales` is not used (may be null). ld_bee_rows13_f32: the
+ * neighbour rows [rows][13][chan] that ld_bee_messages_scalar_f32_split reads (ld_bee_messages_vd_f32 takes them with feat_bf16 = 3). */
 int ld_bee_split_elems(int chan, int dim_a, long long* elems);
 int ld_bee_split_pack(const float* Yt, const float* W1t, const float* b1, const float* W2t, const float* b2, const float* W3t,
                       const float* Wdt, int chan, int dim_a, void* packed_f16, float* scales, void* stream);

@@ -13,17 +13,37 @@
 // A block owns a node-aligned slice of the CSR and walks it 64 edges at a time; roles as in painn_message_split.cu. The
 // neighbours' rows are read component-major, [node][13][C], so that a warp's loads are 128 consecutive bytes. The sizes of
 // the products are not bounded beforehand: the scale of an edge's operands comes from its largest product, those of the
-// later layers from that and from row sums of the weights. Every step of the pipeline is two weight slabs: the two blocks
+// later layers from that and from each channel's row sum of the weights (split_pack.cuh). Every step of the pipeline is two weight slabs: the two blocks
 // of 128 channels of a hidden layer, or two chunks of K of a layer with one block.
 #include "common.cuh"
 #include "split_f16.cuh"
+#include "split_pack.cuh"
 #include "bee_edge.cuh"
 
 namespace {
 using namespace sf;
 
 constexpr int NE = 64, PANEL = NE * 16 + 16, EPT = 16;
-// scales[10] = swY, sw1, sw2, sw3, swd, max row sums of |Y|, |W1|, max |b1|, max row sum of |W2|, max |b2|
+// weight slabs in the ring. A warp that waits for a slab has to know that the one before it in the same stage has landed, or
+// the parity it waits for means nothing: five stages back is the other warp's slab, of two or three steps before, and this warp
+// has waited for the accumulators of the step two before to be taken.
+constexpr int STAGES = 5;
+
+// floats behind the packed weights: per channel what takes an accumulator back (inv_*), the scale of its stored value
+// (sc_*), its bound (p_*, q_*); the extremes of q / p of the hidden layers
+template <typename T>
+struct BeeScales {
+  T *inv_y, *inv_3, *inv_d, *sc_psi, *inv_1, *sc_1, *inv_2, *sc_2;   // [A] x 4, [2 A] x 4: read by the edge kernel
+  T *ratio_1, *ratio_2;                                              // [2], [2]
+  T *p_psi, *p_1, *q_1, *p_2, *q_2;
+  __host__ __device__ BeeScales(T* f, int A) {
+    inv_y = f; inv_3 = f + A; inv_d = f + 2 * A; sc_psi = f + 3 * A;
+    inv_1 = f + 4 * A; sc_1 = f + 6 * A; inv_2 = f + 8 * A; sc_2 = f + 10 * A;
+    ratio_1 = f + 12 * A; ratio_2 = ratio_1 + 2;
+    p_psi = ratio_1 + 4; p_1 = p_psi + A; q_1 = p_1 + 2 * A; p_2 = q_1 + 2 * A; q_2 = p_2 + 2 * A;
+  }
+};
+constexpr int READ_PER_A = 12, FLOATS_PER_A = 21, FLOATS_EXTRA = 4;
 
 // C product channels, A scalar channels
 template <int C, int A>
@@ -31,7 +51,7 @@ struct BeeShape {
   static constexpr int HB = 2 * A / 128;                 // blocks of 128 channels of a hidden layer
   static constexpr int YPLANE = (3 * C / 8) * PANEL, HPLANE = (2 * A / 8) * PANEL, PPLANE = (A / 8) * PANEL;
   static constexpr int FRONT = YPLANE > HPLANE ? 2 * YPLANE : 2 * HPLANE;   // products, then hidden layers
-  static constexpr size_t SMEM = (size_t)FRONT + 2 * PPLANE + STAGES * SLAB_BYTES;
+  static constexpr size_t SMEM = (size_t)FRONT + 2 * PPLANE + STAGES * SLAB_BYTES + READ_PER_A * A * 4;
   // slabs (K = 32 each) of the four matrix products, in the order they are streamed
   static constexpr int SY = 3 * C / 32, S1 = A / 32 * HB, S2 = 2 * A / 32 * HB, S3 = 2 * A / 32, SD = A / 32;
   static constexpr int SLABS = SY + S1 + S2 + S3 + SD;
@@ -46,7 +66,7 @@ struct BeeSplitParams {
   const float* rows;                       // [Nt][13][C]
   const float* enc_w; const float* enc_b; const float* jacobi;
   const __half* w;                         // packed slabs of Y, W1, W2, W3, Wd
-  const float* scales;                     // [10]
+  const float* scales;                     // BeeScales
   const float* b1; const float* b2; const float* b3;
   float* out_a;
   int* status;
@@ -54,8 +74,15 @@ struct BeeSplitParams {
 
 __device__ __forceinline__ float leaky(float v) { return v > 0.f ? v : 0.1f * v; }
 
-// scales of one edge: operand scales and the inverse products that take an accumulator back
-struct EdgeScales { float y, inv_y, psi, inv_1, inv_d, h1, inv_2, h2, inv_3; };
+// of one edge: scale of its products, and the powers of two above the sizes of the products and the hidden layers (and one
+// over them); a channel's scale stands beside them
+struct EdgeScales { float y, up_y, down_y, up_1, down_1, up_2, down_2; };
+
+// above (by p + q) / (p + q) for every q / p in [lo, hi]: falls with q / p when by >= 1, else rises
+__device__ __forceinline__ float edge_size(float by, float lo, float hi) {
+  const float r = by >= 1.f ? lo : hi;
+  return isinf(r) ? 1.f : (by + r) / (1.f + r) * 1.001f;
+}
 
 template <int C, int A>
 __global__ void __launch_bounds__(THREADS, 1)
@@ -76,8 +103,11 @@ bee_scalar_split_kernel(const __grid_constant__ BeeSplitParams P) {
   float* vals = reinterpret_cast<float*>(smem);      // [A][NE + 1], after the last layer
   unsigned char* psi_pl = smem + S::FRONT;           // planes of psi
   unsigned char* ring = psi_pl + 2 * S::PPLANE;
+  float* s_scales = reinterpret_cast<float*>(ring + STAGES * SLAB_BYTES);
+  const BeeScales<const float> chan(s_scales, A);
 
   if (tid < 8) ld_poly8_to_chebyshev(P.jacobi + tid * 9, s_jac + tid * 9);   // Chebyshev form of the radial polynomials
+  for (int i = tid; i < READ_PER_A * A; i += THREADS) s_scales[i] = P.scales[i];
   if (tid == 0) {
     for (int s = 0; s < STAGES; s++) { tc::mbar_init(&bar_full[s], 1); tc::mbar_init(&bar_empty[s], 1); }
     for (int s = 0; s < 4; s++) tc::mbar_init(&bar_done[s], 1);            // MMAs of slab q: accumulator q % 4
@@ -286,13 +316,13 @@ bee_scalar_split_kernel(const __grid_constant__ BeeSplitParams P) {
         }
         sync_workers();
         if (tid < NE) {
-          const float by = __uint_as_float(s_max[tid]), bp = P.scales[5] * by, bh1 = fmaf(P.scales[6], bp, P.scales[7]) * 1.001f,
-                      bh2 = fmaf(P.scales[8], bh1, P.scales[9]) * 1.001f;   // (row sums already carry their rounding)
+          const float by = __uint_as_float(s_max[tid]);
+          const BeeScales<const float> all(P.scales, A);
           EdgeScales c;
-          c.y = scale_for(by); c.psi = scale_for(bp); c.h1 = scale_for(bh1); c.h2 = scale_for(bh2);
-          c.inv_y = 1.0f / (c.y * P.scales[0]);
-          c.inv_1 = 1.0f / (c.psi * P.scales[1]); c.inv_d = 1.0f / (c.psi * P.scales[4]);
-          c.inv_2 = 1.0f / (c.h1 * P.scales[2]); c.inv_3 = 1.0f / (c.h2 * P.scales[3]);
+          c.y = scale_for(by);
+          c.down_y = c.y * (1.f / 16384.f); c.up_y = 1.0f / c.down_y;
+          c.down_1 = scale_for(edge_size(by, all.ratio_1[0], all.ratio_1[1])) * (1.f / 16384.f); c.up_1 = 1.0f / c.down_1;
+          c.down_2 = scale_for(edge_size(by, all.ratio_2[0], all.ratio_2[1])) * (1.f / 16384.f); c.up_2 = 1.0f / c.down_2;
           s_sc[tid] = c;
         }
         sync_workers();
@@ -311,10 +341,12 @@ bee_scalar_split_kernel(const __grid_constant__ BeeSplitParams P) {
         take1(S::SY, psi);
         fail = __any_sync(0xffffffffu, fail);
         if (sync_or(fail)) { fail = 1; break; }                                              // [A0]
+        const float inv_y = live ? chan.inv_y[o1] : 0.f, sc_psi = live ? chan.sc_psi[o1] : 0.f;
 #pragma unroll
         for (int i = 0; i < EPT; i++) {
-          psi[i] *= s_sc[e1 + i].inv_y;
-          if (live) put(psi_pl, S::PPLANE, o1, e1 + i, psi[i] * s_sc[e1 + i].psi);
+          psi[i] *= inv_y;
+          if (live) put(psi_pl, S::PPLANE, o1, e1 + i, psi[i] * sc_psi);
+          psi[i] *= s_sc[e1 + i].up_y;
         }
         tc::fence_async_smem();
         if (sync_or(fail)) { fail = 1; break; }                                              // [X1]
@@ -327,10 +359,11 @@ bee_scalar_split_kernel(const __grid_constant__ BeeSplitParams P) {
           take_hidden(layer == 1 ? S::S1 : S::S2, acc);
           fail = __any_sync(0xffffffffu, fail);
           if (sync_or(fail)) { fail = 1; break; }                                            // [A1], [A2]
+          const float inv = layer == 1 ? chan.inv_1[oh] : chan.inv_2[oh], sc = layer == 1 ? chan.sc_1[oh] : chan.sc_2[oh];
 #pragma unroll
           for (int i = 0; i < EH; i++) {
             const EdgeScales& c = s_sc[eh + i];
-            const float h = layer == 1 ? leaky(fmaf(acc[i], c.inv_1, b1)) * c.h1 : leaky(fmaf(acc[i], c.inv_2, b2)) * c.h2;
+            const float h = layer == 1 ? leaky(fmaf(acc[i], c.up_y * inv, b1)) * (c.down_1 * sc) : leaky(fmaf(acc[i], c.up_1 * inv, b2)) * (c.down_2 * sc);
             put(front, S::HPLANE, oh, eh + i, h);
           }
           tc::fence_async_smem();
@@ -349,9 +382,10 @@ bee_scalar_split_kernel(const __grid_constant__ BeeSplitParams P) {
         // edges fall in a tile or a block -----------------------------------------------------------------------------
         node_lo = s_src[cnt - 1];
         if (live) {
+          const float inv_3 = chan.inv_3[o1], inv_d = chan.inv_d[o1];
 #pragma unroll
           for (int i = 0; i < EPT; i++)
-            vals[o1 * (NE + 1) + e1 + i] = psi[i] + (fmaf(o3[i], s_sc[e1 + i].inv_3, b3) + od[i] * s_sc[e1 + i].inv_d);
+            vals[o1 * (NE + 1) + e1 + i] = psi[i] + (fmaf(o3[i], s_sc[e1 + i].up_2 * inv_3, b3) + od[i] * (s_sc[e1 + i].up_y * inv_d));
         }
         for (int i = tid; i <= NE; i += WORK_THREADS) s_rowwin[i] = P.row_ptr[min(node_lo + i, n_end)];   // for the next tile
         sync_workers();
@@ -388,44 +422,6 @@ bee_scalar_split_kernel(const __grid_constant__ BeeSplitParams P) {
   if (warp == 0) tc::tmem_dealloc(tmem_base, 256);
 }
 
-// Wt: [in][out]. One block per matrix (Y, W1, W2, W3, Wd): its scale, and for the first three the largest row sum (over the
-// inputs) and the largest bias.
-__global__ void __launch_bounds__(256) bee_split_scales_kernel(const float* Yt, const float* W1t, const float* b1, const float* W2t,
-                                                               const float* b2, const float* W3t, const float* Wdt, int C, int A, float* scales) {
-  __shared__ float s_sum[256], s_max[256], s_b[256];
-  const int which = blockIdx.x, o = threadIdx.x;
-  const float* W = which == 0 ? Yt : which == 1 ? W1t : which == 2 ? W2t : which == 3 ? W3t : Wdt;
-  const int K = which == 0 ? 3 * C : (which == 1 || which == 4) ? A : 2 * A, N = (which == 1 || which == 2) ? 2 * A : A;
-  const float* b = which == 1 ? b1 : which == 2 ? b2 : nullptr;
-  float sum = 0.f, mx = 0.f;
-  if (o < N)
-    for (int k = 0; k < K; k++) { const float a = fabsf(W[(size_t)k * N + o]); sum += a; mx = fmaxf(mx, a); }
-  s_sum[o] = sum * 1.001f; s_max[o] = mx; s_b[o] = o < N && b != nullptr ? fabsf(b[o]) : 0.f;
-  __syncthreads();
-  for (int d = 128; d > 0; d >>= 1) {
-    if (o < d) { s_sum[o] = fmaxf(s_sum[o], s_sum[o + d]); s_max[o] = fmaxf(s_max[o], s_max[o + d]); s_b[o] = fmaxf(s_b[o], s_b[o + d]); }
-    __syncthreads();
-  }
-  if (o == 0) {
-    scales[which] = scale_for(s_max[0]);
-    if (which == 0) scales[5] = s_sum[0];
-    if (which == 1) { scales[6] = s_sum[0]; scales[7] = s_b[0]; }
-    if (which == 2) { scales[8] = s_sum[0]; scales[9] = s_b[0]; }
-  }
-}
-
-// Wt [K][N] -> slabs [K chunk of 32][block of 128 outputs][plane][4][128][8]; outputs from N on are zeros
-__global__ void bee_split_pack_kernel(const float* __restrict__ Wt, int K, int N, const float* __restrict__ scale, __half* __restrict__ out) {
-  const int Np = (N + 127) / 128 * 128;
-  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= K * Np) return;
-  const int o = idx % Np, k = idx / Np;
-  const float v = o < N ? Wt[(size_t)k * N + o] * scale[0] : 0.f;
-  __half* slab = out + ((size_t)(k / SLAB_K) * (Np / 128) + o / 128) * (SLAB_BYTES / 2);
-  __half* at = slab + (size_t)((k % SLAB_K) / 8) * 128 * 8 + (o % 128) * 8 + k % 8;
-  split(v, at, at + SLAB_K * 128);
-}
-
 // l0 [rows][C], l1 [rows][C][3], l2 [rows][C][9] -> [rows][13][C]
 __global__ void __launch_bounds__(256) bee_rows13_kernel(const float* __restrict__ l0, const float* __restrict__ l1, const float* __restrict__ l2,
                                                          long long n, int C, float* __restrict__ out) {
@@ -454,31 +450,38 @@ bool split_form(int C, int A) { return (C == 64 || C == 128) && (A == 64 || A ==
 
 }  // namespace
 
+static long long packed_slabs(int chan, int dim_a) {
+  const long long hb = 2 * dim_a / 128;
+  return (3 * chan / 32 + (dim_a / 32 + 2 * dim_a / 32) * hb + 3 * dim_a / 32) * (long long)(SLAB_BYTES / 2);
+}
+
 // FP16 elements of the packed weights of a layer with `chan` product and dim_a scalar channels (0: no split form)
 extern "C" int ld_bee_split_elems(int chan, int dim_a, long long* elems) {
   if (chan <= 0 || dim_a <= 0) return LD_ERR_SHAPE;
-  const long long hb = 2 * dim_a / 128;
-  *elems = split_form(chan, dim_a) ? (3 * chan / 32 + (dim_a / 32 + 2 * dim_a / 32) * hb + 3 * dim_a / 32) * (long long)(SLAB_BYTES / 2) : 0;
+  *elems = split_form(chan, dim_a) ? packed_slabs(chan, dim_a) + 2LL * (FLOATS_PER_A * dim_a + FLOATS_EXTRA) : 0;
   return LD_OK;
 }
 
-// packed: as many FP16 values as ld_bee_split_elems says, 16-byte aligned; scales: ten floats. Weights [in][out], FP32.
+// packed: as many FP16 values as ld_bee_split_elems says, 16-byte aligned. Weights [in][out], FP32. scales: not used.
 extern "C" int ld_bee_split_pack(const float* Yt, const float* W1t, const float* b1, const float* W2t, const float* b2, const float* W3t,
                                  const float* Wdt, int chan, int dim_a, void* packed, float* scales, void* stream) {
+  (void)scales;
   if (!split_form(chan, dim_a)) { ld_set_last_message("bee split pack: chan and dim_a must be 64 or 128"); return LD_ERR_UNSUPPORTED; }
+  if (((uintptr_t)packed % 16) != 0) return LD_ERR_SHAPE;
   cudaStream_t st = (cudaStream_t)stream;
-  bee_split_scales_kernel<<<5, 256, 0, st>>>(Yt, W1t, b1, W2t, b2, W3t, Wdt, chan, dim_a, scales);
-  LD_LAUNCH_CHECK();
-  const float* W[5] = {Yt, W1t, W2t, W3t, Wdt};
-  const int K[5] = {3 * chan, dim_a, 2 * dim_a, 2 * dim_a, dim_a}, N[5] = {dim_a, 2 * dim_a, 2 * dim_a, dim_a, dim_a};
-  __half* out = (__half*)packed;
-  for (int l = 0; l < 5; l++) {
-    const int Np = (N[l] + 127) / 128 * 128;
-    bee_split_pack_kernel<<<ld_cdiv((long long)K[l] * Np, 256), 256, 0, st>>>(W[l], K[l], N[l], scales + l, out);
-    LD_LAUNCH_CHECK();
-    out += (size_t)K[l] / SLAB_K * (Np / 128) * (SLAB_BYTES / 2);
-  }
-  return LD_OK;
+  const int A = dim_a, hb = 2 * A / 128;
+  __half* wy = (__half*)packed;
+  const BeeScales<float> c((float*)(wy + packed_slabs(chan, A)), A);
+  __half* w1 = wy + (size_t)(3 * chan / 32) * (SLAB_BYTES / 2);
+  __half* w2 = w1 + (size_t)(A / 32 * hb) * (SLAB_BYTES / 2);
+  __half* w3 = w2 + (size_t)(2 * A / 32 * hb) * (SLAB_BYTES / 2);
+  __half* wd = w3 + (size_t)(2 * A / 32) * (SLAB_BYTES / 2);
+  int rc = split_layer<SPLIT_LINEAR>(SplitLayer{Yt, 3 * chan, A, nullptr, nullptr, nullptr, nullptr, wy, c.inv_y, c.sc_psi, c.p_psi, nullptr, nullptr}, st);
+  if (rc == LD_OK) rc = split_layer<SPLIT_LEAKY>(SplitLayer{W1t, A, 2 * A, c.p_psi, nullptr, c.sc_psi, b1, w1, c.inv_1, c.sc_1, c.p_1, c.q_1, nullptr}, st);
+  if (rc == LD_OK) rc = split_layer<SPLIT_LEAKY>(SplitLayer{W2t, 2 * A, 2 * A, c.p_1, c.q_1, c.sc_1, b2, w2, c.inv_2, c.sc_2, c.p_2, c.q_2, c.ratio_1}, st);
+  if (rc == LD_OK) rc = split_layer<SPLIT_LAST>(SplitLayer{W3t, 2 * A, A, c.p_2, c.q_2, c.sc_2, nullptr, w3, c.inv_3, nullptr, nullptr, nullptr, c.ratio_2}, st);
+  if (rc == LD_OK) rc = split_layer<SPLIT_LAST>(SplitLayer{Wdt, A, A, c.p_psi, nullptr, c.sc_psi, nullptr, wd, c.inv_d, nullptr, nullptr, nullptr, nullptr}, st);
+  return rc;
 }
 
 // rows13 [rows][13][chan] = (l0 | l1 | l2 component-major): the neighbour rows of the two FP32 edge kernels
@@ -492,11 +495,12 @@ extern "C" int ld_bee_rows13_f32(const float* l0, const float* l1, const float* 
 }
 
 // ld_bee_messages_scalar_f32 on neighbour rows from ld_bee_rows13_f32 and weights from ld_bee_split_pack. status_dev
-// receives LD_FLAG_TIMEOUT if a bounded wait ran out.
+// receives LD_FLAG_TIMEOUT if a bounded wait ran out. scales: not used.
 extern "C" int ld_bee_messages_scalar_f32_split(const int* row_ptr, const int* dst, const float* rij, int Nt, int chan, int dim_a, float r0,
                                                 const float* rows13, const float* enc_w, const float* enc_b, const float* jacobi,
                                                 const void* packed, const float* scales, const float* b1, const float* b2,
                                                 const float* b3, float scale, float* out_a, int* status_dev, void* stream) {
+  (void)scales;
   if (Nt < 0 || chan <= 0 || dim_a <= 0 || !(r0 > 0.f)) return LD_ERR_SHAPE;
   if (!split_form(chan, dim_a)) { ld_set_last_message("bee messages (split path): chan and dim_a must be 64 or 128"); return LD_ERR_UNSUPPORTED; }
   if (b1 == nullptr || b2 == nullptr || b3 == nullptr || ((uintptr_t)packed % 16) != 0) return LD_ERR_SHAPE;
@@ -505,7 +509,7 @@ extern "C" int ld_bee_messages_scalar_f32_split(const int* row_ptr, const int* d
   P.row_ptr = row_ptr; P.dst = dst; P.rij = rij; P.Nt = Nt;
   P.seg_nodes = ld_even_segments(Nt, (40LL << 20) / (52LL * chan));   // the gathered rows of a segment stay in L2
   P.r0 = r0; P.scale = scale; P.rows = rows13; P.enc_w = enc_w; P.enc_b = enc_b; P.jacobi = jacobi;
-  P.w = (const __half*)packed; P.scales = scales; P.b1 = b1; P.b2 = b2; P.b3 = b3; P.out_a = out_a; P.status = status_dev;
+  P.w = (const __half*)packed; P.scales = (const float*)(P.w + packed_slabs(chan, dim_a)); P.b1 = b1; P.b2 = b2; P.b3 = b3; P.out_a = out_a; P.status = status_dev;
   cudaStream_t st = (cudaStream_t)stream;
   if (chan == 128) return dim_a == 128 ? launch<128, 128>(P, st) : launch<128, 64>(P, st);
   return dim_a == 128 ? launch<64, 128>(P, st) : launch<64, 64>(P, st);

@@ -2,7 +2,8 @@
 //   v * s = v1 + v2,   v1 = fp16(v * s),  v2 = fp16(v * s - v1)      (s a power of two)
 // which carries 22 significant bits and more, and a product of two operands is three MMAs (v1 w1, v1 w2, v2 w1; the
 // dropped v2 w2 is below 2^-24 of v1 w1). The scale s keeps v * s below 2^14: nothing overflows, and since the absolute
-// error of the pair never exceeds 2^-39 of that bound, a bound that is loose by a factor of 2^15 costs no accuracy.
+// error of the pair never exceeds 2^-39 of that bound, a bound that is loose by a factor of 2^15 costs no accuracy. Bounds and
+// scales are a channel's own (split_pack.cuh).
 //
 // The tensor cores truncate as they accumulate, which over a long K would cost more than FP32 FMAs do. So a partial sum
 // covers K = 32 only, its two small products first, and is then added to an FP32 register (round to nearest).
@@ -24,7 +25,6 @@ constexpr int WORK_WARPS = 16, WORK_THREADS = WORK_WARPS * 32;
 constexpr int MMA_WARPS = 2, MMA_WARP = WORK_WARPS, PROD_WARP = WORK_WARPS + MMA_WARPS;
 constexpr int THREADS = (WORK_WARPS + MMA_WARPS + 1) * 32;
 constexpr int SYNC_THREADS = (WORK_WARPS + MMA_WARPS) * 32;   // working and MMA warps meet at barrier 1
-constexpr int STAGES = 5;                             // weight slabs in the ring
 
 // ---- operands and products -----------------------------------------------------------------------------------
 constexpr int SLAB_K = 32;                                    // K of one weight slab = one partial sum

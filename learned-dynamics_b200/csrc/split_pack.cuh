@@ -3,7 +3,8 @@
 // A hidden channel o is stored as h * 2^(14 - e_o), where 2^e_o bounds |h| over all inputs; the next layer's weights take
 // 2^e_o up for their input o and are then scaled per output by their own largest value. So a channel that is far larger or
 // smaller than the others costs these no bits (with one scale for a whole layer, a hidden unit of 10^5 beside others of 1,
-// or one that its bias keeps off, left the results 8e-5 to 2.4e-4 off, against 1e-7 to 3e-7 of FP32 FMAs), and a thread, which owns an output channel, only reads its own scales.
+// or one that its bias keeps off, left the results 8e-5 to 2.4e-4 off, against 1e-7 to 3e-7 of FP32 FMAs), and a thread, which
+// owns an output channel, only reads its own scales.
 //
 // The bounds are those of interval arithmetic: |pre-activation| <= sum |W| bound + |b|. For SiLU, whose negative side is
 // at most 0.2785 and falls off exponentially, a unit that a large negative bias keeps off is bounded by what it can reach.

@@ -132,7 +132,7 @@ class Messages(nn.Module):
                 check(lib().ld_bee_split_elems(self.chan, self.dim_a, ctypes.byref(elems)))
                 if elems.value > 0 and dev.type == "cuda":
                     p["split"] = torch.empty(elems.value, dtype=torch.float16, device=dev)
-                    p["split_scales"] = torch.empty(10, dtype=torch.float32, device=dev)
+                    p["split_scales"] = None   # (they lie behind the packed weights)
                     check(lib().ld_bee_split_pack(ptr(p["Yt"]), ptr(p["W1t"]), ptr(p["b1"]), ptr(p["W2t"]), ptr(p["b2"]), ptr(p["W3t"]),
                                                   ptr(p["Wdt"]), self.chan, self.dim_a, ptr(p["split"]), ptr(p["split_scales"]),
                                                   stream_ptr(dev)))

@@ -445,3 +445,67 @@ def test_split_message_with_uneven_channels(n, n_rbf, kind):
     for w, a, b in zip(want, split, fma):
         off = lambda t: float((t.cpu().double() - w).norm())  # noqa: E731
         assert off(a) <= 1.2 * off(b) + U * float(w.norm()), (off(a) / float(w.norm()), off(b) / float(w.norm()))
+
+
+@pytest.mark.parametrize("chan,dim_a", [(128, 128), (64, 64), (128, 64)])
+@pytest.mark.parametrize("kind", ["even", "spread", "unit", "off"])
+@pytest.mark.parametrize("size", [1e-3, 1.0, 1e3])
+def test_split_scalar_channel_with_uneven_channels(chan, dim_a, kind, size):
+    """as above, for the l<=2 layer's scalar channel; the sizes of the features move the biases against the products"""
+    from ld_b200 import bee, ops
+    from ld_b200.graph_layers import Graph
+    from ld_b200._lib import lib, check, ptr, stream_ptr
+    g = torch.Generator().manual_seed(chan + dim_a)
+    Nt, deg = 23, 13
+    src, dst = torch.arange(Nt).repeat_interleave(deg), torch.randint(0, Nt, (Nt * deg,), generator=g)
+    rij = torch.randn(Nt * deg, 3, generator=g) * 1.5
+    torch.manual_seed(3)
+    m = bee.Messages(5.0, dim_a, 32, 32, chan)
+    _uneven([m.mlp_a.layers[k] for k in (0, 2, 4)], kind)
+    if kind == "spread":   # psi as well
+        with torch.no_grad():
+            s = 10.0 ** (6 * torch.rand(dim_a, generator=g) - 3)
+            for k in ("000", "110", "220"):
+                getattr(m, f"Y_{k}").W *= s[:, None]
+            m.mlp_a.layers[0].weight /= s
+            m.mlp_a.lin_direct.weight /= s
+    if kind == "off":   # the leaky slope lets a tenth of it through: as large as the others after the next weights
+        with torch.no_grad():
+            m.mlp_a.layers[2].weight[:, 5] *= 1e-5
+            m.mlp_a.layers[4].weight[:, 5] *= 1e-5
+    m = m.cuda()
+    rows = torch.randn(Nt, 13, chan, generator=g) * size
+    graph = Graph(src.cuda(), dst.cuda(), None, 1, Nt)
+    with torch.no_grad():
+        w = m._pack()
+    r13, rc = rows.cuda(), rij.cuda()
+    l = [r13[:, 0].contiguous(), r13[:, 1:4].transpose(1, 2).contiguous(), r13[:, 4:].transpose(1, 2).contiguous()]
+    split, fma = torch.empty(Nt, dim_a, device="cuda"), torch.empty(Nt, dim_a, device="cuda")
+    geo = (ptr(graph.row_ptr), ptr(graph.dst32), ptr(rc), Nt, chan, dim_a, 5.0)
+    enc = (ptr(w["enc_w"]), ptr(w["enc_b"]), ptr(w["jac"]))
+    check(lib().ld_bee_messages_scalar_f32_split(*geo, ptr(r13), *enc, ptr(w["split"]), None, ptr(w["b1"]), ptr(w["b2"]), ptr(w["b3"]), 0.1,
+                                                 ptr(split), ptr(ops.tc_status(r13.device)), stream_ptr()))
+    check(lib().ld_bee_messages_scalar_f32(*geo, *[ptr(t) for t in l], *enc, ptr(w["Yt"]), ptr(w["W1t"]), ptr(w["b1"]), ptr(w["W2t"]),
+                                           ptr(w["b2"]), ptr(w["W3t"]), ptr(w["b3"]), ptr(w["Wdt"]), 0.1, ptr(fma), stream_ptr()))
+    assert int(ops.tc_status(r13.device)) == 0
+    p = {k: v.detach().cpu().double() for k, v in m.state_dict().items()}
+    r = rij.double()
+    phi = bee.radial_encode_8(r, 5.0) @ p["lin_enc.weight"].t() + p["lin_enc.bias"]
+    u = r * 1.4
+    u = u / torch.sqrt(1 + (u ** 2).sum(-1, keepdim=True))
+    f = rows.double()[dst]
+    y = [f[:, 0] * phi, torch.einsum("ekc,ek->ec", f[:, 1:4], u) * phi,
+         torch.einsum("exyc,ex,ey->ec", f[:, 4:].reshape(-1, 3, 3, chan), u, u) * phi]
+    psi = sum(t @ p[f"Y_{k}.W"].t() for t, k in zip(y, ("000", "110", "220")))
+    h, terms = psi, psi.abs() @ p["mlp_a.lin_direct.weight"].abs().t() + psi.abs()
+    for k in (0, 2, 4):
+        last = h.abs()
+        h = h @ p[f"mlp_a.layers.{k}.weight"].t() + p[f"mlp_a.layers.{k}.bias"]
+        h = torch.nn.functional.leaky_relu(h, 0.1) if k < 4 else h
+    terms += last @ p["mlp_a.layers.4.weight"].abs().t() + p["mlp_a.layers.4.bias"].abs()
+    add = lambda t: torch.zeros(Nt, dim_a, dtype=torch.float64).index_add(0, src, 0.1 * t)  # noqa: E731
+    want, size = add(psi + psi @ p["mlp_a.lin_direct.weight"].t() + h), add(terms)
+    # per channel (their sizes differ by orders of magnitude). Both operands of a product are held to 2^-23 of their own size or
+    # better, so that the last layer's products are off by 4 U at most where one term outweighs the others (the FMA kernel: U)
+    a, b = ((t.cpu().double() - want).norm(dim=0) for t in (split, fma))
+    assert bool((a <= 1.5 * b + 4 * U * size.norm(dim=0)).all()), float((a / (b + U * size.norm(dim=0))).max())
