@@ -206,7 +206,7 @@ bee_scalar_split_kernel(const __grid_constant__ BeeSplitParams P) {
     auto take1 = [&](int nslabs, float* acc) {
       for (int q = 0; q < nslabs && !fail; q += 2, steps++) {
         const uint32_t slot = (steps & 1) * 2, ph = (steps >> 1) & 1;
-        if (!tc::mbar_wait(&bar_done[slot], ph) || !tc::mbar_wait(&bar_done[slot + 1], ph)) { fail = 1; break; }
+        if (!warp_wait(&bar_done[slot], ph) || !warp_wait(&bar_done[slot + 1], ph)) { fail = 1; break; }
         tc::fence_after_sync();
         float v[32];
         tc::tmem_ld16x2(tlane + slot * NE + e1, tlane + (slot + 1) * NE + e1, v);
@@ -224,7 +224,7 @@ bee_scalar_split_kernel(const __grid_constant__ BeeSplitParams P) {
       } else {
       for (int q = 0; q < nslabs && !fail; q += 2, steps++) {
         const uint32_t slot = (steps & 1) * 2 + hblk;
-        if (!tc::mbar_wait(&bar_done[slot], (steps >> 1) & 1)) { fail = 1; break; }
+        if (!warp_wait(&bar_done[slot], (steps >> 1) & 1)) { fail = 1; break; }
         tc::fence_after_sync();
         float v[32];
         tc::tmem_ld32(tlane + slot * NE + eh, v);
@@ -339,7 +339,6 @@ bee_scalar_split_kernel(const __grid_constant__ BeeSplitParams P) {
 #pragma unroll
         for (int i = 0; i < EPT; i++) psi[i] = 0.f;
         take1(S::SY, psi);
-        fail = __any_sync(0xffffffffu, fail);
         if (sync_or(fail)) { fail = 1; break; }                                              // [A0]
         const float inv_y = live ? chan.inv_y[o1] : 0.f, sc_psi = live ? chan.sc_psi[o1] : 0.f;
 #pragma unroll
@@ -357,7 +356,6 @@ bee_scalar_split_kernel(const __grid_constant__ BeeSplitParams P) {
 #pragma unroll
           for (int i = 0; i < EH; i++) acc[i] = 0.f;
           take_hidden(layer == 1 ? S::S1 : S::S2, acc);
-          fail = __any_sync(0xffffffffu, fail);
           if (sync_or(fail)) { fail = 1; break; }                                            // [A1], [A2]
           const float inv = layer == 1 ? chan.inv_1[oh] : chan.inv_2[oh], sc = layer == 1 ? chan.sc_1[oh] : chan.sc_2[oh];
 #pragma unroll
@@ -376,7 +374,6 @@ bee_scalar_split_kernel(const __grid_constant__ BeeSplitParams P) {
         for (int i = 0; i < EPT; i++) o3[i] = od[i] = 0.f;
         take1(S::S3, o3);
         take1(S::SD, od);
-        fail = __any_sync(0xffffffffu, fail);
         if (sync_or(fail)) { fail = 1; break; }                                              // [A3]
         // ---- per-node sums, thread = channel: one edge after the other, so that a node's sum does not depend on where its
         // edges fall in a tile or a block -----------------------------------------------------------------------------

@@ -233,8 +233,7 @@ painn_message_bf16_kernel(const __grid_constant__ Bf16Params P) {
           tc::fence_before_sync();
           if (sync_or(fail)) { fail = 1; break; }                                            // [X]
           // this block of channels as soon as it is complete; the planes are overwritten when all are
-          if (!tc::mbar_wait(&bar_done[mblk], layers & 1)) fail = 1;
-          fail = __any_sync(0xffffffffu, fail);
+          if (!warp_wait(&bar_done[mblk], layers & 1)) fail = 1;
           tc::fence_after_sync();
           const float bias = layer == 0 ? bias1 : bias2;
           unsigned char* at = act + (o >> 3) * PANEL + (part * EW) * 16 + (o & 7) * 2;
@@ -269,9 +268,8 @@ painn_message_bf16_kernel(const __grid_constant__ Bf16Params P) {
         if (fail) break;
         tc::fence_before_sync();
         if (sync_or(fail)) { fail = 1; break; }                                              // [X]
-        if (!tc::mbar_wait(&bar_done[mblk], layers & 1)) fail = 1;
+        if (!warp_wait(&bar_done[mblk], layers & 1)) fail = 1;
         layers++;
-        fail = __any_sync(0xffffffffu, fail);
         if (sync_or(fail)) { fail = 1; break; }                                              // [A]
         tc::fence_after_sync();
         node_lo = s_src[cnt - 1];

@@ -266,7 +266,7 @@ painn_message_split_kernel(const __grid_constant__ SplitParams P) {
           for (int i = 0; i < 64; i++) acc[i] = 0.f;
           for (int ch = 0; ch < nch && !fail; ch++, chunks++) {
             const uint32_t slot = (chunks & 1) * MB + mblk;
-            if (!tc::mbar_wait(&bar_done[slot], (chunks >> 1) & 1)) { fail = 1; break; }
+            if (!warp_wait(&bar_done[slot], (chunks >> 1) & 1)) { fail = 1; break; }
             tc::fence_after_sync();
 #pragma unroll
             for (int q = 0; q < 4; q++) {
@@ -279,7 +279,6 @@ painn_message_split_kernel(const __grid_constant__ SplitParams P) {
             __syncwarp();
             if (lane == 0) tc::mbar_arrive(&bar_taken[chunks & 1]);
           }
-          fail = __any_sync(0xffffffffu, fail);
           if (sync_or(fail)) { fail = 1; break; }                                            // [A] the planes may be overwritten
           const float bias = s_bias[layer * N + o], inv = s_inv[layer * N + o];
           if (layer < 2) {

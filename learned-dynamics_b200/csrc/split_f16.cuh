@@ -119,6 +119,9 @@ __device__ __forceinline__ int sync_or(int flag) {
       : "=r"(out) : "r"(flag), "n"(SYNC_THREADS) : "memory");
   return out;
 }
+// a bounded wait of a whole warp: every lane leaves with the same answer, since the loads from tensor memory and the barriers
+// that follow need all of them (a lane that gave up alone would meet the others at different instructions)
+__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, tc::mbar_wait(bar, parity)) != 0; }
 // barrier 2: working warps only
 __device__ __forceinline__ void sync_workers() { asm volatile("barrier.cta.sync 2, %0;" ::"n"(WORK_THREADS) : "memory"); }
 
