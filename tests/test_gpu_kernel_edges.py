@@ -509,3 +509,29 @@ def test_split_scalar_channel_with_uneven_channels(chan, dim_a, kind, size):
     # better, so that the last layer's products are off by 4 U at most where one term outweighs the others (the FMA kernel: U)
     a, b = ((t.cpu().double() - want).norm(dim=0) for t in (split, fma))
     assert bool((a <= 1.5 * b + 4 * U * size.norm(dim=0)).all()), float((a / (b + U * size.norm(dim=0))).max())
+
+
+# many particles in a cell: all of them sorted by (cell, index) instead of ranked by counting, in blocks of 256 and 1024 threads
+# and at counts that are no powers of two
+@pytest.mark.parametrize("batch,nodes,box,cutoff,scale", [(2, 3001, (7.0, 7.1, 7.2), 2.3, 1.0), (1, 1500, None, 1.0, 0.02), (3, 300, None, 3.0, 0.01),
+                                                         (2, 512, None, 0.5, 0.05), (1, 129, None, 3.0, 0.0), (1, 2500, None, 2.0, 0.25)])
+def test_radius_graph_of_dense_systems(batch, nodes, box, cutoff, scale):
+    from ld_b200 import graph as G
+    from oracle import reference_math as R
+    g = torch.Generator().manual_seed(nodes)
+    pos = torch.rand(batch, nodes, 3, generator=g) * torch.tensor(box) if box else \
+        scale * torch.cumsum(torch.randn(batch, nodes, 3, generator=g) / 3 ** 0.5, dim=1)
+    b = G.RadiusGraphBuilder(batch, nodes, cutoff, box)
+    got = b.build(pos.cuda())
+    assert int(b.status) == 0
+    oracle = R.radius_graph(pos, cutoff, box)
+    key = lambda s, d: s.cpu().long() * (batch * nodes) + d.cpu().long()  # noqa: E731
+    mine, want = key(got["src"], got["dst"]), key(oracle["src"], oracle["dst"])
+    assert torch.equal(mine.sort().values, want.sort().values)
+    assert torch.equal(got["rij"].cpu()[mine.argsort()], oracle["rij"][want.argsort()])
+    # a node's neighbours come cell by cell and ascend inside a cell: at most as many descents as there are cells around it
+    s, d = got["src"].long(), got["dst"].long()
+    down = (s[1:] == s[:-1]) & (d[1:] < d[:-1])
+    assert int(torch.bincount(s[1:][down], minlength=batch * nodes).max()) <= 27
+    if scale in (0.0, 0.01):   # one cell
+        assert not bool(down.any())
