@@ -143,25 +143,67 @@ tensor_linear_kernel(const TlWeights W, const float* __restrict__ x, float* __re
     }
   }
   const int oc = o0 + ty * OU;
+  if (OU % 4 == 0 && O % 4 == 0 && (reinterpret_cast<uintptr_t>(y) & 15) == 0) {
 #pragma unroll
-  for (int n = 0; n < NR; n++) {
-    const int rl = tx + TX * n;
-    if (rl >= rcnt) continue;
-    float* yr = y + ((r0 + rl) * O + oc) * S;   // OU * S consecutive floats
-    if (OU % 4 == 0 && O % 4 == 0 && oc + OU <= O && (reinterpret_cast<uintptr_t>(y) & 15) == 0) {
+    for (int n = 0; n < NR; n++) {
+      const int rl = tx + TX * n;
+      if (rl >= rcnt || oc >= O) continue;
+      float* yr = y + ((r0 + rl) * O + oc) * S;   // OU * S consecutive floats, fewer at the end of the outputs
 #pragma unroll
       for (int q = 0; q < OU * S / 4; q++) {
         float4 v;
         v.x = acc[(4 * q) / S][n * S + (4 * q) % S];         v.y = acc[(4 * q + 1) / S][n * S + (4 * q + 1) % S];
         v.z = acc[(4 * q + 2) / S][n * S + (4 * q + 2) % S]; v.w = acc[(4 * q + 3) / S][n * S + (4 * q + 3) % S];
-        reinterpret_cast<float4*>(yr)[q] = v;
+        if (OU == 4 || oc + OU <= O || 4 * q < (O - oc) * S) reinterpret_cast<float4*>(yr)[q] = v;
       }
-    } else {
+    }
+    return;
+  }
+  if (OU % 4 != 0) {   // the small tiles
+#pragma unroll
+    for (int n = 0; n < NR; n++) {
+      const int rl = tx + TX * n;
+      if (rl >= rcnt) continue;
+      float* yr = y + ((r0 + rl) * O + oc) * S;
 #pragma unroll
       for (int u = 0; u < OU; u++)
 #pragma unroll
         for (int s = 0; s < S; s++)
           if (oc + u < O) yr[u * S + s] = acc[u][n * S + s];
+    }
+    return;
+  }
+  // rows that 16-byte words do not fit: through shared memory, some rows at a time, so that a warp stores consecutive
+  // floats (stored lane by lane, every 4-byte store of a warp went to 32 sectors; 16384 rows, S = 9, 33 -> 47: 67 -> 41 us)
+  const int live = min(TO, O - o0) * S, pitch = live | 1;       // (odd: no bank conflicts)
+  const int rp = min(rcnt, (int)(T::BYTES / 4) / pitch);        // rows per pass
+  tl_wait<0>();
+#pragma unroll 1
+  for (int p0 = 0; p0 < rcnt; p0 += rp) {
+    __syncthreads();   // the stages, or the rows of the pass before, have been read
+#pragma unroll
+    for (int n = 0; n < NR; n++) {
+      const int rl = tx + TX * n - p0;
+      if (rl < 0 || rl >= rp) continue;
+      float* at = smem + rl * pitch + ty * OU * S;
+#pragma unroll
+      for (int u = 0; u < OU; u++)
+        if (oc + u < O) {
+#pragma unroll
+          for (int s = 0; s < S; s++) at[u * S + s] = acc[u][n * S + s];
+        }
+    }
+    __syncthreads();
+    const int rows_here = min(rp, rcnt - p0);
+    float* yp = y + ((r0 + p0) * O + o0) * S;
+    if (O <= TO && live < 32) {   // short rows that follow one another
+      for (int f = tid; f < rows_here * live; f += TL_THREADS) {
+        const int rl = f / live;
+        yp[f] = smem[rl * pitch + f - rl * live];
+      }
+    } else {
+      for (int rl = tid >> 5; rl < rows_here; rl += TL_THREADS / 32)
+        for (int i = tid & 31; i < live; i += 32) yp[(long long)rl * O * S + i] = smem[rl * pitch + i];
     }
   }
 }
@@ -315,16 +357,22 @@ int tl_launch(const TlWeights& W, const float* x, float* y, long long rows, int 
 }
 
 // Which tile: 8 outputs x 6 to 9 columns per thread, as many outputs per block as there are (32, 64 or 128) and the rest of
-// the threads along the rows, so that x is read once. Where that leaves SMs without a block, tiles of 32 outputs and a
-// quarter of the columns (twice the shared loads per FMA, but up to sixteen times the blocks).
-template <int S, int NR, int NR_SMALL, int PARTS = 1>
+// the threads along the rows, so that x is read once. Where that leaves SMs without a block, tiles of 64 outputs and half the
+// accumulators per thread, and where those do as well, tiles of 32 outputs and a quarter of the columns (twice the shared loads
+// per FMA, but up to sixteen times the blocks). 128 -> 128 channels: 2048 rows, S = 9, 50 us in small tiles, 32 in the middle
+// ones; 16384 rows, S = 1, 49 and 36.
+template <int S, int NR, int NR_MID, int NR_SMALL, int PARTS = 1>
 int tl_pick(const TlWeights& W, const float* x, float* y, long long rows, int I, int O, cudaStream_t st) {
   const int tr = O <= 32 ? TlTile<S, 4, 8, NR>::TR : (O <= 64 ? TlTile<S, 8, 8, NR>::TR : TlTile<S, 16, 8, NR>::TR);
   const long long blocks = (rows + tr - 1) / tr * (O <= 128 ? 1 : ld_cdiv(O, 128));
-  if (blocks < 148) return tl_launch<S, 16, 2, NR_SMALL, PARTS>(W, x, y, rows, I, O, st);
-  if (O <= 32) return tl_launch<S, 4, 8, NR, PARTS>(W, x, y, rows, I, O, st);
-  if (O <= 64) return tl_launch<S, 8, 8, NR, PARTS>(W, x, y, rows, I, O, st);
-  return tl_launch<S, 16, 8, NR, PARTS>(W, x, y, rows, I, O, st);
+  if (blocks >= 148) {
+    if (O <= 32) return tl_launch<S, 4, 8, NR, PARTS>(W, x, y, rows, I, O, st);
+    if (O <= 64) return tl_launch<S, 8, 8, NR, PARTS>(W, x, y, rows, I, O, st);
+    return tl_launch<S, 16, 8, NR, PARTS>(W, x, y, rows, I, O, st);
+  }
+  constexpr int TR_MID = TlTile<S, 16, 4, NR_MID>::TR;
+  if (O > 32 && (rows + TR_MID - 1) / TR_MID * ld_cdiv(O, 64) >= 148) return tl_launch<S, 16, 4, NR_MID, PARTS>(W, x, y, rows, I, O, st);
+  return tl_launch<S, 16, 2, NR_SMALL, PARTS>(W, x, y, rows, I, O, st);
 }
 
 template <int S, int TO, int TI, int VEC>
@@ -368,9 +416,9 @@ extern "C" int ld_tensor_linear(int inds, const float* W, long long sw0, long lo
   if (rows == 0 || dim_out == 0) return LD_OK;
   cudaStream_t st = (cudaStream_t)stream;
   const TlWeights Ws{{W, W, W}, sw0, sw1, dim_out};
-  if (inds == 0) return tl_pick<1, 8, 2>(Ws, x, y, rows, dim_in, dim_out, st);
-  if (inds == 1) return tl_pick<3, 2, 1>(Ws, x, y, rows, dim_in, dim_out, st);
-  return tl_pick<9, 1, 1>(Ws, x, y, rows, dim_in, dim_out, st);
+  if (inds == 0) return tl_pick<1, 8, 4, 2>(Ws, x, y, rows, dim_in, dim_out, st);
+  if (inds == 1) return tl_pick<3, 2, 2, 1>(Ws, x, y, rows, dim_in, dim_out, st);
+  return tl_pick<9, 1, 1, 1>(Ws, x, y, rows, dim_in, dim_out, st);
 }
 
 // The three channel mixings of PaiNN's Update in one launch, the weights read where they lie: y [rows][3n][3] = (W_l x | W_r x |
@@ -379,7 +427,7 @@ extern "C" int ld_painn_update_mix(const float* W_l, const float* W_r, const flo
                                    void* stream) {
   if (rows < 0 || n <= 0 || n > 0x7fffffff / 3) return LD_ERR_SHAPE;
   if (rows == 0) return LD_OK;
-  return tl_pick<3, 2, 1, 3>(TlWeights{{W_l, W_r, W_v}, n, 1, n}, x_v, y, rows, n, 3 * n, (cudaStream_t)stream);
+  return tl_pick<3, 2, 2, 1, 3>(TlWeights{{W_l, W_r, W_v}, n, 1, n}, x_v, y, rows, n, 3 * n, (cudaStream_t)stream);
 }
 
 extern "C" int ld_tensor_linear_dw_workspace(int inds, long long rows, int dim_in, int dim_out, size_t* bytes) {

@@ -535,3 +535,22 @@ def test_radius_graph_of_dense_systems(batch, nodes, box, cutoff, scale):
     assert int(torch.bincount(s[1:][down], minlength=batch * nodes).max()) <= 27
     if scale in (0.0, 0.01):   # one cell
         assert not bool(down.any())
+
+
+# the tiles between the large and the small ones, rows that 16-byte stores do not fit, in every tile
+@pytest.mark.parametrize("inds,rows,dim_in,dim_out", [(0, 5000, 20, 100), (0, 4801, 9, 128), (0, 20001, 12, 127), (1, 3000, 33, 127), (1, 2999, 18, 68),
+                                                      (1, 5001, 6, 129), (2, 1500, 18, 65), (2, 2047, 10, 128), (2, 2500, 5, 126), (2, 40, 8, 7)])
+def test_tensor_linear_middle_tiles_and_ragged_rows(inds, rows, dim_in, dim_out):
+    from ld_b200 import ops
+    g = torch.Generator().manual_seed(rows)
+    W, x = torch.randn(dim_out, dim_in, generator=g), torch.randn(rows, dim_in, *[3] * inds, generator=g)
+    bound = dim_in * U * _linear64(W.abs(), x.abs(), inds)   # n products in any order, with FMAs
+    guard = torch.full((rows * dim_out * 3 ** inds + 64,), 7.0, device="cuda")
+    from ld_b200._lib import lib, check, ptr, stream_ptr
+    Wc, xc = W.cuda(), x.cuda()
+    for shift in (0, 1):   # an output that starts at no 16-byte boundary
+        out = guard[shift: rows * dim_out * 3 ** inds + shift].reshape(rows, dim_out, *[3] * inds)
+        check(lib().ld_tensor_linear(inds, ptr(Wc), dim_in, 1, ptr(xc), out.data_ptr(), rows, dim_in, dim_out, stream_ptr()))
+        assert bool(((out.cpu().double() - _linear64(W, x, inds)).abs() <= bound).all())
+        assert bool((guard[rows * dim_out * 3 ** inds + shift:] == 7.0).all())
+        guard.fill_(7.0)
