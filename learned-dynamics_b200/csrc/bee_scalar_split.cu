@@ -51,7 +51,7 @@ struct BeeShape {
   static constexpr int HB = 2 * A / 128;                 // blocks of 128 channels of a hidden layer
   static constexpr int YPLANE = (3 * C / 8) * PANEL, HPLANE = (2 * A / 8) * PANEL, PPLANE = (A / 8) * PANEL;
   static constexpr int FRONT = YPLANE > HPLANE ? 2 * YPLANE : 2 * HPLANE;   // products, then hidden layers
-  static constexpr size_t SMEM = (size_t)FRONT + 2 * PPLANE + STAGES * SLAB_BYTES + READ_PER_A * A * 4;
+  static constexpr size_t SMEM = (size_t)FRONT + 2 * PPLANE + STAGES * SLAB_BYTES + (READ_PER_A + 2) * A * 4;
   // slabs (K = 32 each) of the four matrix products, in the order they are streamed
   static constexpr int SY = 3 * C / 32, S1 = A / 32 * HB, S2 = 2 * A / 32 * HB, S3 = 2 * A / 32, SD = A / 32;
   static constexpr int SLABS = SY + S1 + S2 + S3 + SD;
@@ -96,6 +96,7 @@ bee_scalar_split_kernel(const __grid_constant__ BeeSplitParams P) {
   __shared__ EdgeScales s_sc[NE];
   __shared__ unsigned s_max[NE];
   __shared__ int s_dst[NE], s_src[NE], s_rowwin[NE + 1];
+  __shared__ uint32_t s_begin[NE / 32];
   __shared__ float s_jac[72];
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -105,6 +106,7 @@ bee_scalar_split_kernel(const __grid_constant__ BeeSplitParams P) {
   unsigned char* ring = psi_pl + 2 * S::PPLANE;
   float* s_scales = reinterpret_cast<float*>(ring + STAGES * SLAB_BYTES);
   const BeeScales<const float> chan(s_scales, A);
+  float* s_carry = s_scales + READ_PER_A * A;   // [2][A]: sum of the node that goes on, in turn
 
   if (tid < 8) ld_poly8_to_chebyshev(P.jacobi + tid * 9, s_jac + tid * 9);   // Chebyshev form of the radial polynomials
   for (int i = tid; i < READ_PER_A * A; i += THREADS) s_scales[i] = P.scales[i];
@@ -200,7 +202,11 @@ bee_scalar_split_kernel(const __grid_constant__ BeeSplitParams P) {
 #pragma unroll
     for (int m = 0; m < 8; m++) w8[m] = P.enc_w[pc * 8 + m];
     const float wb = P.enc_b[pc];
-    uint32_t steps = 0;
+    uint32_t steps = 0, tiles = 0;
+    constexpr int GROUPS = WORK_THREADS / A;          // per-node sums: threads per channel
+    const int comp = tid % A, sgrp = tid / A;
+    auto load = [](int) { return 0.f; };
+    auto store = [&](int v, float val, float) { P.out_a[(size_t)v * A + comp] = val * P.scale; };
 
     // adds the partial sums of `nslabs` slabs with one channel block to acc (16 edges)
     auto take1 = [&](int nslabs, float* acc) {
@@ -247,17 +253,12 @@ bee_scalar_split_kernel(const __grid_constant__ BeeSplitParams P) {
     for (int seg_lo = 0; seg_lo < P.Nt && !fail; seg_lo += seg_nodes) {
       const BlockRange br = block_range(P.row_ptr, seg_lo, min(seg_lo + seg_nodes, P.Nt), NE);
       const int n_begin = br.n_begin, n_end = br.n_end;
-      float carry = 0.f;          // thread tid < A: sum of channel tid of node `cur`
-      int cur = n_begin;
+      int cur = n_begin;          // node that s_carry belongs to
       int node_lo = n_begin;      // source node of the next tile's first edge (or an earlier one)
       sync_workers();             // the previous segment's last readers of s_rowwin are done
-      for (int i = tid; i <= NE; i += WORK_THREADS) s_rowwin[i] = P.row_ptr[min(node_lo + i, n_end > n_begin ? n_end : n_begin)];
+      stage_window<NE>(s_rowwin, P.row_ptr, node_lo, max(n_end, n_begin), tid);
+      if (tid < A) s_carry[(tiles & 1) * A + tid] = 0.f;
       sync_workers();
-      // output of node `from`, zeros for the nodes (from, next)
-      auto flush_until = [&](int from, int next, float val) {
-        if (tid < A)
-          for (int v = from; v < next; v++) P.out_a[(size_t)v * A + tid] = v == from ? val * P.scale : 0.f;
-      };
 
       for (long long e0 = br.e_begin; e0 < br.e_end; e0 += NE) {
         const int cnt = (int)(br.e_end - e0 < NE ? br.e_end - e0 : NE);
@@ -268,16 +269,7 @@ bee_scalar_split_kernel(const __grid_constant__ BeeSplitParams P) {
             const long long e = e0 + tid;
             edge_geometry(P.rij, e, P.r0, s_jac, &s_geom[tid]);
             j = P.dst[e];
-            int lo, hi;   // source node: largest v with row_ptr[v] <= e, in the staged window first
-            if ((long long)s_rowwin[NE] > e) {
-              lo = 0; hi = NE;
-              while (hi - lo > 1) { const int mid = (lo + hi) >> 1; if ((long long)s_rowwin[mid] > e) hi = mid; else lo = mid; }
-              s = node_lo + lo;
-            } else {
-              lo = node_lo + NE; hi = n_end;
-              while (hi - lo > 1) { const int mid = (lo + hi) >> 1; if ((long long)P.row_ptr[mid] > e) hi = mid; else lo = mid; }
-              s = lo;
-            }
+            s = source_node<NE>(s_rowwin, P.row_ptr, node_lo, n_end, e);
           }
           s_dst[tid] = j;
           s_src[tid] = s;
@@ -375,8 +367,7 @@ bee_scalar_split_kernel(const __grid_constant__ BeeSplitParams P) {
         take1(S::S3, o3);
         take1(S::SD, od);
         if (sync_or(fail)) { fail = 1; break; }                                              // [A3]
-        // ---- per-node sums, thread = channel: one edge after the other, so that a node's sum does not depend on where its
-        // edges fall in a tile or a block -----------------------------------------------------------------------------
+        // ---- per-node sums ------------------------------------------------------------------------------------------------
         node_lo = s_src[cnt - 1];
         if (live) {
           const float inv_3 = chan.inv_3[o1], inv_d = chan.inv_d[o1];
@@ -384,34 +375,19 @@ bee_scalar_split_kernel(const __grid_constant__ BeeSplitParams P) {
           for (int i = 0; i < EPT; i++)
             vals[o1 * (NE + 1) + e1 + i] = psi[i] + (fmaf(o3[i], s_sc[e1 + i].up_2 * inv_3, b3) + od[i] * (s_sc[e1 + i].up_y * inv_d));
         }
-        for (int i = tid; i <= NE; i += WORK_THREADS) s_rowwin[i] = P.row_ptr[min(node_lo + i, n_end)];   // for the next tile
+        stage_window<NE>(s_rowwin, P.row_ptr, node_lo, n_end, tid);   // for the next tile
+        mark_nodes<NE>(s_begin, s_src, cnt, cur, tid);
         sync_workers();
-        if (tid < A) {
-          const float* m = vals + tid * (NE + 1);
-          int c_node = cur;
-          for (int eb = 0; eb < cnt; eb += 8) {
-            float v[8];
-#pragma unroll
-            for (int i = 0; i < 8; i++) v[i] = m[eb + i];
-            const int last = min(eb + 8, cnt) - 1;
-            if (s_src[last] == c_node && last == eb + 7) {
-#pragma unroll
-              for (int i = 0; i < 8; i++) carry += v[i];
-            } else {
-#pragma unroll
-              for (int i = 0; i < 8; i++)
-                if (eb + i < cnt) {
-                  const int s = s_src[eb + i];
-                  if (s != c_node) { flush_until(c_node, s, carry); carry = 0.f; c_node = s; }
-                  carry += v[i];
-                }
-            }
-          }
-        }
+        node_sums<1, GROUPS, NE / GROUPS>(vals + comp * (NE + 1), s_src, s_begin, 0, cnt, sgrp, cur, s_carry + (tiles & 1) * A + comp,
+                                       s_carry + (~tiles & 1) * A + comp, load, store);
+        tiles++;
         cur = node_lo;
         sync_workers();   // geometry and planes are rewritten by the next tile
       }
-      if (!fail && n_begin < n_end) flush_until(cur, n_end, carry);
+      if (!fail && n_begin < n_end && sgrp == 0) {
+        store(cur, s_carry[(tiles & 1) * A + comp], 0.f);
+        empty_nodes<1>(cur + 1, n_end, load, store);
+      }
     }
   }
   if (fail && lane == 0 && P.status != nullptr) atomicOr(P.status, LD_FLAG_TIMEOUT);

@@ -24,6 +24,8 @@ constexpr int KSLAB = 64;                       // K of a weight slab
 // has landed, or the parity it waits for means nothing, and with two warps in turn both are then its own
 constexpr int RING = 4;
 
+constexpr int SUM_BATCH = 4;                          // nodes whose residuals are in flight together in the per-node sums
+
 template <int MB>
 struct Shape {
   static constexpr int N = 128 * MB, n = 32 * MB;
@@ -31,7 +33,8 @@ struct Shape {
   static constexpr int EP = MB == 4 ? 64 : NE;             // edges per pass of the message phase
   static constexpr int G = WORK_THREADS / n, EPT = EP / G; // threads per channel and edges per thread there
   static constexpr int FRONT = (N / 8) * PANEL > N * (EP + 1) * 4 ? (N / 8) * PANEL : N * (EP + 1) * 4;
-  static constexpr size_t SMEM = (size_t)FRONT + RING * SLAB_BYTES;
+  static constexpr int GROUPS = WORK_THREADS / N;          // threads per component in the per-node sums
+  static constexpr size_t SMEM = (size_t)FRONT + RING * SLAB_BYTES + 2 * N * 4;
 };
 
 struct Bf16Params {
@@ -57,11 +60,13 @@ painn_message_bf16_kernel(const __grid_constant__ Bf16Params P) {
   __shared__ float s_dir[NE][3];
   __shared__ float s_dist[NE], s_env[NE];
   __shared__ int s_dst[NE], s_src[NE], s_rowwin[NE + 1];
+  __shared__ uint32_t s_begin[NE / 32];
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   unsigned char* act = smem;                           // activations [N/8 panels][NE][8] BF16
   float* prod = reinterpret_cast<float*>(smem);        // [N][EP + 1], after the last layer
   unsigned char* ring = smem + S::FRONT;
+  float* s_carry = reinterpret_cast<float*>(ring + RING * SLAB_BYTES);   // [2][N]: sum of the node that goes on, in turn
 
   if (tid == 0) {
     for (int s = 0; s < RING; s++) { tc::mbar_init(&bar_full[s], 1); tc::mbar_init(&bar_empty[s], 1); }
@@ -151,31 +156,32 @@ painn_message_bf16_kernel(const __grid_constant__ Bf16Params P) {
     const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + mblk * NE + part * EW;
     const float bias1 = P.b[0][o], bias2 = P.b[1][o], bias3 = P.b[2][o];
     const int mc = tid % n, mg = tid / n;             // message phase: channel, group of EPT edges
+    // per-node sums: row of the products (component sc of channel mc), group
+    const int grp = S::GROUPS == 1 ? 0 : tid / N, comp = S::GROUPS == 1 ? tid : tid % N, sc = S::GROUPS == 1 ? mg : comp / n;
+    float sum = 0.f;                                  // one group: of node `cur` (more: in s_carry)
     uint32_t layers = 0;                              // layers completed: phase of bar_done
+    uint32_t passes = 0;
     long long edges_done = 0;
+    // residual of this thread's component, and its result
+    auto load = [&](int v) {
+      if (sc < 3) return P.res_v != nullptr ? __ldg(P.res_v + ((size_t)v * n + mc) * 3 + sc) : 0.f;
+      return P.res_a != nullptr ? __ldg(P.res_a + (size_t)v * n + mc) : 0.f;
+    };
+    auto store = [&](int v, float val, float r) {
+      if (sc < 3) P.out_v[((size_t)v * n + mc) * 3 + sc] = P.res_v != nullptr ? val + r : val;
+      else P.out_a[(size_t)v * n + mc] = P.res_a != nullptr ? val + r : val;
+    };
 
     for (int seg_lo = 0; seg_lo < P.Nt && !fail; seg_lo += seg_nodes) {
       const BlockRange br = block_range(P.row_ptr, seg_lo, min(seg_lo + seg_nodes, P.Nt), NE);
       const int n_begin = br.n_begin, n_end = br.n_end;
-      float carry = 0.f;          // thread tid < N: sum of output (component mg, channel mc) of node `cur`
-      int cur = n_begin;
+      int cur = n_begin;          // node that s_carry belongs to
       int node_lo = n_begin;      // source node of the next tile's first edge (or an earlier one)
       sync_workers();             // the previous segment's last readers of s_rowwin are done
-      for (int i = tid; i <= NE; i += WORK_THREADS) s_rowwin[i] = P.row_ptr[min(node_lo + i, n_end > n_begin ? n_end : n_begin)];
+      stage_window<NE>(s_rowwin, P.row_ptr, node_lo, max(n_end, n_begin), tid);
+      sum = 0.f;
+      if (S::GROUPS > 1 && tid < N) s_carry[(passes & 1) * N + tid] = 0.f;
       sync_workers();
-      // output of node `from`, zeros for the nodes (from, next)
-      auto flush_until = [&](int from, int next, float val) {
-        if (tid >= N) return;
-        for (int v = from; v < next; v++, val = 0.f) {
-          if (mg < 3) {
-            const size_t off = ((size_t)v * n + mc) * 3 + mg;
-            P.out_v[off] = P.res_v != nullptr ? val + P.res_v[off] : val;
-          } else {
-            const size_t off = (size_t)v * n + mc;
-            P.out_a[off] = P.res_a != nullptr ? val + P.res_a[off] : val;
-          }
-        }
-      };
 
       for (long long e0 = br.e_begin; e0 < br.e_end; e0 += NE) {
         const int cnt = (int)(br.e_end - e0 < NE ? br.e_end - e0 : NE);
@@ -187,16 +193,7 @@ painn_message_bf16_kernel(const __grid_constant__ Bf16Params P) {
             const long long e = e0 + tid;
             dx = P.rij[e * 3]; dy = P.rij[e * 3 + 1]; dz = P.rij[e * 3 + 2];
             j = P.dst[e];
-            int lo, hi;   // source node: largest v with row_ptr[v] <= e, in the staged window first
-            if ((long long)s_rowwin[NE] > e) {
-              lo = 0; hi = NE;
-              while (hi - lo > 1) { const int mid = (lo + hi) >> 1; if ((long long)s_rowwin[mid] > e) hi = mid; else lo = mid; }
-              s = node_lo + lo;
-            } else {
-              lo = node_lo + NE; hi = n_end;   // row_ptr[lo] <= e < row_ptr[hi]
-              while (hi - lo > 1) { const int mid = (lo + hi) >> 1; if ((long long)P.row_ptr[mid] > e) hi = mid; else lo = mid; }
-              s = lo;
-            }
+            s = source_node<NE>(s_rowwin, P.row_ptr, node_lo, n_end, e);
           }
           const float r2 = dx * dx + dy * dy + dz * dz, inv = rsqrtf(P.eps + r2), d = sqrtf(r2);
           s_dir[tid][0] = dx * inv; s_dir[tid][1] = dy * inv; s_dir[tid][2] = dz * inv;
@@ -273,7 +270,8 @@ painn_message_bf16_kernel(const __grid_constant__ Bf16Params P) {
         if (sync_or(fail)) { fail = 1; break; }                                              // [A]
         tc::fence_after_sync();
         node_lo = s_src[cnt - 1];
-        for (int i = tid; i <= NE; i += WORK_THREADS) s_rowwin[i] = P.row_ptr[min(node_lo + i, n_end)];   // for the next tile
+        stage_window<NE>(s_rowwin, P.row_ptr, node_lo, n_end, tid);   // for the next tile
+        if (S::GROUPS > 1) mark_nodes<NE>(s_begin, s_src, cnt, cur, tid);
         // ---- EP edges at a time: last layer to shared memory in FP32, messages, per-node sums -----------------------------
         for (int p0 = 0; p0 < cnt; p0 += EP) {
           // columns of the pass that this thread holds (MB = 4: the pass' half of its edges, else all of them)
@@ -316,36 +314,23 @@ painn_message_bf16_kernel(const __grid_constant__ Bf16Params P) {
             }
           }
           sync_workers();
-          // thread = (component, channel): one edge after the other, so that a node's sum does not depend on where its
-          // edges fall in a tile or a block
-          if (tid < N) {
-            const float* m = prod + tid * (EP + 1);
-            const int live = min(EP, cnt - p0);
-            for (int eb = 0; eb < live; eb += 8) {
-              float v[8];
-#pragma unroll
-              for (int i = 0; i < 8; i++) v[i] = m[eb + i];
-              const int last = min(eb + 8, live) - 1;
-              if (s_src[p0 + last] == cur && last == eb + 7) {
-#pragma unroll
-                for (int i = 0; i < 8; i++) carry += v[i];
-              } else {
-#pragma unroll
-                for (int i = 0; i < 8; i++)
-                  if (eb + i < live) {
-                    const int s = s_src[p0 + eb + i];
-                    if (s != cur) { flush_until(cur, s, carry); carry = 0.f; cur = s; }
-                    carry += v[i];
-                  }
-              }
-            }
+          const int live = min(EP, cnt - p0);
+          if constexpr (S::GROUPS == 1) {
+            node_walk<false>(prod + comp * (EP + 1), s_src, p0, live, sum, cur, load, store);
+          } else {
+            node_sums<SUM_BATCH, S::GROUPS, EP / S::GROUPS>(prod + comp * (EP + 1), s_src, s_begin, p0, live, grp, cur,
+                                                            s_carry + (passes & 1) * N + comp, s_carry + (~passes & 1) * N + comp, load, store);
+            cur = s_src[p0 + live - 1];
           }
+          passes++;
           sync_workers();   // the products (and geometry and planes) are rewritten
         }
-        cur = node_lo;
       }
       if (!fail && n_begin < n_end) {
-        flush_until(cur, n_end, carry);
+        if (grp == 0) {
+          store(cur, S::GROUPS == 1 ? sum : s_carry[(passes & 1) * N + comp], load(cur));
+          empty_nodes<SUM_BATCH>(cur + 1, n_end, load, store);
+        }
         edges_done += br.e_end - br.e_begin;
       }
     }

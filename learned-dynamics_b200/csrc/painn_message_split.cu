@@ -25,6 +25,7 @@ namespace {
 
 using namespace sf;
 
+constexpr int SUM_BATCH = 4;                          // nodes whose residuals are in flight together in the per-node sums
 constexpr int EPT = 16;                               // edges per thread in the message phase
 
 // MB: blocks of 128 channels; n = 32 MB
@@ -43,7 +44,8 @@ struct Shape {
   static constexpr int G = WORK_THREADS / n;          // threads per channel in the message phase
   static_assert(N * (NE + 1) * 4 <= ACT, "the products reuse the activation planes");
   static_assert(G * EPT == NE, "the message phase covers the tile");
-  static constexpr size_t SMEM = (size_t)ACT + STAGES * sf::SLAB_BYTES + 8 * N * 4;
+  static constexpr int GROUPS = WORK_THREADS / N;     // threads per component in the per-node sums
+  static constexpr size_t SMEM = (size_t)ACT + STAGES * sf::SLAB_BYTES + 10 * N * 4;
 };
 
 struct SplitParams {
@@ -68,6 +70,7 @@ __device__ __forceinline__ float radial_gaussian(int m, int n, float d, float rm
   const float u = (d - (float)m * width) / width;
   return expf(-0.5f * u * u);
 }
+
 // SiLU with the quotient from the reciprocal instruction (2 ulp)
 __device__ __forceinline__ float silu_fdiv(float x) { return __fdividef(x, 1.0f + expf(-x)); }
 
@@ -83,6 +86,7 @@ painn_message_split_kernel(const __grid_constant__ SplitParams P) {
   __shared__ float s_dist[NE], s_env[NE];
   __shared__ int s_dst[NE], s_src[NE];
   __shared__ int s_rowwin[NE + 1];   // row_ptr[node_lo .. node_lo + NE] of the coming tile
+  __shared__ uint32_t s_begin[NE / 32];
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   unsigned char* act = smem;                                              // two activation planes
@@ -91,6 +95,7 @@ painn_message_split_kernel(const __grid_constant__ SplitParams P) {
   float* s_bias = reinterpret_cast<float*>(ring + STAGES * sf::SLAB_BYTES);   // [3][N]
   float* s_inv = s_bias + 3 * N;                                          // [3][N]
   float* s_scale = s_inv + 3 * N;                                         // [2][N]
+  float* s_carry = s_scale + 2 * N;                                       // [2][N]: sum of the node that goes on, in turn
 
   for (int i = tid; i < 3 * N; i += THREADS) s_bias[i] = P.b[i / N][i % N];
   for (int i = tid; i < 5 * N; i += THREADS) s_inv[i] = P.scales[i];
@@ -185,31 +190,31 @@ painn_message_split_kernel(const __grid_constant__ SplitParams P) {
     const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + half * 64;
     uint32_t chunks = 0;                              // partial sums taken so far by this thread's channel block
     const int mc = tid % n, mg = tid / n;             // message phase: channel, group of EPT edges
+    // per-node sums: row of the products (component sc of channel mc), group
+    const int grp = S::GROUPS == 1 ? 0 : tid / N, comp = S::GROUPS == 1 ? tid : tid % N, sc = S::GROUPS == 1 ? mg : comp / n;
+    float sum = 0.f;                                  // one group: of node `cur` (more: in s_carry)
+    uint32_t tiles = 0;
     long long edges_done = 0;
+    // residual of this thread's component, and its result
+    auto load = [&](int v) {
+      if (sc < 3) return P.res_v != nullptr ? __ldg(P.res_v + ((size_t)v * n + mc) * 3 + sc) : 0.f;
+      return P.res_a != nullptr ? __ldg(P.res_a + (size_t)v * n + mc) : 0.f;
+    };
+    auto store = [&](int v, float val, float r) {
+      if (sc < 3) P.out_v[((size_t)v * n + mc) * 3 + sc] = P.res_v != nullptr ? val + r : val;
+      else P.out_a[(size_t)v * n + mc] = P.res_a != nullptr ? val + r : val;
+    };
 
     for (int seg_lo = 0; seg_lo < P.Nt && !fail; seg_lo += seg_nodes) {
       const BlockRange br = block_range(P.row_ptr, seg_lo, min(seg_lo + seg_nodes, P.Nt), NE);
       const int n_begin = br.n_begin, n_end = br.n_end;
-      float carry = 0.f;          // thread tid < N: sum of output (component tid / n, channel tid % n) of node `cur`
-      int cur = n_begin;
+      int cur = n_begin;          // node that s_carry belongs to
       int node_lo = n_begin;      // source node of the next tile's first edge (or an earlier one)
       sync_workers();             // the previous segment's last readers of s_rowwin are done
-      for (int i = tid; i <= NE; i += WORK_THREADS) s_rowwin[i] = P.row_ptr[min(node_lo + i, n_end > n_begin ? n_end : n_begin)];
+      stage_window<NE>(s_rowwin, P.row_ptr, node_lo, max(n_end, n_begin), tid);
+      sum = 0.f;
+      if (S::GROUPS > 1 && tid < N) s_carry[(tiles & 1) * N + tid] = 0.f;
       sync_workers();
-
-      // output of node `from`, zeros for the nodes (from, next)
-      auto flush_until = [&](int from, int next, float val) {
-        if (tid >= N) return;
-        for (int v = from; v < next; v++, val = 0.f) {
-          if (mg < 3) {
-            const size_t off = ((size_t)v * n + mc) * 3 + mg;
-            P.out_v[off] = P.res_v != nullptr ? val + P.res_v[off] : val;
-          } else {
-            const size_t off = (size_t)v * n + mc;
-            P.out_a[off] = P.res_a != nullptr ? val + P.res_a[off] : val;
-          }
-        }
-      };
 
       for (long long e0 = br.e_begin; e0 < br.e_end; e0 += NE) {
         const int cnt = (int)(br.e_end - e0 < NE ? br.e_end - e0 : NE);
@@ -221,17 +226,7 @@ painn_message_split_kernel(const __grid_constant__ SplitParams P) {
             const long long e = e0 + tid;
             dx = P.rij[e * 3]; dy = P.rij[e * 3 + 1]; dz = P.rij[e * 3 + 2];
             j = P.dst[e];
-            // source node: largest v with row_ptr[v] <= e, in the staged window first
-            int lo, hi;
-            if ((long long)s_rowwin[NE] > e) {
-              lo = 0; hi = NE;
-              while (hi - lo > 1) { const int mid = (lo + hi) >> 1; if ((long long)s_rowwin[mid] > e) hi = mid; else lo = mid; }
-              s = node_lo + lo;
-            } else {
-              lo = node_lo + NE; hi = n_end;   // row_ptr[lo] <= e < row_ptr[hi]
-              while (hi - lo > 1) { const int mid = (lo + hi) >> 1; if ((long long)P.row_ptr[mid] > e) hi = mid; else lo = mid; }
-              s = lo;
-            }
+            s = source_node<NE>(s_rowwin, P.row_ptr, node_lo, n_end, e);
           }
           const float r2 = dx * dx + dy * dy + dz * dz;
           const float inv = 1.0f / sqrtf(P.eps + r2);
@@ -301,7 +296,8 @@ painn_message_split_kernel(const __grid_constant__ SplitParams P) {
         }
         if (fail) break;
         node_lo = s_src[cnt - 1];
-        for (int i = tid; i <= NE; i += WORK_THREADS) s_rowwin[i] = P.row_ptr[min(node_lo + i, n_end)];   // for the next tile
+        stage_window<NE>(s_rowwin, P.row_ptr, node_lo, n_end, tid);   // for the next tile
+        if (S::GROUPS > 1) mark_nodes<NE>(s_begin, s_src, cnt, cur, tid);
         sync_workers();
         // ---- messages of channel mc, edges [EPT mg, EPT mg + EPT), in the place of the products they are made of ------------
         {
@@ -333,35 +329,20 @@ painn_message_split_kernel(const __grid_constant__ SplitParams P) {
           }
         }
         sync_workers();
-        // ---- per-node sums, thread = (component, channel): one edge after the other, so that a node's sum does not depend on
-        // where its edges fall in a tile or a block ----------------------------------------------------------------------
-        if (tid < N) {
-          const float* m = prod + tid * (NE + 1);
-          int c_node = cur;
-          for (int eb = 0; eb < cnt; eb += 8) {
-            float v[8];
-#pragma unroll
-            for (int i = 0; i < 8; i++) v[i] = m[eb + i];
-            const int last = min(eb + 8, cnt) - 1;
-            if (s_src[last] == c_node && last == eb + 7) {
-#pragma unroll
-              for (int i = 0; i < 8; i++) carry += v[i];
-            } else {
-#pragma unroll
-              for (int i = 0; i < 8; i++)
-                if (eb + i < cnt) {
-                  const int s = s_src[eb + i];
-                  if (s != c_node) { flush_until(c_node, s, carry); carry = 0.f; c_node = s; }
-                  carry += v[i];
-                }
-            }
-          }
-        }
+        if constexpr (S::GROUPS == 1)
+          node_walk<true>(prod + comp * (NE + 1), s_src, 0, cnt, sum, cur, load, store);
+        else
+          node_sums<SUM_BATCH, S::GROUPS, NE / S::GROUPS>(prod + comp * (NE + 1), s_src, s_begin, 0, cnt, grp, cur, s_carry + (tiles & 1) * N + comp,
+                                                          s_carry + (~tiles & 1) * N + comp, load, store);
+        tiles++;
         cur = node_lo;
         sync_workers();   // geometry and planes are rewritten by the next tile
       }
       if (!fail && n_begin < n_end) {
-        flush_until(cur, n_end, carry);
+        if (grp == 0) {
+          store(cur, S::GROUPS == 1 ? sum : s_carry[(tiles & 1) * N + comp], load(cur));
+          empty_nodes<SUM_BATCH>(cur + 1, n_end, load, store);
+        }
         edges_done += br.e_end - br.e_begin;
       }
     }

@@ -554,3 +554,71 @@ def test_tensor_linear_middle_tiles_and_ragged_rows(inds, rows, dim_in, dim_out)
         assert bool(((out.cpu().double() - _linear64(W, x, inds)).abs() <= bound).all())
         assert bool((guard[rows * dim_out * 3 ** inds + shift:] == 7.0).all())
         guard.fill_(7.0)
+
+
+def _chunk_graph(nodes, chunk, seed):
+    """0 to 3 edges a node, whose ends lie in the same chunk of nodes; one stretch without edges, one node with many"""
+    g = torch.Generator().manual_seed(seed)
+    deg = torch.randint(0, 4, (nodes,), generator=g)
+    deg[nodes // 3: nodes // 3 + chunk // 2] = 0
+    deg[nodes // 2] = 300
+    src = torch.repeat_interleave(torch.arange(nodes), deg)
+    lo = src // chunk * chunk
+    dst = lo + (torch.rand(len(src), generator=g) * (torch.clamp(lo + chunk, max=nodes) - lo)).long()
+    return deg, src, dst, torch.randn(len(src), 3, generator=g) * 1.3
+
+
+# the blocks walk the nodes in segments of about 40 MB of gathered rows (11.7 k nodes at n = 128): rings, accumulators and sums go
+# on from one segment to the next, blocks have no edges in some of them
+@pytest.mark.parametrize("n,nodes", [(32, 100_000), (64, 52_000), (128, 26_000)])
+@pytest.mark.parametrize("precision", ["fp32", "bf16"])
+def test_messages_over_several_segments(n, nodes, precision):
+    """the whole graph against its chunks of less than one segment, computed by themselves: the same bits"""
+    from ld_b200 import ops
+    chunk = 5000
+    deg, src, dst, rij = _chunk_graph(nodes, chunk, n)
+    torch.manual_seed(n)
+    mlp = ops.PackedMLP([torch.nn.Linear(k, 4 * n).cuda() for k in (8, 4 * n, 4 * n)])
+    fused = ops.painn_message_bf16_tc if precision == "bf16" else ops.painn_message_f32
+    actv, x_v, res_a = torch.randn(nodes, 4 * n, device="cuda"), torch.randn(nodes, n, 3, device="cuda"), torch.randn(nodes, n, device="cuda")
+    row_ptr = torch.cat([torch.zeros(1, dtype=torch.long), deg.cumsum(0)])
+
+    def run(lo, hi, residual):
+        e = slice(int(row_ptr[lo]), int(row_ptr[hi]))
+        return fused((row_ptr[lo:hi + 1] - row_ptr[lo]).int().cuda(), (dst[e] - lo).int().cuda(), rij[e].cuda(), mlp, actv[lo:hi], x_v[lo:hi], 4.0,
+                     radial_kind=1, res_a=res_a[lo:hi] if residual else None, res_v=x_v[lo:hi] if residual else None)
+
+    for residual in (False, True):
+        whole = run(0, nodes, residual)
+        for lo in range(0, nodes, chunk):
+            for w, p in zip(whole, run(lo, min(lo + chunk, nodes), residual)):
+                assert torch.equal(w[lo:lo + chunk], p), lo
+    assert bool((run(0, nodes, False)[0][deg == 0] == 0).all()) and int(ops.tc_status("cuda")) == 0
+
+
+@pytest.mark.parametrize("chan,dim_a,nodes", [(128, 128, 20_000), (64, 64, 40_000), (128, 64, 20_000), (64, 128, 40_000)])
+def test_scalar_channel_over_several_segments(chan, dim_a, nodes):
+    from ld_b200 import bee, ops
+    from ld_b200._lib import lib, check, ptr, stream_ptr
+    chunk = 5000
+    deg, src, dst, rij = _chunk_graph(nodes, chunk, chan)
+    torch.manual_seed(chan)
+    m = bee.Messages(5.0, dim_a, 32, 32, chan).cuda()
+    with torch.no_grad():
+        w = m._pack()
+    rows = torch.randn(nodes, 13, chan, device="cuda")
+    row_ptr = torch.cat([torch.zeros(1, dtype=torch.long), deg.cumsum(0)])
+
+    def run(lo, hi):
+        e = slice(int(row_ptr[lo]), int(row_ptr[hi]))
+        rp, d, r, part = (row_ptr[lo:hi + 1] - row_ptr[lo]).int().cuda(), (dst[e] - lo).int().cuda(), rij[e].cuda(), rows[lo:hi]
+        out = torch.full((hi - lo, dim_a), 7.0, device="cuda")
+        check(lib().ld_bee_messages_scalar_f32_split(ptr(rp), ptr(d), ptr(r), hi - lo, chan, dim_a, 5.0, ptr(part), ptr(w["enc_w"]), ptr(w["enc_b"]),
+                                                     ptr(w["jac"]), ptr(w["split"]), None, ptr(w["b1"]), ptr(w["b2"]), ptr(w["b3"]), 0.1, ptr(out),
+                                                     ptr(ops.tc_status("cuda")), stream_ptr()))
+        return out
+
+    whole = run(0, nodes)
+    for lo in range(0, nodes, chunk):
+        assert torch.equal(whole[lo:lo + chunk], run(lo, min(lo + chunk, nodes))), lo
+    assert bool((whole[deg == 0] == 0).all()) and int(ops.tc_status("cuda")) == 0
