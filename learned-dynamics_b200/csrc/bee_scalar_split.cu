@@ -389,6 +389,7 @@ bee_scalar_split_kernel(const __grid_constant__ BeeSplitParams P) {
         empty_nodes<1>(cur + 1, n_end, load, store);
       }
     }
+    if (fail && sgrp == 0) mark_failed(P.row_ptr, P.Nt, seg_nodes, NE, store);
   }
   if (fail && lane == 0 && P.status != nullptr) atomicOr(P.status, LD_FLAG_TIMEOUT);
   __syncthreads();

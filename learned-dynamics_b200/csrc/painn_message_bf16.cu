@@ -9,8 +9,8 @@
 // n = 128, 8 radial functions, 2.25 M edges: 3.80 ms, against 4.52 ms (+ 10 us of packing).
 //
 // A block owns a node-aligned, contiguous slice of the CSR. Roles: 16 working warps, 2 MMA warps (of every pair of channel
-// blocks one each), 1 producer warp. Every wait is bounded (LD_FLAG_TIMEOUT): a failed wait is OR-ed into the next block
-// barrier so that all threads leave together.
+// blocks one each), 1 producer warp. Every wait is bounded: a failed wait is OR-ed into the next block barrier so that all
+// threads leave together, raises LD_FLAG_TIMEOUT and leaves NaN in the outputs of the block.
 #include "common.cuh"
 #include "split_f16.cuh"
 #include "tp_math.h"
@@ -334,6 +334,7 @@ painn_message_bf16_kernel(const __grid_constant__ Bf16Params P) {
         edges_done += br.e_end - br.e_begin;
       }
     }
+    if (fail && grp == 0) mark_failed(P.row_ptr, P.Nt, seg_nodes, NE, store);
     if (!fail && P.edge_counter != nullptr && tid == 0 && edges_done > 0)
       atomicAdd((unsigned long long*)P.edge_counter, (unsigned long long)edges_done);
   }

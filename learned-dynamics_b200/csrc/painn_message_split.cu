@@ -14,8 +14,8 @@
 //     thread) and summed per node in edge order (no atomics; every node written once; the same bits wherever a node's
 //     edges fall in a tile).
 //   * 2 MMA warps and 1 producer warp (lane 0 of each): six MMAs per 16 KB weight slab; slabs stream through a ring.
-// Every wait is bounded (LD_FLAG_TIMEOUT): a failed wait is OR-ed into the next block barrier so that all threads leave
-// together.
+// Every wait is bounded: a failed wait is OR-ed into the next block barrier so that all threads leave together, raises
+// LD_FLAG_TIMEOUT and leaves NaN in the outputs of the block.
 #include "common.cuh"
 #include "split_f16.cuh"
 #include "split_pack.cuh"
@@ -346,6 +346,7 @@ painn_message_split_kernel(const __grid_constant__ SplitParams P) {
         edges_done += br.e_end - br.e_begin;
       }
     }
+    if (fail && grp == 0) mark_failed(P.row_ptr, P.Nt, seg_nodes, NE, store);
     if (!fail && P.edge_counter != nullptr && tid == 0 && edges_done > 0)
       atomicAdd((unsigned long long*)P.edge_counter, (unsigned long long)edges_done);
   }

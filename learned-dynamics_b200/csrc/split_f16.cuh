@@ -292,4 +292,14 @@ __device__ __forceinline__ void node_sums(const float* m, const int* s_src, cons
   }
 }
 
+// After a wait that ran out: NaN for every node of this block, so that the outputs themselves show that they are incomplete
+// (callers that do not read the status word would take what was in the buffer for results).
+template <class Store>
+__device__ __forceinline__ void mark_failed(const int* __restrict__ row_ptr, int Nt, int seg_nodes, int tile, const Store& store) {
+  for (int seg_lo = 0; seg_lo < Nt; seg_lo += seg_nodes) {
+    const BlockRange br = block_range(row_ptr, seg_lo, min(seg_lo + seg_nodes, Nt), tile);
+    for (int v = br.n_begin; v < br.n_end; v++) store(v, __int_as_float(0x7fc00000), 0.f);
+  }
+}
+
 }  // namespace sf
