@@ -85,7 +85,8 @@ class ScalGroupNorm(nn.Module):
 
 def _as_built(m, cls):
     """m is a plain `cls`, with nothing registered or replaced that a call of it would run"""
-    return type(m) is cls and not m._forward_hooks and not m._forward_pre_hooks and "forward" not in vars(m)
+    d = m.__dict__
+    return type(m) is cls and not d["_forward_hooks"] and not d["_forward_pre_hooks"] and "forward" not in d
 
 
 class Update(nn.Module):
@@ -99,23 +100,31 @@ class Update(nn.Module):
         assert n % 4 == 0
         self.gn = ScalGroupNorm(n, 4, epsilon=1.)
 
-    def _fusable(self):
-        return (_as_built(self, Update) and all(_as_built(l, TensLinear) and l.inds == 1 for l in (self.lin_l, self.lin_r, self.lin_v))
-                and _as_built(self.mlp, MLP) and _as_built(self.gn, ScalGroupNorm)
-                and not nn_module._global_forward_hooks and not nn_module._global_forward_pre_hooks)
+    def _mixing_weights(self):
+        """the weights of lin_l, lin_r and lin_v where the fused form may read them, else None"""
+        parts = self._modules   # (attribute access of a module looks its parts up last)
+        lins = [parts[k] for k in ("lin_l", "lin_r", "lin_v")]
+        if not (_as_built(self, Update) and all(_as_built(l, TensLinear) and l.inds == 1 and l.precision == "fp32" for l in lins)
+                and _as_built(parts["mlp"], MLP) and _as_built(parts["gn"], ScalGroupNorm)
+                and not nn_module._global_forward_hooks and not nn_module._global_forward_pre_hooks):
+            return None
+        W = [l._parameters["W"] for l in lins]
+        return W if all(w.dtype == torch.float32 and w.is_contiguous() for w in W) else None
 
     def residual(self, x_a, x_v):
         """x_a + dx_a, x_v + dx_v. Without autograd: the three channel mixings as one launch on the weights as they are, and
-        what is pointwise around the MLP and the norm as two kernels instead of some twenty; not where hooks or replaced parts want to see the separate calls."""
-        lins = (self.lin_l, self.lin_r, self.lin_v)
-        if (torch.is_grad_enabled() or not x_a.is_cuda or not self._fusable() or x_a.dim() != 3 or x_a.dtype != torch.float32 or x_v.dtype != torch.float32
-                or x_a.shape[2] != self.n or x_v.shape != (*x_a.shape, 3) or x_v.device != x_a.device   # (what does not fit is refused there)
-                or any(l.precision != "fp32" or l.W.dtype != torch.float32 or not l.W.is_contiguous() for l in lins)):
+        what is pointwise around the MLP and the norm as two kernels instead of some twenty; not where hooks or replaced parts
+        want to see the separate calls, and not for inputs that do not fit (which the separate operations refuse)."""
+        W = None
+        if (not torch.is_grad_enabled() and x_a.is_cuda and x_a.dim() == 3 and x_a.dtype == torch.float32 and x_v.dtype == torch.float32
+                and x_a.shape[2] == self.n and x_v.shape == (*x_a.shape, 3) and x_v.device == x_a.device):
+            W = self._mixing_weights()
+        if W is None:
             dx_a, dx_v = self(x_a, x_v)
             return x_a + dx_a, x_v + dx_v
         n, rows = self.n, x_a.shape[0] * x_a.shape[1]
         x_a, x_v = x_a.contiguous(), x_v.contiguous()
-        y = ops.painn_update_mix(self.lin_l.W, self.lin_r.W, self.lin_v.W, x_v, rows, n)
+        y = ops.painn_update_mix(*W, x_v, rows, n)
         inner, cat = ops.painn_update_front(y, x_a, rows, n)
         scaled, base, out_v = ops.painn_update_back(y, self.mlp(cat), inner, x_a, x_v, rows, n)
         return self.gn(scaled.reshape(x_a.shape), residual=base.reshape(x_a.shape)), out_v
