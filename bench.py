@@ -50,8 +50,10 @@ DEFAULT_WORKLOAD = "polymers_l2_1024x256"
 DRAM_BYTES_PER_EDGE = {"bee_scalar_tc_kernel": 83.0, "bee_vd_kernel": 200.4, "bee_vd_tc_kernel": 208.0, "bee_fused_tc_kernel": 217.2}
 # timer regions of the edge kernels of an l<=2 message layer -> kernel names
 BEE_EDGE_REGIONS = {"bee_messages_fused_tc": "bee_fused_tc_kernel", "bee_messages_scalar_tc": "bee_scalar_tc_kernel",
-                    "bee_messages_scalar": "bee_scalar_split_kernel", "bee_messages_vd": "bee_vd_kernel",
+                    "bee_messages_scalar_split": "bee_scalar_split_kernel", "bee_messages_scalar": "bee_scalar_kernel", "bee_messages_vd": "bee_vd_kernel",
                     "bee_messages_vd_tc": "bee_vd_tc_kernel"}
+PAINN_REGIONS = {"painn_message_slabs": "painn_message_bf16_kernel", "painn_message_tc": "painn_message_tc_kernel",
+                 "painn_message_split": "painn_message_split_kernel", "painn_message": "painn_message_kernel"}
 
 
 def make_positions(w, systems, seed):
@@ -303,7 +305,7 @@ def run_graph_bench(args, w):
         "config": {"workload": args.workload, "systems": w["systems"], "nodes_per_system": w["nodes"], "box": w["box"],
                    "cutoff": w["cutoff"], "edges": E, "l2_policy": "256 MB flush buffer written between timed iterations"},
         "e2e": {"value": E * args.steps / (e2e_ms * 1e-3), "unit": "edges/s", "h2d_bytes_per_step": Nt * 12, "d2h_bytes_per_step": 12 * E},
-        "gpu_launches": 14 * args.steps, "clocks": clocks,
+        "gpu_launches": (builder.count_launches + 1) * args.steps, "clocks": clocks,
         "roofline": {"bound": "hbm", "kernel": "radius graph build (neighbour_kernel<0/1> dominate)", "achieved": achieved,
                      "peak": hbm, "unit": "GB/s", "frac": achieved / hbm, "traffic": None, "peak_source": f"hbm_gbs, {how}"},
     }
@@ -514,8 +516,8 @@ def main():
         if is_bee:
             roof = bee_layer_roofline(w, ktimes, local_edges, per, tc_path, hbm, tf_sus, how)
         else:
-            kname = "painn_message_bf16_kernel" if tc_path else "painn_message_split_kernel"
-            msg = ktimes.get("painn_message_tc" if tc_path else "painn_message", {"launches": 0, "ms": 0.0})
+            region = next((r for r in PAINN_REGIONS if r in ktimes), None)   # one kernel form per run: it depends on widths only
+            kname, msg = PAINN_REGIONS.get(region), ktimes.get(region, {"launches": 0, "ms": 0.0})
             flops = message_flops_per_edge(w["n"], w["n_rbf"])
             if msg["launches"]:
                 per_launch_s = msg["ms"] * 1e-3 / msg["launches"]
@@ -526,7 +528,8 @@ def main():
                         "traffic": DRAM_BYTES_PER_EDGE[kname] * edges_launch if kname in DRAM_BYTES_PER_EDGE else None,
                         "peak_source": f"bf16_tflops_sustained, {how}", "launches": msg["launches"], "avg_launch_ms": per_launch_s * 1e3,
                         "note": ("tcgen05 BF16 MMAs of the per-edge distance MLP (algorithmic flops: 2*(n_rbf*4n + 2*(4n)^2) per edge)"
-                                 if tc_path else "FP32-accurate products as three FP16 MMAs each, algorithmic flops against the dense bf16 tensor peak")}
+                                 if tc_path else ("FP32-accurate products as three FP16 MMAs each" if region == "painn_message_split" else "FP32 FMAs") +
+                                 ", algorithmic flops against the dense bf16 tensor peak")}
         line = {
             "metric": "edge_messages_per_sec", "value": value, "unit": "edge-messages/s", "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": total_ms / args.steps, "higher_is_better": True, "scaling": "strong",

@@ -51,6 +51,9 @@ const char* ld_status_string(int status);
  * node is deterministic. shift/rij may be NULL. */
 int ld_radius_graph_workspace_size(int batch, int nodes, int periodic, float cutoff, const float* box, int mode,
                                    int open_cells_cap, size_t* bytes);
+/* kernels that one _count (with edge_counts) launches for these sizes; a _fill is one */
+int ld_radius_graph_launches(int batch, int nodes, int periodic, float cutoff, const float* box, int mode, int open_cells_cap,
+                             int* launches);
 int ld_radius_graph_count(const float* pos, int batch, int nodes, int periodic, float cutoff, const float* box, int mode,
                           int open_cells_cap, void* workspace, size_t workspace_bytes, int* row_ptr, int* edge_counts,
                           int* status_dev, void* stream);

@@ -693,6 +693,23 @@ __global__ void capacity_flag_kernel(const int* __restrict__ row_ptr, int Nt, in
 }
 }  // namespace
 
+// which kernels a count launches: a system's cells by one block where it can hold them; up to 16384 nodes the prefix sum in one
+// launch of a few us instead of four (its serial part grows with the count); row_ptr is int32, so only problems whose edge count
+// could pass 2^31-1 pay for the 64-bit check of the degree sum
+static bool block_holds_system(const GraphParams& P) { return P.nodes <= CELL_MAX_NODES && P.cells_cap <= CELL_MAX_CELLS; }
+static bool one_scan(const GraphParams& P) { return (long long)P.batch * P.nodes <= ONE_SCAN_MAX; }
+static bool may_overflow(const GraphParams& P) { return (long long)P.batch * P.nodes * (P.nodes - 1) > 0x7fffffffLL; }
+
+// kernels that one ld_radius_graph_count with edge counts launches (a fill: one)
+extern "C" int ld_radius_graph_launches(int batch, int nodes, int periodic, float cutoff, const float* box, int mode, int open_cells_cap,
+                                        int* launches) {
+  GraphParams P;
+  const int rc = make_params(batch, nodes, periodic, cutoff, box, mode, open_cells_cap, &P);
+  if (rc != LD_OK) return rc;
+  *launches = batch > 0 && nodes > 0 ? (block_holds_system(P) ? 1 : 7) + 1 + (one_scan(P) ? 1 : 4) + (may_overflow(P) ? 1 : 0) : 0;
+  return LD_OK;
+}
+
 extern "C" int ld_radius_graph_workspace_size(int batch, int nodes, int periodic, float cutoff, const float* box,
                                               int mode, int open_cells_cap, size_t* bytes) {
   GraphParams P;
@@ -724,7 +741,7 @@ extern "C" int ld_radius_graph_count(const float* pos, int batch, int nodes, int
     LD_CUDA_TRY(cudaMemsetAsync(row_ptr, 0, 4, stream));
     return LD_OK;
   }
-  if (nodes <= CELL_MAX_NODES && P.cells_cap <= CELL_MAX_CELLS) {
+  if (block_holds_system(P)) {
     int span = 1;
     while (span < nodes) span <<= 1;
     const size_t smem = 4 * ((size_t)2 * (P.cells_cap + 1) + (size_t)nodes + key_at(span));
@@ -757,21 +774,18 @@ extern "C" int ld_radius_graph_count(const float* pos, int batch, int nodes, int
     neighbour_kernel<false, false><<<nblk, NB_WARPS * 32, 0, stream>>>(pos, P, w.desc, w.cell_start, w.sorted, w.sorted_cell, group, w.degree, nullptr,
                                                                        0, nullptr, nullptr, nullptr, nullptr, status_dev);
   LD_LAUNCH_CHECK();
-  // up to 16384 nodes the prefix sum is one launch of a few us instead of four (its serial part grows with the count)
-  const bool one_scan = Nt <= ONE_SCAN_MAX;
-  if (one_scan) {
+  if (one_scan(P)) {
     degree_scan_kernel<<<1, ONE_SCAN_THREADS, 0, stream>>>(w.degree, Nt, nodes, row_ptr, edge_counts);
     LD_LAUNCH_CHECK();
   } else {
     rc = ld_scan_exclusive(w.degree, row_ptr, (long long)Nt, w.scan, stream);
     if (rc != LD_OK) return rc;
   }
-  // row_ptr is int32: only problems whose edge count could pass 2^31-1 pay for the 64-bit check of the degree sum
-  if ((long long)Nt * (nodes - 1) > 0x7fffffffLL) {
+  if (may_overflow(P)) {
     degree_overflow_kernel<<<1, 256, 0, stream>>>(w.degree, Nt, status_dev);
     LD_LAUNCH_CHECK();
   }
-  if (edge_counts != nullptr && !one_scan) {
+  if (edge_counts != nullptr && !one_scan(P)) {
     edge_counts_kernel<<<ld_cdiv(batch, 256), 256, 0, stream>>>(row_ptr, batch, nodes, edge_counts);
     LD_LAUNCH_CHECK();
   }

@@ -16,6 +16,7 @@ LD_FLAG_CAPACITY, LD_FLAG_NONFINITE, LD_FLAG_TIMEOUT, LD_FLAG_OVERFLOW = 1, 2, 4
 # name -> argtypes ; every entry point declared in include/ld_hotpath.h
 P, I, F, LL, SZ = c_void_p, c_int, c_float, c_ll, c_size_t
 SIGNATURES = {
+    "ld_radius_graph_launches": [I, I, I, F, P, I, I, P],
     "ld_radius_graph_workspace_size": [I, I, I, F, P, I, I, P],
     "ld_radius_graph_count": [P, I, I, I, F, P, I, I, P, SZ, P, P, P, P],
     "ld_radius_graph_fill": [P, I, I, I, F, P, I, I, P, SZ, P, LL, P, P, P, P, P, P],

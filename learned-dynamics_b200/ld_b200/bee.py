@@ -252,7 +252,8 @@ class Messages(nn.Module):
             if "split" in w:
                 # both edge kernels read the neighbours' rows component-major, [node][13][chan]
                 rows13 = torch.empty(Nt, 13, C, dtype=torch.float32, device=dev)
-                check(lib().ld_bee_rows13_f32(ptr(l0), ptr(l1), ptr(l2), Nt, C, ptr(rows13), stream_ptr(dev)))
+                with KERNEL_TIMER.region("bee_rows13"):
+                    check(lib().ld_bee_rows13_f32(ptr(l0), ptr(l1), ptr(l2), Nt, C, ptr(rows13), stream_ptr(dev)))
                 l0 = l1 = l2 = rows13
         rij = r_ij.contiguous()
         # the per-node product sums feed tensor-core channel mixings on the bf16 path, which round them to BF16 anyway
@@ -286,7 +287,7 @@ class Messages(nn.Module):
             if fuse_add:
                 B_a += x_a.reshape(Nt, -1)
         elif "split" in w:
-            with KERNEL_TIMER.region("bee_messages_scalar"):
+            with KERNEL_TIMER.region("bee_messages_scalar_split"):
                 check(lib().ld_bee_messages_scalar_f32_split(ptr(graph.row_ptr), ptr(graph.dst32), ptr(rij), Nt, C, self.dim_a,
                                                              float(self.r0), ptr(l0), ptr(w["enc_w"]), ptr(w["enc_b"]), ptr(w["jac"]),
                                                              ptr(w["split"]), ptr(w["split_scales"]), ptr(w["b1"]), ptr(w["b2"]),

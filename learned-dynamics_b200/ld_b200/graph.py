@@ -34,8 +34,10 @@ class RadiusGraphBuilder:
         self.workspace = torch.empty(max(nbytes.value, 16), dtype=torch.uint8, device=self.device)
         self.status = torch.zeros(1, dtype=torch.int32, device=self.device)
         Nt = self.batch * self.nodes
-        # kernels of a count: cells (one block per system, or seven over all particles), search, prefix sum
-        self._launches = (1 if self.nodes <= 8192 else 7) + 1 + (1 if Nt <= 16384 else 4)
+        launches = ctypes.c_int(0)
+        check(lib().ld_radius_graph_launches(self.batch, self.nodes, self.periodic, self.cutoff, self._box_ptr, self.mode,
+                                             self.open_cells_cap, ctypes.byref(launches)))
+        self.count_launches = launches.value
         self.row_ptr = torch.empty(Nt + 1, dtype=torch.int32, device=self.device)
         self.edge_counts = torch.empty(max(self.batch, 1), dtype=torch.int32, device=self.device)[: self.batch]
 
@@ -43,7 +45,7 @@ class RadiusGraphBuilder:
         require_cuda_f32(pos, "pos")
         if tuple(pos.shape) != (self.batch, self.nodes, 3):
             raise RuntimeError("x must have shape (batch, nodes, 3)")
-        with KERNEL_TIMER.region("radius_graph_count", launches=self._launches):
+        with KERNEL_TIMER.region("radius_graph_count", launches=self.count_launches):
             check(lib().ld_radius_graph_count(ptr(pos), self.batch, self.nodes, self.periodic, self.cutoff, self._box_ptr,
                                               self.mode, self.open_cells_cap, ptr(self.workspace), self.workspace.numel(),
                                               ptr(self.row_ptr), ptr(self.edge_counts), ptr(self.status),

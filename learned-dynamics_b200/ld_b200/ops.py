@@ -366,7 +366,7 @@ def painn_message_f32(row_ptr, dst, rij, mlp_dist, actv, x_v, rmax, eps=0.1, rad
     out_v = torch.empty(Nt, n, 3, dtype=torch.float32, device=x_v.device)
     split = _packed_split(mlp_dist, n)
     if split is not None:   # n = 32, 64, 128: the distance MLP on the tensor cores, operands as sums of two FP16 values
-        with KERNEL_TIMER.region("painn_message"):
+        with KERNEL_TIMER.region("painn_message_split"):
             check(lib().ld_painn_message_f32_split(ptr(row_ptr), ptr(dst), ptr(rij), Nt, n, n_rbf, radial_kind, float(rmax), float(eps),
                                                    ptr(split), None, ptr(mlp_dist.b[0]), ptr(mlp_dist.b[1]),
                                                    ptr(mlp_dist.b[2]), ptr(actv), ptr(x_v), ptr(res_a), ptr(res_v), ptr(out_a),
@@ -535,7 +535,7 @@ def painn_message_bf16_tc(row_ptr, dst, rij, mlp_dist, actv, x_v, rmax, eps=0.1,
         w = _packed_slabs(mlp_dist)
         out_a = torch.empty(Nt, n, dtype=torch.float32, device=x_v.device)
         out_v = torch.empty(Nt, n, 3, dtype=torch.float32, device=x_v.device)
-        with KERNEL_TIMER.region("painn_message_tc"):
+        with KERNEL_TIMER.region("painn_message_slabs"):
             check(lib().ld_painn_message_bf16_slabs(ptr(row_ptr), ptr(dst), ptr(rij), Nt, n, n_rbf, radial_kind, float(rmax), float(eps),
                                                     ptr(w[0]), ptr(mlp_dist.b[0]), ptr(w[1]), ptr(mlp_dist.b[1]), ptr(w[2]),
                                                     ptr(mlp_dist.b[2]), ptr(actv), ptr(x_v), ptr(res_a), ptr(res_v), ptr(out_a), ptr(out_v),

@@ -52,3 +52,8 @@ def test_argument_errors_without_gpu():
     # the direct weight of ld_mlp3_rows need not be aligned, the three layers' have to be
     mlp = lambda w, wd: L.ld_mlp3_rows(None, 0, 8, w, None, 16, w, None, 16, w, None, 16, 1, wd, None, None)  # noqa: E731
     assert mlp(16, 20) == 0 and mlp(20, 16) == _lib.LD_ERR_SHAPE
+    # kernels of a graph build's count: one block per system up to 8192 nodes and cells, one prefix sum up to 16384 nodes
+    k = C.c_int(0)
+    for batch, nodes, side, want in ((2, 512, 20.0, 3), (32, 4096, 16.0, 6), (1, 8193, 20.0, 9), (2, 300, 30.0, 9), (0, 4, 20.0, 0)):
+        cube = (C.c_float * 3)(side, side, 2 * side if side == 30.0 else side)   # (30 x 30 x 60 cells of 1)
+        assert L.ld_radius_graph_launches(batch, nodes, 1, 1.0, C.cast(cube, C.c_void_p), 0, 0, C.byref(k)) == 0 and k.value == want
