@@ -622,3 +622,38 @@ def test_scalar_channel_over_several_segments(chan, dim_a, nodes):
     for lo in range(0, nodes, chunk):
         assert torch.equal(whole[lo:lo + chunk], run(lo, min(lo + chunk, nodes))), lo
     assert bool((whole[deg == 0] == 0).all()) and int(ops.tc_status("cuda")) == 0
+
+
+@pytest.mark.parametrize("kernel", ["f32-32", "f32-64", "f32-128", "bf16-32", "bf16-64", "bf16-128", "scalar-64-64", "scalar-128-128"])
+def test_edge_kernels_repeat_themselves(kernel):
+    """a slab that is read before it has landed, or a plane that is still being written, would show as bits that differ from one
+    launch to the next: a few tiles a block, 600 launches"""
+    from ld_b200 import bee, ops
+    from ld_b200._lib import lib, check, ptr, stream_ptr
+    kind, n = kernel.split("-")[0], int(kernel.split("-")[1])
+    deg, src, dst, rij = _chunk_graph(9000, 9000, 3)
+    row_ptr = torch.cat([torch.zeros(1, dtype=torch.long), deg.cumsum(0)]).int().cuda()
+    dst, rij, nodes = dst.int().cuda(), rij.cuda(), len(deg)
+    torch.manual_seed(n)
+    if kind == "scalar":
+        m = bee.Messages(5.0, n, 32, 32, n).cuda()
+        with torch.no_grad():
+            w = m._pack()
+        rows = torch.randn(nodes, 13, n, device="cuda")
+
+        def run():
+            out = torch.empty(nodes, n, device="cuda")
+            check(lib().ld_bee_messages_scalar_f32_split(ptr(row_ptr), ptr(dst), ptr(rij), nodes, n, n, 5.0, ptr(rows), ptr(w["enc_w"]),
+                                                         ptr(w["enc_b"]), ptr(w["jac"]), ptr(w["split"]), None, ptr(w["b1"]), ptr(w["b2"]),
+                                                         ptr(w["b3"]), 0.1, ptr(out), ptr(ops.tc_status("cuda")), stream_ptr()))
+            return (out,)
+    else:
+        mlp = ops.PackedMLP([torch.nn.Linear(k, 4 * n).cuda() for k in (8, 4 * n, 4 * n)])
+        actv, x_v = torch.randn(nodes, 4 * n, device="cuda"), torch.randn(nodes, n, 3, device="cuda")
+        fused = ops.painn_message_bf16_tc if kind == "bf16" else ops.painn_message_f32
+        run = lambda: fused(row_ptr, dst, rij, mlp, actv, x_v, 4.0, radial_kind=1)  # noqa: E731
+    first, other = run(), torch.zeros((), dtype=torch.bool, device="cuda")
+    for _ in range(600):
+        for a, b in zip(first, run()):
+            other |= (a != b).any()
+    assert not bool(other) and int(ops.tc_status("cuda")) == 0
