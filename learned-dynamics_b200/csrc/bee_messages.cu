@@ -81,8 +81,8 @@ __device__ __forceinline__ void edge_phi(const EdgeGeom& g, const float* w8, flo
 // the layouts a channel mixing with 5*chan inputs expects. Thread = channel; a block walks its nodes
 // and stages the geometry of up to 32 edges at a time in shared memory.
 // CC: the channel count as a compile-time constant (0: taken from the parameters). PACKED: BF16 rows [node][chan][16].
-// ROWS13: FP32 rows [node][13][chan], so that a warp's loads are consecutive addresses (219 k edges, 128 channels: 180 us
-// with the strided loads of the separate rank-1 and rank-2 features, 152 us so).
+// ROWS13: FP32 rows [node][13][chan], so that a warp's loads are consecutive addresses (176 k edges, 128 channels: 183 us
+// with the strided loads of the separate rank-1 and rank-2 features, 162 us so).
 template <typename FT, bool PACKED, int CC, bool ROWS13 = false>
 __global__ void __launch_bounds__(128, 4)   // four blocks per SM: at most 128 registers
 bee_vd_kernel(BeeEdgeParams P, float* __restrict__ S_v, float* __restrict__ S_d, float scale, int out_bf16_) {

@@ -6,15 +6,15 @@
 //   psi = Y y ;  h1 = leaky(W1 psi + b1) ;  h2 = leaky(W2 h1 + b2)      widths A, 2 A, 2 A
 //   out = psi + Wd psi + W3 h2 + b3, summed per source node, times `scale`
 //
-// What bounds it: the shared-memory port under the MMAs (48 cycles per 128 x 64 x 16 MMA plus the weight slabs that arrive
-// through it) and the phases of a tile that follow one another. C = A = 128, 219 k edges: 0.68 ms, against 7.39 ms on
-// the FMA pipe.
+// What bounds it: the phases of a tile, which follow one another (the tensor pipe is active 15 % of the time), and within the
+// products the shared-memory port (48 cycles per 128 x 64 x 16 MMA, and the weight slabs that arrive through it).
+// C = A = 128, 176 k edges: 0.71 ms, against 7.38 ms on the FMA pipe.
 //
 // A block owns a node-aligned slice of the CSR and walks it 64 edges at a time; roles as in painn_message_split.cu. The
 // neighbours' rows are read component-major, [node][13][C], so that a warp's loads are 128 consecutive bytes. The sizes of
 // the products are not bounded beforehand: the scale of an edge's operands comes from its largest product, those of the
-// later layers from that and from each channel's row sum of the weights (split_pack.cuh). Every step of the pipeline is two weight slabs: the two blocks
-// of 128 channels of a hidden layer, or two chunks of K of a layer with one block.
+// later layers from that and from each channel's bounds (split_pack.cuh). Every step of the pipeline is two weight slabs: the
+// two blocks of 128 channels of a hidden layer, or two chunks of K of a layer with one block.
 #include "common.cuh"
 #include "split_f16.cuh"
 #include "split_pack.cuh"

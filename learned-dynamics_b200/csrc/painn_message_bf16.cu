@@ -6,7 +6,7 @@
 // them) the ring holds more and smaller slabs, a thread owns one channel, so that an epilogue needs one bias and the messages
 // of a channel are formed from coalesced FP32 rows, and the half of the channels that is complete first goes through its
 // activation while the other half is multiplied.
-// n = 128, 8 radial functions, 2.25 M edges: 3.80 ms, against 4.52 ms (+ 10 us of packing).
+// n = 128, 8 radial functions, 2.25 M edges: 3.75 ms, against 4.52 ms (+ 10 us of packing).
 //
 // A block owns a node-aligned, contiguous slice of the CSR. Roles: 16 working warps, 2 MMA warps (of every pair of channel
 // blocks one each), 1 producer warp. Every wait is bounded: a failed wait is OR-ed into the next block barrier so that all

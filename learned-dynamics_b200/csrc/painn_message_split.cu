@@ -1,11 +1,13 @@
 // PaiNN message step at FP32 accuracy with the distance MLP on the tensor cores: the computation of painn_message.cu
 // (Message.forward, archs/meanflow_painn8.py:77-100) with operands split into two FP16 values (split_f16.cuh).
 //
-// What bounds it: the shared-memory port. The two 4n x 4n layers are 3 x 2 x (4n)^2 flops an edge on the tensor cores; an MMA
-// of 128 x 64 x 16 (n = 128) takes 48 cycles, the time to read its 6 KB of operands, not the 32 of the tensor pipe, and the
-// weight slabs (2 MB per tile) come in through the same port: 433 cycles a slab of six MMAs measured, 416 by that count.
-// n = 128, 8 radial functions, 562 k edges: 3.06 ms, against 22.8 ms on the FMA pipe (painn_message.cu); n = 64, 11 k edges:
-// 68 us against 195. Error against 64 bits: 6.1e-7, against 7.5e-7.
+// What bounds it: the phases of a tile, which follow one another (matrix products, epilogue, messages, sums), and within the
+// products the shared-memory port. The two 4n x 4n layers are 3 x 2 x (4n)^2 flops an edge on the tensor cores; an MMA of
+// 128 x 64 x 16 (n = 128) takes 48 cycles, the time to read its 6 KB of operands, not the 32 of the tensor pipe, and the weight
+// slabs (2 MB per tile) come in through the same port: 433 cycles a slab of six MMAs measured, 416 by that count. Over the
+// launch the tensor pipe is active 29 % of the time.
+// n = 128, 8 radial functions, 562 k edges: 3.01 ms, against 22.8 ms on the FMA pipe (painn_message.cu); n = 64, 1024 edges of
+// 512 nodes: 55 us against 79. Error against 64 bits in the first case: 4.5e-7, against 7.3e-7.
 //
 // A block owns a node-aligned, contiguous slice of the CSR and walks it 256 / (n / 32) edges at a time. Roles:
 //   * 16 working warps: geometry, radial features -> activation planes in shared memory; per layer each thread adds the
@@ -71,7 +73,8 @@ __device__ __forceinline__ float radial_gaussian(int m, int n, float d, float rm
   return expf(-0.5f * u * u);
 }
 
-// SiLU with the quotient from the reciprocal instruction (2 ulp)
+// SiLU with the quotient from the reciprocal instruction (2 ulp; zero below -87.3, where the pair that holds the result resolves
+// 2^-79 at best). The exact quotient: 3.29 ms instead of 3.11 (n = 128, 562 k edges), the same distance from 64 bits.
 __device__ __forceinline__ float silu_fdiv(float x) { return __fdividef(x, 1.0f + expf(-x)); }
 
 template <int MB>
