@@ -308,19 +308,16 @@ def mlp3_rows(x, mlp, act=ACT_SILU):
     return out
 
 
-def _require_numel(t, name, numel):
-    require_cuda_f32(t, name)
-    if t.numel() != numel:
-        raise RuntimeError(f"{name}: {numel} elements expected, got {tuple(t.shape)}")
+def _require_sizes(*pairs):
+    """(tensor, elements) pairs: what a kernel reads without a look at shapes"""
+    for t, numel in pairs:
+        if t.numel() != numel or not t.is_cuda or not t.is_contiguous() or t.dtype != torch.float32:
+            raise RuntimeError(f"PaiNN update: {numel} contiguous float32 elements expected on the GPU, got {tuple(t.shape)}, {t.dtype}, {t.device}")
 
 
 def painn_update_mix(W_l, W_r, W_v, x_v, rows, n):
     """y [rows, 3n, 3] = the three channel mixings of x_v, stacked; the weights (contiguous float32 [n, n]) are read in place"""
-    _require_numel(x_v, "x_v", rows * n * 3)
-    for W in (W_l, W_r, W_v):
-        require_cuda_f32(W, "W")
-        if tuple(W.shape) != (n, n):
-            raise RuntimeError("painn_update_mix: weights must be [n, n]")
+    _require_sizes((x_v, rows * n * 3), (W_l, n * n), (W_r, n * n), (W_v, n * n))
     y = torch.empty(rows, 3 * n, 3, dtype=torch.float32, device=x_v.device)
     with KERNEL_TIMER.region("tensor_linear"):
         check(lib().ld_painn_update_mix(ptr(W_l), ptr(W_r), ptr(W_v), ptr(x_v), rows, n, ptr(y), stream_ptr(x_v.device)))
@@ -329,8 +326,7 @@ def painn_update_mix(W_l, W_r, W_v, x_v, rows, n):
 
 def painn_update_front(y, x_a, rows, n):
     """y [rows, 3n, 3] = the stacked mixings of x_v: (inner [rows, n], cat [rows, 2n]) of PaiNN's Update"""
-    _require_numel(y, "y", rows * 9 * n)
-    _require_numel(x_a, "x_a", rows * n)
+    _require_sizes((y, rows * 9 * n), (x_a, rows * n))
     inner = torch.empty(rows, n, dtype=torch.float32, device=y.device)
     cat = torch.empty(rows, 2 * n, dtype=torch.float32, device=y.device)
     with KERNEL_TIMER.region("painn_update"):
@@ -339,10 +335,9 @@ def painn_update_front(y, x_a, rows, n):
 
 
 def painn_update_back(y, m, inner, x_a, x_v, rows, n):
-    """(scaled, base [rows, n]; the new x_v, shaped as x_v): the group norm of `scaled` plus `base` is the new x_a"""
-    for t, name, width in ((y, "y", 9 * n), (m, "m", 3 * n), (inner, "inner", n), (x_a, "x_a", n), (x_v, "x_v", 3 * n)):
-        _require_numel(t, name, rows * width)
-    scaled, base = torch.empty_like(inner), torch.empty_like(inner)
+    """(scaled, base, shaped as x_a; the new x_v, shaped as x_v): the group norm of `scaled` plus `base` is the new x_a"""
+    _require_sizes((y, rows * 9 * n), (m, rows * 3 * n), (inner, rows * n), (x_a, rows * n), (x_v, rows * 3 * n))
+    scaled, base = torch.empty_like(x_a), torch.empty_like(x_a)
     out_v = torch.empty_like(x_v)
     with KERNEL_TIMER.region("painn_update"):
         check(lib().ld_painn_update_back(ptr(y), ptr(m), ptr(inner), ptr(x_a), ptr(x_v), rows, n, ptr(scaled), ptr(base), ptr(out_v),

@@ -100,16 +100,21 @@ class Update(nn.Module):
         assert n % 4 == 0
         self.gn = ScalGroupNorm(n, 4, epsilon=1.)
 
-    def _mixing_weights(self):
-        """the weights of lin_l, lin_r and lin_v where the fused form may read them, else None"""
+    def _mixing_weights(self, device):
+        """the weights of lin_l, lin_r and lin_v where the fused form may read them on `device`, else None"""
         parts = self._modules   # (attribute access of a module looks its parts up last)
-        lins = [parts[k] for k in ("lin_l", "lin_r", "lin_v")]
-        if not (_as_built(self, Update) and all(_as_built(l, TensLinear) and l.inds == 1 and l.precision == "fp32" for l in lins)
-                and _as_built(parts["mlp"], MLP) and _as_built(parts["gn"], ScalGroupNorm)
+        lins = parts["lin_l"], parts["lin_r"], parts["lin_v"]
+        if not (_as_built(self, Update) and _as_built(parts["mlp"], MLP) and _as_built(parts["gn"], ScalGroupNorm)
                 and not nn_module._global_forward_hooks and not nn_module._global_forward_pre_hooks):
             return None
+        for l in lins:
+            if not _as_built(l, TensLinear) or l.inds != 1 or l.precision != "fp32":
+                return None
         W = [l._parameters["W"] for l in lins]
-        return W if all(w.dtype == torch.float32 and w.is_contiguous() for w in W) else None
+        for w in W:
+            if w.dtype != torch.float32 or w.device != device or not w.is_contiguous():
+                return None
+        return W
 
     def residual(self, x_a, x_v):
         """x_a + dx_a, x_v + dx_v. Without autograd: the three channel mixings as one launch on the weights as they are, and
@@ -118,7 +123,7 @@ class Update(nn.Module):
         W = None
         if (not torch.is_grad_enabled() and x_a.is_cuda and x_a.dim() == 3 and x_a.dtype == torch.float32 and x_v.dtype == torch.float32
                 and x_a.shape[2] == self.n and x_v.shape == (*x_a.shape, 3) and x_v.device == x_a.device):
-            W = self._mixing_weights()
+            W = self._mixing_weights(x_a.device)
         if W is None:
             dx_a, dx_v = self(x_a, x_v)
             return x_a + dx_a, x_v + dx_v
@@ -127,7 +132,7 @@ class Update(nn.Module):
         y = ops.painn_update_mix(*W, x_v, rows, n)
         inner, cat = ops.painn_update_front(y, x_a, rows, n)
         scaled, base, out_v = ops.painn_update_back(y, self.mlp(cat), inner, x_a, x_v, rows, n)
-        return self.gn(scaled.reshape(x_a.shape), residual=base.reshape(x_a.shape)), out_v
+        return self.gn(scaled, residual=base), out_v
 
     def forward(self, x_a, x_v):
         x_v_l = self.lin_l(x_v)

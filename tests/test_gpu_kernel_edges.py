@@ -657,3 +657,19 @@ def test_edge_kernels_repeat_themselves(kernel):
         for a, b in zip(first, run()):
             other |= (a != b).any()
     assert not bool(other) and int(ops.tc_status("cuda")) == 0
+
+
+def test_painn_update_refuses_weights_that_are_elsewhere():
+    """weights in host memory are refused, weights that are not contiguous float32 take the separate operations"""
+    from ld_b200 import painn
+    torch.manual_seed(8)
+    x_a, x_v = torch.randn(2, 5, 32).cuda(), torch.randn(2, 5, 32, 3).cuda()
+    with torch.no_grad(), pytest.raises(RuntimeError):
+        painn.Update(32).residual(x_a, x_v)
+    m = painn.Update(32).cuda()
+    with torch.no_grad():
+        want = m.residual(x_a, x_v)
+        m.lin_v.W.data = m.lin_v.W.data.t().contiguous().t()
+        got = m.residual(x_a, x_v)
+    assert not m.lin_v.W.is_contiguous()
+    assert all(float((a - b).norm()) <= 1e-5 * float(b.norm()) for a, b in zip(got, want))
