@@ -673,3 +673,13 @@ def test_painn_update_refuses_weights_that_are_elsewhere():
         got = m.residual(x_a, x_v)
     assert not m.lin_v.W.is_contiguous()
     assert all(float((a - b).norm()) <= 1e-5 * float(b.norm()) for a, b in zip(got, want))
+
+
+# tiles of 32, 64 and 128 outputs that lie in one of the three matrices, that straddle two, that hold all three
+@pytest.mark.parametrize("n,rows", [(4, 100), (24, 6000), (32, 37), (40, 5001), (64, 2500), (64, 6000), (100, 3000), (128, 37), (128, 3000), (128, 6001)])
+def test_update_mix_equals_the_stacked_mixing(n, rows):
+    from ld_b200 import ops
+    torch.manual_seed(n)
+    W = [torch.randn(n, n).cuda() for _ in range(3)]
+    x = torch.randn(rows, n, 3).cuda()
+    assert torch.equal(ops.painn_update_mix(*W, x, rows, n), ops.tensor_linear_fwd(1, torch.cat(W), x))
